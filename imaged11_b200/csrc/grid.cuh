@@ -274,66 +274,129 @@ __device__ __forceinline__ void column_l_range(const volatile WarpPlan* wp, doub
     }
 }
 
+// How the lookup's work is split: every UBI into slabs (the lattice points by
+// the z of UB.hkl) x cols (its (h, k) columns).  The slabs are the outermost
+// order of the work items, so the warps that run together read one z range of
+// the index: where the index is larger than L2, each slab's share of it stays
+// there while all UBIs pass over it.
+struct Item {
+    int64_t i;                       // UBI
+    int part, slab, slabs, col, cols;  // part = slab * cols + col
+};
+
+struct Split {
+    int slabs, cols;
+    __host__ __device__ __forceinline__ int parts() const { return slabs * cols; }
+    __device__ __forceinline__ Item item(int64_t wk, int64_t m) const {
+        const int64_t per = m * cols;
+        const int slab = (int)(wk / per);
+        const int64_t r = wk - slab * per;
+        const int64_t i = r / cols;
+        const int col = (int)(r - i * cols);
+        return Item{i, slab * cols + col, slab, slabs, col, cols};
+    }
+};
+
 // Every hkl whose box [UB.hkl - w, UB.hkl + w] can reach a regular g (inside
-// the data cube and within rmax of the origin), for the (h, k) columns of work
-// item `part` of `parts`.  32 (h, k) columns at a time, each lane solving for
+// the data cube and within rmax of the origin), for the work item's (h, k)
+// columns and the slab of its centre.  32 (h, k) columns at a time, each lane solving for
 // the range of l whose lattice point lies within rmax + |w| of the origin, the
-// 32 ranges flattened across the warp.  emit(pass, h, k, l, c) is called by
-// every lane of the warp together (warp-synchronous); pass says whether the
-// lane holds a box, c is its centre UB.hkl.
-template <class Emit>
-__device__ __forceinline__ void enumerate_boxes(const volatile WarpPlan* wp, int part, int parts,
-                                                int lane, const Header& H, Emit& emit) {
-    const int nh0 = wp->nh[0];
-    const int64_t nhk = (int64_t)nh0 * wp->nh[1];
+// 32 ranges flattened across the warp.  next() is called by every lane of the
+// warp together: false after the last step; else pass says whether the lane
+// holds a box, of hkl (h, k, l).
+struct BoxWalk {
+    int64_t hb, stride, nhk;  // the next 32 columns, of nhk
+    int hc, kc, l0, excl;     // the lane's column, its first l and its prefix of the flattened l
+    int f0, total;            // the next step's first candidate, of total
+    int slab, slabs;
     double n0, n1;
-    ub_column_norms(wp, n0, n1);
-    for (int64_t hb = (int64_t)part * 32; hb < nhk; hb += 32 * (int64_t)parts) {
-        const int64_t hk = hb + lane;
-        int len = 0, l0 = 0, h = 0, k = 0;
-        if (hk < nhk) {
-            h = wp->lo[0] + (int)(hk % nh0);
-            k = wp->lo[1] + (int)(hk / nh0);
-            const double R = (H.rmax + sqrt(wp->w[0] * wp->w[0] + wp->w[1] * wp->w[1] +
-                                            wp->w[2] * wp->w[2])) * (1. + 1e-9) + 1e-12;
-            column_l_range(wp, n0, n1, h, k, R, l0, len);
-        }
-        int total;
-        const int excl = warp_excl_scan(len, lane, total);
-        for (int f0 = 0; f0 < total; f0 += 32) {
-            const int f = f0 + lane;
-            const int j = owner(excl, f);
-            const int hj = __shfl_sync(0xffffffffu, h, j);
-            const int kj = __shfl_sync(0xffffffffu, k, j);
-            const int lj = __shfl_sync(0xffffffffu, l0, j) + f - __shfl_sync(0xffffffffu, excl, j);
-            bool pass = false;
-            double c[3] = {0., 0., 0.};
-            if (f < total) {
-                const double hkl[3] = {(double)hj, (double)kj, (double)lj};
-                bool in = true;
-                double d2 = 0.;
-                const double G = -H.lo;
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    c[r] = wp->ub[3 * r] * hkl[0] + wp->ub[3 * r + 1] * hkl[1] +
-                           wp->ub[3 * r + 2] * hkl[2];
-                    const double wr = wp->w[r];
-                    in = in && (c[r] - wr <= G) && (c[r] + wr >= -G);
-                    const double e = fmax(fabs(c[r]) - wr, 0.);
-                    d2 += e * e;
-                }
-                pass = in && d2 <= H.rmax * H.rmax * (1. + 1e-9);
+
+    __device__ __forceinline__ BoxWalk(const volatile WarpPlan* wp, const Item& it)
+        : hb((int64_t)it.col * 32), stride(32 * (int64_t)it.cols),
+          nhk((int64_t)wp->nh[0] * wp->nh[1]), hc(0), kc(0), l0(0), excl(0), f0(0), total(0),
+          slab(it.slab), slabs(it.slabs) {
+        ub_column_norms(wp, n0, n1);
+    }
+
+    __device__ __forceinline__ bool next(const volatile WarpPlan* wp,
+                                         const Header* __restrict__ Hp, int lane, bool& pass,
+                                         int& h, int& k, int& l) {
+        while (f0 >= total) {
+            if (hb >= nhk) return false;
+            const int64_t hk = hb + lane;
+            hb += stride;
+            int len = 0;
+            hc = kc = l0 = 0;
+            if (hk < nhk) {
+                const int nh0 = wp->nh[0];
+                hc = wp->lo[0] + (int)(hk % nh0);
+                kc = wp->lo[1] + (int)(hk / nh0);
+                const double R = (Hp->rmax + sqrt(wp->w[0] * wp->w[0] + wp->w[1] * wp->w[1] +
+                                                  wp->w[2] * wp->w[2])) * (1. + 1e-9) + 1e-12;
+                column_l_range(wp, n0, n1, hc, kc, R, l0, len);
+                if (slabs > 1) clip_to_slab(wp, -Hp->lo, len);
             }
-            emit(pass, hj, kj, lj, c);
+            excl = warp_excl_scan(len, lane, total);
+            f0 = 0;
+        }
+        const int f = f0 + lane;
+        f0 += 32;
+        const int j = owner(excl, f);
+        h = __shfl_sync(0xffffffffu, hc, j);
+        k = __shfl_sync(0xffffffffu, kc, j);
+        l = __shfl_sync(0xffffffffu, l0, j) + f - __shfl_sync(0xffffffffu, excl, j);
+        pass = false;
+        if (f < total) {
+            const double hkl[3] = {(double)h, (double)k, (double)l};
+            bool in = true;
+            double d2 = 0., c = 0.;
+            const double G = -Hp->lo, rmax = Hp->rmax;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                c = wp->ub[3 * r] * hkl[0] + wp->ub[3 * r + 1] * hkl[1] +
+                                 wp->ub[3 * r + 2] * hkl[2];
+                const double wr = wp->w[r];
+                in = in && (c - wr <= G) && (c + wr >= -G);
+                const double e = fmax(fabs(c) - wr, 0.);
+                d2 += e * e;
+            }
+            pass = in && d2 <= rmax * rmax * (1. + 1e-9);
+            // every point is in one slab: the same operations on the same values
+            // whichever work item asks
+            if (slabs > 1 && pass)
+                pass = slab == (int)fmin(fmax((c + G) * ((0.5 * slabs) / G), 0.), slabs - 1.);
+        }
+        return true;
+    }
+
+    // The column's l range cut to the lattice points that can be in the slab
+    // (one l and the rounding of the cut wider; next() decides).
+    __device__ __forceinline__ void clip_to_slab(const volatile WarpPlan* wp, double G, int& len) {
+        const double bz = wp->ub[8], az = wp->ub[6] * hc + wp->ub[7] * kc;
+        const double dz = 2. * G / slabs;
+        const double z0 = slab == 0 ? -INFINITY : -G + slab * dz;
+        const double z1 = slab == slabs - 1 ? INFINITY : -G + (slab + 1) * dz;
+        const double a = (z0 - az) / bz, b = (z1 - az) / bz;
+        const double more = 1. + 1e-14 * (fabs(az) + G) / fabs(bz);
+        const double lo = fmin(a, b) - more, hi = fmax(a, b) + more;
+        const double la = l0, lb = l0 + len - 1;
+        // (a NaN bound, for bz = 0, cuts nothing)
+        const double na = lo > la ? ceil(lo) : la, nb = hi < lb ? floor(hi) : lb;
+        if (na > nb) {
+            len = 0;
+        } else {
+            l0 = (int)na;
+            len = (int)(nb - na) + 1;
         }
     }
-}
+};
 
 // host helpers defined in gvec_grid.cu
 int num_sms();
 unsigned grid_for(int64_t items, int per);
 int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st);
 int score_parts(int64_t m);
+Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells);
 bool grid_dims_ok(int32_t nx, int32_t xsub);
 
 }  // namespace grid

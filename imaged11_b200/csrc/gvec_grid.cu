@@ -24,6 +24,8 @@
 // scored by a plain scan of every regular g; g-vectors outside the regular
 // range (non-finite or |g_j| > 1024), or outside the cube and ball of radius
 // rmax the index was built for, by a scan over that list.
+#include <algorithm>
+
 #include "grid.cuh"
 
 namespace id11b {
@@ -31,9 +33,8 @@ namespace grid {
 
 // scoring CTAs: warps (one per work item) and the resident CTAs per SM the
 // register budget is compiled for.  Occupancy decides the speed of the
-// latency-bound lookups: 20,000 UBIs x 1.1M g on B200 took 13.0 ms at 8 warps
-// x 2 CTAs (107 registers), 9.9 ms at 8 x 3, 9.5 ms at 2 x 12, 9.4 ms at
-// 1 x 24 (80 registers) and 8.0 ms at 1 x 32 (64 registers, a few spilled).
+// latency-bound lookups: 20,000 grains assigned over 10M g took 9.5 ms at 1 x 24
+// (80 registers) and 8.7 ms at 1 x 32 (64 registers, a few spilled).
 #ifndef ID11B_GRID_WARPS
 #define ID11B_GRID_WARPS 1
 #endif
@@ -235,154 +236,296 @@ k_sort_cells_f32(const int* __restrict__ start, const Header* __restrict__ Hp, d
 // queued the warp runs the 32 lookups together (lookup_batch).  The UBI's plan
 // lives in shared memory, not in registers.
 constexpr int kQueue = 64;
+constexpr int kSeg = 160;    // row segments a warp lists before it scans their g
+constexpr int kMark = 1024;  // g they may start within (one mark bit each)
+// (2 and 2: 20,000 grains assigned over 10M g in 8.7 ms; 4 and 4, which spill more
+// registers, 13.1 ms; 3 and 2 9.7 ms; 2 and 3 8.6 ms but refinement 1.35 -> 1.44 ms)
+constexpr int kRowsAhead = 2;  // rows of cells whose bounds a lane loads together
+constexpr int kGAhead = 2;     // steps of 32 g whose loads are in flight together
 
-// Per-warp scratch for one batch of up to 32 lookups.
+// Per-warp scratch of the lookups.
 struct Batch {
-    double c[32][3];
+    float4 c[32];                 // centres of the boxes being looked up
     unsigned long long hkl[32];
-    int ix0[32], ix1[32], iy0[32], ny[32], iz0[32];
-    // g found inside a box, waiting for the FP64 evaluation (32 at a time)
-    double cg[64][3];
-    unsigned long long ch[64];
-    int cp[64];
-    int cn;
+    int2 seg[kSeg];               // rows of cells with g: (first position - prefix, box)
+    unsigned mark[kMark / 32];    // a bit at each segment's prefix
+    float u[9];                   // the UBI in FP32
+    // g that passed the screen, waiting for the FP64 evaluation (32 at a time)
+    unsigned long long ch[32 * (kGAhead + 1)];
+    int cp[32 * (kGAhead + 1)];
+    float cs[32 * (kGAhead + 1)];  // its FP32 screening value
 };
 
-// Evaluate the first `take` waiting candidates (one per lane) in the
+// How far the FP32 screening vector UBI32.(g32 - c32) of a g can be from its
+// exact UBI.g - hkl (c: the box's centre UB.hkl), in the 2-norm: a g of exact
+// drlv2 below t^2 has a screening value below (t + margin)^2 (1 + 1e-6).
+// Each component of the screened vector is within
+//   E = eps S (2 G + W) + 5 eps S |g - c|,  |g - c| <= 2 (G + W),  eps = 2^-24
+// of UBI.(g - c): g and c rounded to FP32, then UBI rounded, the difference and
+// three roundings of partial sums (S: largest row sum of |UBI|, G: largest |g_j|,
+// W: largest half width); 1e-6 covers the FP64 rounding of UB.hkl, as in the
+// half widths.  NaN (every g of the cells is evaluated) where FP32 could
+// overflow or lose denormals.
+__device__ __forceinline__ float screen_margin(const volatile WarpPlan* wp, double G) {
+    double S = 0., W = 0.;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        S = fmax(S, fabs(wp->u[3 * r]) + fabs(wp->u[3 * r + 1]) + fabs(wp->u[3 * r + 2]));
+        W = fmax(W, wp->w[r]);
+    }
+    const double E = 5.9604644775390625e-08 * S * (12. * G + 11. * W);
+    const double m = kHklMargin + 1.75 * E;  // > sqrt(3) E
+    if (!(S < 1e15) || !(G > 1e-15) || !(m < 1e15)) return __int_as_float(0x7fc00000);
+    return __double2float_ru(m * (1. + 1e-6));
+}
+
+// The screening value from which a g's exact drlv2 cannot be below t^2.
+__device__ __forceinline__ float screen_limit(float t, float margin) {
+    const float r = t + margin;  // the factor covers its rounding and the squares'
+    return r * r * (1.f + 4e-6f);
+}
+
+// Evaluate the last `take` waiting candidates (one per lane) in the
 // reference's FP64 arithmetic, hand them to act, and drop them from the list.
 template <class Act>
-__device__ __forceinline__ void eval_candidates(const volatile WarpPlan* wp, Batch* bt, int take,
-                                                int lane, Act& act) {
-    if (lane < take) {
+__device__ __forceinline__ void eval_candidates(const volatile WarpPlan* wp, Batch* bt, int first,
+                                                int take, int lane, const double* __restrict__ gs,
+                                                Act& act) {
+    const int pos = lane < take ? bt->cp[first + lane] : 0;
+    if (lane < take && act.want(pos, bt->cs[first + lane])) {
         double u[9], ih[3], hkl[3];
+        const double g[3] = {__ldg(gs + 3 * (int64_t)pos), __ldg(gs + 3 * (int64_t)pos + 1),
+                             __ldg(gs + 3 * (int64_t)pos + 2)};
 #pragma unroll
         for (int e = 0; e < 9; e++) u[e] = wp->u[e];
-        const double g[3] = {bt->cg[lane][0], bt->cg[lane][1], bt->cg[lane][2]};
         const double sv = drlv2_exact(u, g[0], g[1], g[2], ih);
-        unpack_hkl(bt->ch[lane], hkl);
-        act(bt->cp[lane], sv, ih[0] == hkl[0] && ih[1] == hkl[1] && ih[2] == hkl[2], g, ih);
+        unpack_hkl(bt->ch[first + lane], hkl);
+        act(pos, sv, ih[0] == hkl[0] && ih[1] == hkl[1] && ih[2] == hkl[2], g, ih);
     }
-    __syncwarp();
-    const int rest = bt->cn - take;  // < 32
-    double a = 0., b = 0., c = 0.;
-    unsigned long long h = 0;
-    int q = 0;
-    if (lane < rest) {
-        a = bt->cg[take + lane][0];
-        b = bt->cg[take + lane][1];
-        c = bt->cg[take + lane][2];
-        h = bt->ch[take + lane];
-        q = bt->cp[take + lane];
-    }
-    __syncwarp();
-    if (lane < rest) {
-        bt->cg[lane][0] = a;
-        bt->cg[lane][1] = b;
-        bt->cg[lane][2] = c;
-        bt->ch[lane] = h;
-        bt->cp[lane] = q;
-    }
-    __syncwarp();
-    if (lane == 0) bt->cn = rest;
     __syncwarp();
 }
 
-// The lookups of `take` queued hkl (slot = lane), warp-cooperatively: the
-// cell rows of all of them are flattened across the lanes, then the g of
-// each 32 rows, so the lanes stay converged whatever the per-query sizes.
-// Every g inside a box is evaluated in the reference's FP64 arithmetic and
-// handed to act(pos, drlv2, own, g, ih), own = (ih, the rounded h, == the
-// box's hkl).
+// The g of the listed segments (`total` of them), 32 at a time, screened in
+// FP32 against the UBI and the box they were found for; those below the limit
+// wait for the FP64 evaluation (whole warps of them are evaluated here; `cn`
+// of them wait).  A step's segments are found from the mark bits: the number
+// of marks up to a lane's g is its segment.
+template <class Act>
+__device__ __forceinline__ void scan_segments(const volatile WarpPlan* wp, Batch* bt, int total,
+                                              bool last, float limit, int& cn, int lane,
+                                              const double* __restrict__ gs,
+                                              const float4* __restrict__ g4, Act& act) {
+    __syncwarp();  // segments and marks written
+    const unsigned le = 0xffffffffu >> (31 - lane);
+    int rank0 = -1;
+    for (int f0 = 0; f0 < total || last; f0 += 32 * kGAhead) {
+        float4 v[kGAhead];
+        int pos[kGAhead], box[kGAhead];
+#pragma unroll
+        for (int q = 0; q < kGAhead; q++) {
+            const int word = (f0 >> 5) + q;
+            const unsigned mk = word < kMark / 32 ? bt->mark[word] : 0u;
+            const int2 sg = bt->seg[max(rank0 + __popc(mk & le), 0)];
+            rank0 += __popc(mk);
+            const int f = f0 + 32 * q + lane;
+            pos[q] = f < total ? f + sg.x : -1;
+            box[q] = sg.y;
+            if (f < total) v[q] = __ldg(g4 + f + sg.x);
+        }
+#pragma unroll
+        for (int q = 0; q < kGAhead; q++) {
+            bool in = false;
+            float s = 0.f;
+            if (pos[q] >= 0) {
+                const float4 c = bt->c[box[q]];
+                const float ex = v[q].x - c.x, ey = v[q].y - c.y, ez = v[q].z - c.z;
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const float d = fmaf(bt->u[3 * r + 2], ez,
+                                         fmaf(bt->u[3 * r + 1], ey, bt->u[3 * r] * ex));
+                    s = fmaf(d, d, s);
+                }
+                in = !(s >= limit);
+            }
+            const unsigned mk = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                const int slot = cn + __popc(mk & (le >> 1));
+                bt->ch[slot] = bt->hkl[box[q]];
+                bt->cp[slot] = pos[q];
+                bt->cs[slot] = s;
+            }
+            cn += __popc(mk);
+        }
+        __syncwarp();
+        const bool all = last && f0 + 32 * kGAhead >= total;
+        while (cn >= 32 || (all && cn > 0)) {
+            const int take = min(cn, 32);
+            cn -= take;
+            eval_candidates(wp, bt, cn, take, lane, gs, act);
+        }
+        if (all) break;
+    }
+    if (lane < kMark / 32) bt->mark[lane] = 0u;
+    __syncwarp();
+}
+
+// The lookups of `take` queued hkl, one box per lane.  Each lane loads the
+// bounds of its box's rows of cells kRowsAhead at a time and lists the rows
+// that hold g as segments of one run of g over the warp; when the list is full
+// (and after the last row) the run is scanned, so the lanes stay converged
+// whatever the boxes' sizes.  Every g within the screen's limit goes to the
+// reference's FP64 arithmetic and to act(pos, drlv2, own, g, ih), own = (ih,
+// the rounded h, == the box's hkl).  last: the warp's last lookups; the
+// candidates still waiting are evaluated too.
+//
+// Bound: latency of the dependent loads (row bounds, then g) and issue.  The
+// g come from the FP32 copy (one 16-byte load instead of three of 8), the
+// screen is the ellipsoid's (half the box's volume) and costs FP32
+// instructions, and only what passes it is read and evaluated in FP64.  20,000
+// UBIs scored at three tolerances over 1.1M g: 6.95 -> 6.1 ms; over 10.2M g at
+// one: 11.6 -> 8.7 ms; 2,000 refined over 1.1M g: 0.49 -> 0.38 ms a round.
 template <class Act>
 __device__ __forceinline__ void lookup_batch(const volatile WarpPlan* wp, Batch* bt,
-                                             const unsigned long long* q_w, int take, int lane,
-                                             const Header& H, const int* __restrict__ start,
-                                             const double* __restrict__ gs, Act& act) {
-    int nrows = 0;
+                                             const unsigned long long* q_w, int take, bool last,
+                                             float limit, int& cn, int lane,
+                                             const Header* __restrict__ Hp,
+                                             const int* __restrict__ start,
+                                             const double* __restrict__ gs,
+                                             const float4* __restrict__ g4, Act& act) {
+    int left = 0, ny = 1, ry = 0, ix1 = 0;
+    const int* row = start;  // bounds of the lane's current row, at its first x cell
+    const int nx = Hp->nx, nxx = Hp->nxx;
     if (lane < take) {
+        Header H;
+        H.lo = Hp->lo;
+        H.inv_cs = Hp->inv_cs;
+        H.inv_csx = Hp->inv_csx;
+        H.nx = nx;
+        H.nxx = nxx;
         const unsigned long long q = q_w[lane];
         double hkl[3], c[3];
         unpack_hkl(q, hkl);
 #pragma unroll
-        for (int r = 0; r < 3; r++) {
+        for (int r = 0; r < 3; r++)
             c[r] = wp->ub[3 * r] * hkl[0] + wp->ub[3 * r + 1] * hkl[1] + wp->ub[3 * r + 2] * hkl[2];
-            bt->c[lane][r] = c[r];
-        }
+        bt->c[lane] = make_float4(__double2float_rn(c[0]), __double2float_rn(c[1]),
+                                  __double2float_rn(c[2]), 0.f);
         bt->hkl[lane] = q;
-        const int iy0 = coord(c[1] - wp->w[1], H), iy1 = coord(c[1] + wp->w[1], H);
-        const int iz0 = coord(c[2] - wp->w[2], H), iz1 = coord(c[2] + wp->w[2], H);
-        bt->ix0[lane] = coord_x(c[0] - wp->w[0], H);
-        bt->ix1[lane] = coord_x(c[0] + wp->w[0], H);
-        bt->iy0[lane] = iy0;
-        bt->ny[lane] = iy1 - iy0 + 1;
-        bt->iz0[lane] = iz0;
-        nrows = (iy1 - iy0 + 1) * (iz1 - iz0 + 1);
+        const int iy0 = coord(c[1] - wp->w[1], H), iz0 = coord(c[2] - wp->w[2], H);
+        const int ix0 = coord_x(c[0] - wp->w[0], H);
+        ny = coord(c[1] + wp->w[1], H) - iy0 + 1;
+        left = ny * (coord(c[2] + wp->w[2], H) - iz0 + 1);
+        ix1 = coord_x(c[0] + wp->w[0], H) + 1 - ix0;
+        row = start + ((int64_t)iz0 * nx + iy0) * nxx + ix0;
     }
-    __syncwarp();
-    int rtotal;
-    const int rexcl = warp_excl_scan(nrows, lane, rtotal);
-    const double w0 = wp->w[0], w1 = wp->w[1], w2 = wp->w[2];
-    for (int r0 = 0; r0 < rtotal; r0 += 32) {
-        const int rf = r0 + lane;
-        const int qj = owner(rexcl, rf);
-        const int rr = rf - __shfl_sync(0xffffffffu, rexcl, qj);
-        int st = 0, len = 0;
-        if (rf < rtotal) {
-            const int ny = bt->ny[qj];
-            const int iy = bt->iy0[qj] + rr % ny, iz = bt->iz0[qj] + rr / ny;
-            const int64_t row = ((int64_t)iz * H.nx + iy) * H.nxx;
-            st = __ldg(start + row + bt->ix0[qj]);
-            len = __ldg(start + row + bt->ix1[qj] + 1) - st;
+    int total = 0, nseg = 0;  // listed (uniform)
+    int st[kRowsAhead], len[kRowsAhead];
+#pragma unroll
+    for (int k = 0; k < kRowsAhead; k++) st[k] = len[k] = 0;
+    bool have = false;  // rows loaded and not listed yet (uniform)
+    for (;;) {
+        if (!have) {
+            if (__any_sync(0xffffffffu, left > 0)) {
+#pragma unroll
+                for (int k = 0; k < kRowsAhead; k++) {
+                    st[k] = len[k] = 0;
+                    if (k < left) {
+                        st[k] = __ldg(row);
+                        len[k] = __ldg(row + ix1);
+                        row += nxx;
+                        if (++ry == ny) {
+                            ry = 0;
+                            row += (int64_t)(nx - ny) * nxx;
+                        }
+                    }
+                }
+                left -= kRowsAhead;
+#pragma unroll
+                for (int k = 0; k < kRowsAhead; k++) len[k] -= st[k];
+                have = true;
+            }
         }
-        int gtotal;
-        const int gexcl = warp_excl_scan(len, lane, gtotal);
-        const int off = st - gexcl;
-        for (int f0 = 0; f0 < gtotal; f0 += 32) {
-            const int f = f0 + lane;
-            const int rj = owner(gexcl, f);
-            const int pos = f + __shfl_sync(0xffffffffu, off, rj);
-            const int qq = __shfl_sync(0xffffffffu, qj, rj);
-            bool inb = false;
-            double g0 = 0., g1 = 0., g2 = 0.;
-            if (f < gtotal) {
-                g0 = __ldg(gs + 3 * (int64_t)pos);
-                g1 = __ldg(gs + 3 * (int64_t)pos + 1);
-                g2 = __ldg(gs + 3 * (int64_t)pos + 2);
-                inb = fabs(g0 - bt->c[qq][0]) <= w0 && fabs(g1 - bt->c[qq][1]) <= w1 &&
-                      fabs(g2 - bt->c[qq][2]) <= w2;
+        bool full = !have;
+        if (have) {
+            // prefixes of g (low half) and segments (high half) over the lanes
+            unsigned long long own = 0;
+#pragma unroll
+            for (int k = 0; k < kRowsAhead; k++)
+                own += ((unsigned long long)(len[k] > 0) << 32) + (unsigned)min(len[k], kMark + 1);
+            unsigned long long incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
             }
-            const unsigned mk = __ballot_sync(0xffffffffu, inb);
-            const int cn = bt->cn;  // < 32 here
-            if (inb) {
-                const int slot = cn + __popc(mk & ((1u << lane) - 1u));
-                bt->cg[slot][0] = g0;
-                bt->cg[slot][1] = g1;
-                bt->cg[slot][2] = g2;
-                bt->ch[slot] = bt->hkl[qq];
-                bt->cp[slot] = pos;
+            const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
+            const int asum = (int)(unsigned)all, acnt = (int)(all >> 32);
+            if (acnt <= kSeg - nseg && asum <= kMark - total) {
+                int at = total + (int)(unsigned)(incl - own);
+                int slot = nseg + (int)((incl - own) >> 32);
+#pragma unroll
+                for (int k = 0; k < kRowsAhead; k++)
+                    if (len[k] > 0) {
+                        bt->seg[slot++] = make_int2(st[k] - at, lane);
+                        atomicOr(bt->mark + (at >> 5), 1u << (at & 31));
+                        at += len[k];
+                    }
+                total += asum;
+                nseg += acnt;
+                have = false;
+            } else if (total > 0) {
+                full = true;
+            } else {  // more g than the marks hold: the first segment by itself
+                const unsigned m = __ballot_sync(0xffffffffu, own > 0);
+                const int j = __ffs(m) - 1;
+                int n = 0;
+                if (lane == j) {
+#pragma unroll
+                    for (int k = kRowsAhead - 1; k >= 0; k--)
+                        if (len[k] > 0) n = len[k];
+                    bool first = true;
+#pragma unroll
+                    for (int k = 0; k < kRowsAhead; k++)
+                        if (first && len[k] > 0) {
+                            bt->seg[0] = make_int2(st[k], lane);
+                            len[k] = 0;
+                            first = false;
+                        }
+                    bt->mark[0] = 1u;
+                }
+                total = __shfl_sync(0xffffffffu, n, j);
+                nseg = 1;
+                full = true;
             }
-            __syncwarp();
-            if (lane == 0) bt->cn = cn + __popc(mk);
-            __syncwarp();
-            if (cn + __popc(mk) >= 32) eval_candidates(wp, bt, 32, lane, act);
+        }
+        if (full) {  // the list is full, or the last row is listed
+            const bool done = !have;
+            if (total > 0 || (done && last))
+                scan_segments(wp, bt, total, done && last, limit, cn, lane, gs, g4, act);
+            total = nseg = 0;
+            if (done) break;
         }
     }
     __syncwarp();
 }
 
-// Every (UBI, g) pair of work item `part` of `parts` whose drlv2 can be below
-// the plan's tolerance goes to act(pos, drlv2, own, g, ih): through the hkl lookup
+// Every (UBI, g) pair of the work item whose drlv2 can be below the plan's
+// tolerance (tmax) goes to act(pos, drlv2, own, g, ih): through the hkl lookup
 // when ok, else by a plain scan of the regular g (own = true: each g once).
+// act.want(pos, s), called first, says whether a g of FP32 screening value s
+// (within `margin` of the exact one, screen_margin) is of interest.
 template <class Act>
 __device__ __forceinline__ void walk(volatile WarpPlan* wp, Batch* bt, unsigned long long* q_w,
-                                     bool ok, int part, int parts, int lane, const Header& H,
-                                     int64_t nreg, const int* __restrict__ start,
-                                     const double* __restrict__ gs, Act& act) {
+                                     bool ok, const Item& it, double tmax, float margin, int lane,
+                                     const Header* __restrict__ Hp, int64_t nreg,
+                                     const int* __restrict__ start,
+                                     const double* __restrict__ gs,
+                                     const float4* __restrict__ g4, Act& act) {
     if (!ok) {
         double u[9];
 #pragma unroll
         for (int e = 0; e < 9; e++) u[e] = wp->u[e];
-        for (int64_t f = (int64_t)part * 32 + lane; f < nreg; f += 32 * (int64_t)parts) {
+        for (int64_t f = (int64_t)it.part * 32 + lane; f < nreg; f += 32 * (int64_t)it.slabs * it.cols) {
             double ih[3];
             const double g[3] = {gs[3 * f], gs[3 * f + 1], gs[3 * f + 2]};
             const double s = drlv2_exact(u, g[0], g[1], g[2], ih);
@@ -390,18 +533,25 @@ __device__ __forceinline__ void walk(volatile WarpPlan* wp, Batch* bt, unsigned 
         }
         return;
     }
-    int qn = 0;  // queued (uniform)
-    if (lane == 0) bt->cn = 0;
+    int qn = 0, cn = 0;  // hkl queued, candidates waiting (uniform)
+    const float limit = screen_limit(__double2float_ru(tmax), margin);
+    if (lane < 9) bt->u[lane] = __double2float_rn(wp->u[lane]);
+    if (lane < kMark / 32) bt->mark[lane] = 0u;
     __syncwarp();
     const unsigned lt = (1u << lane) - 1u;
-    auto queue = [&](bool pass, int hj, int kj, int lj, const double*) {
-        const unsigned mask = __ballot_sync(0xffffffffu, pass);
-        if (pass) q_w[qn + __popc(mask & lt)] = pack_hkl(hj, kj, lj);
+    BoxWalk bw(wp, it);
+    for (;;) {
+        int h, k, l;
+        bool pass;
+        const bool more = bw.next(wp, Hp, lane, pass, h, k, l);
+        const unsigned mask = __ballot_sync(0xffffffffu, more && pass);
+        if (more && pass) q_w[qn + __popc(mask & lt)] = pack_hkl(h, k, l);
         qn += __popc(mask);
         __syncwarp();
-        if (qn >= 32) {
-            lookup_batch(wp, bt, q_w, 32, lane, H, start, gs, act);
-            const int rest = qn - 32;
+        if (qn >= 32 || !more) {
+            const int take = min(qn, 32);
+            lookup_batch(wp, bt, q_w, take, !more, limit, cn, lane, Hp, start, gs, g4, act);
+            const int rest = qn - take;
             unsigned long long v = 0;
             if (lane < rest) v = q_w[32 + lane];
             __syncwarp();
@@ -409,28 +559,36 @@ __device__ __forceinline__ void walk(volatile WarpPlan* wp, Batch* bt, unsigned 
             __syncwarp();
             qn = rest;
         }
-    };
-    enumerate_boxes(wp, part, parts, lane, H, queue);
-    if (qn > 0) lookup_batch(wp, bt, q_w, qn, lane, H, start, gs, act);
-    const int cn = bt->cn;
-    if (cn > 0) eval_candidates(wp, bt, cn, lane, act);
+        if (!more) break;
+    }
 }
+
+// An act that wants every g the screen lets through.
+template <class F>
+struct EveryG {
+    F& f;
+    __device__ __forceinline__ bool want(int, float) const { return true; }
+    __device__ __forceinline__ void operator()(int pos, double s, bool own, const double* g,
+                                               const double* ih) const {
+        f(pos, s, own, g, ih);
+    }
+};
 
 template <int NT>
 __global__ void __launch_bounds__(kST, ID11B_GRID_MINB)
-k_score(const double* __restrict__ ubis, int64_t m, int parts, Header* __restrict__ Hp,
-        const int* __restrict__ start, const double* __restrict__ gs, Tols tols,
+k_score(const double* __restrict__ ubis, int64_t m, Split sp, Header* __restrict__ Hp,
+        const int* __restrict__ start, const double* __restrict__ gs,
+        const float4* __restrict__ g4, Tols tols,
         int* __restrict__ pcnt, double* __restrict__ psum) {
     __shared__ unsigned long long s_q[kSW][kQueue];
     __shared__ WarpPlan s_plan[kSW];
     __shared__ Batch s_batch[kSW];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t wk = ((int64_t)blockIdx.x * kST + threadIdx.x) >> 5;
-    if (wk >= m * parts) return;  // uniform per warp
-    const int64_t i = wk / parts;
-    const int part = (int)(wk % parts);
-    const Header H = *Hp;
-    const int64_t nreg = start[H.ncells];
+    if (wk >= m * sp.parts()) return;  // uniform per warp
+    const Item it = sp.item(wk, m);
+    const int64_t i = it.i;
+    const int64_t nreg = start[Hp->ncells];
     double t2[NT];
     double tmax = 0.;
     int cnt[NT];
@@ -443,8 +601,8 @@ k_score(const double* __restrict__ ubis, int64_t m, int parts, Header* __restric
         sum[j] = 0.;
     }
     unsigned long long tested = 0;
-    const bool ok = setup_plan(s_plan + w, ubis, i, tmax, H, nreg, lane);
-    auto act = [&](int, double s, bool own, const double*, const double*) {
+    const bool ok = setup_plan(s_plan + w, ubis, i, tmax, *Hp, nreg, lane);
+    auto count = [&](int, double s, bool own, const double*, const double*) {
         tested++;
         if (own) {
 #pragma unroll
@@ -455,15 +613,17 @@ k_score(const double* __restrict__ ubis, int64_t m, int parts, Header* __restric
                 }
         }
     };
-    walk(s_plan + w, s_batch + w, s_q[w], ok, part, parts, lane, H, nreg, start, gs, act);
-    if (!ok && part == 0 && lane == 0) atomicAdd(&Hp->nfallback, 1ull);
+    EveryG<decltype(count)> act{count};
+    walk(s_plan + w, s_batch + w, s_q[w], ok, it, tmax, screen_margin(s_plan + w, -Hp->lo), lane,
+         Hp, nreg, start, gs, g4, act);
+    if (!ok && it.part == 0 && lane == 0) atomicAdd(&Hp->nfallback, 1ull);
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         const int cs = warp_sum(cnt[j]);
         const double ss = warp_sum(sum[j]);
         if (lane == 0) {
-            pcnt[(i * parts + part) * NT + j] = cs;
-            psum[(i * parts + part) * NT + j] = ss;
+            pcnt[(i * sp.parts() + it.part) * NT + j] = cs;
+            psum[(i * sp.parts() + it.part) * NT + j] = ss;
         }
     }
     const long long tt = warp_sum((long long)tested);
@@ -554,35 +714,38 @@ __device__ __forceinline__ void lsq_add(double* acc, double s, const double* g,
     acc[16 * 32] += 1.0;
 }
 
-__global__ void __launch_bounds__(kST, ID11B_GRID_MINB)
-k_refine(const double* __restrict__ ubis, int64_t m, int parts, const Header* __restrict__ Hp,
-         const int* __restrict__ start, const double* __restrict__ gs, double tol,
-         double* __restrict__ part_out) {
+// (24 CTAs, what its shared memory allows, with 80 registers: 2,000 UBIs x 1.1M g
+// 0.42 ms a round; compiled for 32 it spills, 0.53 ms)
+__global__ void __launch_bounds__(kST, 24)
+k_refine(const double* __restrict__ ubis, int64_t m, Split sp, const Header* __restrict__ Hp,
+         const int* __restrict__ start, const double* __restrict__ gs,
+         const float4* __restrict__ g4, double tol, double* __restrict__ part_out) {
     __shared__ unsigned long long s_q[kSW][kQueue];
     __shared__ WarpPlan s_plan[kSW];
     __shared__ Batch s_batch[kSW];
     __shared__ double s_lsq[kSW][kLsqF * 32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t wk = ((int64_t)blockIdx.x * kST + threadIdx.x) >> 5;
-    if (wk >= m * parts) return;  // uniform per warp
-    const int64_t i = wk / parts;
-    const int part = (int)(wk % parts);
-    const Header H = *Hp;
-    const int64_t nreg = start[H.ncells];
+    if (wk >= m * sp.parts()) return;  // uniform per warp
+    const Item it = sp.item(wk, m);
+    const int64_t i = it.i;
+    const int64_t nreg = start[Hp->ncells];
     const double t2 = tol * tol;
     double* acc = s_lsq[w] + lane;
 #pragma unroll
     for (int f = 0; f < kLsqF; f++) acc[f * 32] = 0.;
-    const bool ok = setup_plan(s_plan + w, ubis, i, tol, H, nreg, lane);
-    auto act = [&](int, double s, bool own, const double* g, const double* ih) {
+    const bool ok = setup_plan(s_plan + w, ubis, i, tol, *Hp, nreg, lane);
+    auto add = [&](int, double s, bool own, const double* g, const double* ih) {
         if (own && s < t2) lsq_add(acc, s, g, ih);
     };
-    walk(s_plan + w, s_batch + w, s_q[w], ok, part, parts, lane, H, nreg, start, gs, act);
+    EveryG<decltype(add)> act{add};
+    walk(s_plan + w, s_batch + w, s_q[w], ok, it, tol, screen_margin(s_plan + w, -Hp->lo), lane,
+         Hp, nreg, start, gs, g4, act);
     __syncwarp();
 #pragma unroll 1
     for (int f = 0; f < kLsqF; f++) {
         const double v = warp_sum(acc[f * 32]);
-        if (lane == 0) part_out[(i * parts + part) * kLsqF + f] = v;
+        if (lane == 0) part_out[(i * sp.parts() + it.part) * kLsqF + f] = v;
     }
 }
 
@@ -654,23 +817,23 @@ k_refine_finish(double* __restrict__ ubis, int64_t m, int parts,
 // reaching it; both passes evaluate the same pairs with the same arithmetic.
 template <int PASS>
 __global__ void __launch_bounds__(kST, ID11B_GRID_MINB)
-k_assign(const double* __restrict__ ubis, int64_t m, int parts, const Header* __restrict__ Hp,
+k_assign(const double* __restrict__ ubis, int64_t m, Split sp, const Header* __restrict__ Hp,
          const int* __restrict__ start, const double* __restrict__ gs,
-         const int* __restrict__ gidx, double tol, const double* __restrict__ drlv2,
+         const float4* __restrict__ g4, const int* __restrict__ gidx, double tol,
+         const double* __restrict__ drlv2,
          unsigned long long* __restrict__ best, int* __restrict__ lab, int64_t base) {
     __shared__ unsigned long long s_q[kSW][kQueue];
     __shared__ WarpPlan s_plan[kSW];
     __shared__ Batch s_batch[kSW];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t wk = ((int64_t)blockIdx.x * kST + threadIdx.x) >> 5;
-    if (wk >= m * parts) return;  // uniform per warp
-    const int64_t i = wk / parts;
-    const int part = (int)(wk % parts);
-    const Header H = *Hp;
-    const int64_t nreg = start[H.ncells];
+    if (wk >= m * sp.parts()) return;  // uniform per warp
+    const Item it = sp.item(wk, m);
+    const int64_t i = it.i;
+    const int64_t nreg = start[Hp->ncells];
     const double t2 = tol * tol;
-    const bool ok = setup_plan(s_plan + w, ubis, i, tol, H, nreg, lane);
-    auto act = [&](int pos, double s, bool own, const double*, const double*) {
+    const bool ok = setup_plan(s_plan + w, ubis, i, tol, *Hp, nreg, lane);
+    auto assign = [&](int pos, double s, bool own, const double*, const double*) {
         if (!own || !(s < t2)) return;
         const int k = __ldg(gidx + pos);
         if (!(s < __ldg(drlv2 + k))) return;
@@ -680,7 +843,111 @@ k_assign(const double* __restrict__ ubis, int64_t m, int parts, const Header* __
         else if (best[k] == b)
             atomicMin(lab + k, (int)(base + i));
     };
-    walk(s_plan + w, s_batch + w, s_q[w], ok, part, parts, lane, H, nreg, start, gs, act);
+    EveryG<decltype(assign)> act{assign};
+    walk(s_plan + w, s_batch + w, s_q[w], ok, it, tol, screen_margin(s_plan + w, -Hp->lo), lane,
+         Hp, nreg, start, gs, g4, act);
+}
+
+// The same in one pass, for grains that are all here: each g's smallest drlv2
+// and the lowest grain reaching it as one 16-byte entry (FP64 bits, grain
+// index), lowered by 128-bit compare-and-swap, so that the order of the grains
+// does not matter.  Entries are kept by sorted position, next to the g the
+// lookups read together, and start at the g's drlv2 on entry (at most tol^2)
+// with grain -1: a tie with it does not replace it.
+//
+// Most pairs below tol^2 lose to a better grain, so each g's current best is
+// also kept as a float rounded up (4 bytes: 40 MB for 10M g, in L2), and a
+// pair whose FP32 screening value cannot be below it is dropped before its
+// FP64 g is read.  The limits only fall, so a stale one drops nothing that
+// would win.
+//
+// Bound: latency and L2 misses of the lookups and the evaluations' random
+// reads.  20,000 grains (true ones, 0.2 degrees off) x 10.2M g, tol 0.05: 8.7 ms,
+// 9.3 for the whole assignment; the lookup it had before in two passes of atomic
+// minima (as k_assign) over every pair, in the caller's g order: 18.8 + 19.1, 38.7 ms.
+struct __align__(16) AssignEntry {
+    unsigned long long bits;
+    long long grain;
+};
+
+__device__ __forceinline__ AssignEntry entry_load(const AssignEntry* p) {
+    AssignEntry e;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\t"
+                 "mov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(e.bits), "=l"(e.grain)
+                 : "l"(p)
+                 : "memory");
+    return e;
+}
+
+__device__ __forceinline__ AssignEntry entry_cas(AssignEntry* p, const AssignEntry& was,
+                                                 const AssignEntry& now) {
+    AssignEntry e;
+    asm volatile("{\n\t.reg .b128 t, a, b;\n\tmov.b128 a, {%3, %4};\n\tmov.b128 b, {%5, %6};\n\t"
+                 "atom.relaxed.gpu.global.cas.b128 t, [%2], a, b;\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(e.bits), "=l"(e.grain)
+                 : "l"(p), "l"(was.bits), "l"(was.grain), "l"(now.bits), "l"(now.grain)
+                 : "memory");
+    return e;
+}
+
+struct AssignAct {
+    AssignEntry* entry;
+    unsigned* limit;  // float bits, rounded up
+    long long grain;
+    float margin;
+
+    __device__ __forceinline__ bool want(int pos, float s) const {
+        return !(s >= screen_limit(__fsqrt_ru(__uint_as_float(__ldcg(limit + pos))), margin));
+    }
+    __device__ __forceinline__ void operator()(int pos, double s, bool own, const double*,
+                                               const double*) const {
+        if (!own || !(s >= 0.)) return;
+        const AssignEntry now{(unsigned long long)__double_as_longlong(s), grain};
+        AssignEntry was = entry_load(entry + pos);
+        while (now.bits < was.bits || (now.bits == was.bits && grain < was.grain)) {
+            const AssignEntry got = entry_cas(entry + pos, was, now);
+            if (got.bits == was.bits && got.grain == was.grain) {
+                atomicMin(limit + pos, __float_as_uint(__double2float_ru(s)));
+                break;
+            }
+            was = got;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kST, ID11B_GRID_MINB)
+k_assign_once(const double* __restrict__ ubis, int64_t m, Split sp,
+              const Header* __restrict__ Hp, const int* __restrict__ start,
+              const double* __restrict__ gs, const float4* __restrict__ g4, double tol,
+              AssignEntry* __restrict__ entry, unsigned* __restrict__ limit) {
+    __shared__ unsigned long long s_q[kSW][kQueue];
+    __shared__ WarpPlan s_plan[kSW];
+    __shared__ Batch s_batch[kSW];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t wk = ((int64_t)blockIdx.x * kST + threadIdx.x) >> 5;
+    if (wk >= m * sp.parts()) return;  // uniform per warp
+    const Item it = sp.item(wk, m);
+    const int64_t nreg = start[Hp->ncells];
+    const bool ok = setup_plan(s_plan + w, ubis, it.i, tol, *Hp, nreg, lane);
+    const float margin = ok ? screen_margin(s_plan + w, -Hp->lo) : 0.f;
+    AssignAct act{entry, limit, (long long)it.i, margin};
+    walk(s_plan + w, s_batch + w, s_q[w], ok, it, tol, margin, lane, Hp, nreg, start, gs, g4, act);
+}
+
+__global__ void __launch_bounds__(kGT)
+k_assign_entries(const int* __restrict__ start, int64_t ncells, const int* __restrict__ gidx,
+                 double tol, const double* __restrict__ drlv2, AssignEntry* __restrict__ entry,
+                 unsigned* __restrict__ limit) {
+    const int64_t nreg = start[ncells];
+    const double t2 = tol * tol;
+    for (int64_t p = (int64_t)blockIdx.x * kGT + threadIdx.x; p < nreg;
+         p += (int64_t)gridDim.x * kGT) {
+        const double d = drlv2[gidx[p]];
+        const double v = d > 0. ? fmin(d, t2) : 0.;  // NaN and values <= 0: no grain is below
+        entry[p] = AssignEntry{(unsigned long long)__double_as_longlong(v), -1};
+        limit[p] = __float_as_uint(__double2float_ru(v));
+    }
 }
 
 constexpr unsigned long long kNoBest = 0x7fffffffffffffffull;
@@ -723,6 +990,26 @@ k_assign_final(const int* __restrict__ start, int64_t ncells, const int* __restr
             labels[k] = gl ? gl[w] : w;
             drlv2[k] = __longlong_as_double((long long)best[k]);
             if (npk) atomicAdd(npk + w, 1);
+        } else if (is_grain_label(labels[k], gl, m)) {
+            labels[k] = -1;
+        }
+    }
+}
+
+// the same from k_assign_once's entries
+__global__ void __launch_bounds__(kGT)
+k_assign_winners(const int* __restrict__ start, int64_t ncells, const int* __restrict__ gidx,
+                 const AssignEntry* __restrict__ entry, const int* __restrict__ gl, int64_t m,
+                 double* __restrict__ drlv2, int* __restrict__ labels, int* __restrict__ npk) {
+    const int64_t nreg = start[ncells];
+    for (int64_t p = (int64_t)blockIdx.x * kGT + threadIdx.x; p < nreg;
+         p += (int64_t)gridDim.x * kGT) {
+        const int k = gidx[p];
+        const AssignEntry e = entry[p];
+        if (e.grain >= 0) {
+            labels[k] = gl ? gl[e.grain] : (int)e.grain;
+            drlv2[k] = __longlong_as_double((long long)e.bits);
+            if (npk) atomicAdd(npk + e.grain, 1);
         } else if (is_grain_label(labels[k], gl, m)) {
             labels[k] = -1;
         }
@@ -795,13 +1082,40 @@ int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st) {
     return ID11B_OK;
 }
 
-// work items (warps) per UBI: enough warps for ~4 waves of 8 warps x 8 CTAs per SM
-int score_parts(int64_t m) {
+// work items (warps) per UBI: about two waves of the resident warps, and two
+// items where there are fewer than about four waves of UBIs.  More items
+// balance better but each sets up the UBI's plan and reduces its sums: 2,000
+// UBIs x 1.1M g refine in 0.39 ms a round at two waves and 0.42 at four, 1,000
+// score in 0.25 and 0.30 ms; 20,000 score in 6.4 ms with one item each, 6.1
+// with two.  A refinement's item also reduces its 17 sums, so it takes the
+// second item only for a second slab of an index past 96 MB: 20,000 UBIs refine
+// in 1.78 ms with one and 2.17 with two over 1.1M g, 13.3 and 11.5 ms over 10.2M.
+static int item_parts(int64_t m, int64_t floor) {
     if (m <= 0) return 1;
-    int64_t want = (int64_t)num_sms() * 64 * 4;
-    int64_t p = (want + m - 1) / m;
-    if (p > kMaxParts) p = kMaxParts;
-    return (int)(p < 1 ? 1 : p);
+    int64_t p = std::max((2 * (int64_t)num_sms() * 64 + m - 1) / m, floor);
+    return (int)std::min<int64_t>(p, kMaxParts);
+}
+
+int score_parts(int64_t m) { return item_parts(m, m < 4 * (int64_t)num_sms() * 64 ? 2 : 1); }
+
+static int refine_parts(int64_t m, int64_t n, int64_t ncells) {
+    return 20 * n + 4 * ncells > (96 << 20) ? score_parts(m) : item_parts(m, 1);
+}
+
+// `parts` work items per UBI as slabs x columns: as many slabs as it takes for a
+// slab's FP32 g, row starts and assignment limits to stay in a part of L2 --
+// at least `parts` items with `more`, else at most.  32 MB: of a 10.2M-g index
+// (250 MB of them), 20,000 grains are assigned in 8.7 ms; one slab 11.8 ms, 96 MB
+// 9.9, 48 MB 9.0, 16 MB 9.2, 12 MB 9.3 (each slab goes through every column).  A
+// 1.1M-g index (52 MB) is two slabs where there are parts to split: 20,000 UBIs
+// score in 6.1 ms, in 6.4 as one.
+Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells) {
+    const double bytes = 20. * (double)n + 4. * (double)ncells;
+    int slabs = (int)fmin(16., ceil(bytes / (32. * 1048576.)));
+    if (slabs < 1) slabs = 1;
+    if (!more && slabs > parts) slabs = parts;
+    while (slabs > 1 && m > INT32_MAX / (2 * (int64_t)slabs)) slabs--;  // one block per item
+    return Split{slabs, more ? (parts + slabs - 1) / slabs : parts / slabs};
 }
 
 }  // namespace grid
@@ -941,22 +1255,23 @@ extern "C" int id11b_dev_score_grid(const double* ubis, int64_t m, const double*
     double* psum = (double*)((char*)ws + al256(sizeof(int) * (size_t)items));
     int* scnt = pcnt + m * parts * ntol;
     double* ssum = psum + m * parts * ntol;
-    const int64_t warps = m * parts;
-    const unsigned blocks = (unsigned)((warps + kSW - 1) / kSW);
+    const Split sp = split_for(parts, false, m, n, (int64_t)nx * nx * nx * xsub);
+    const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     const int* start = (const int*)(b + L.start);
     const double* gs = (const double*)(b + L.g);
+    const float4* g4 = (const float4*)(b + L.g4);
     switch (ntol) {
-        case 1: k_score<1><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, T, pcnt, psum); break;
-        case 2: k_score<2><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, T, pcnt, psum); break;
-        case 3: k_score<3><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, T, pcnt, psum); break;
-        default: k_score<4><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, T, pcnt, psum); break;
+        case 1: k_score<1><<<blocks, kST, 0, st>>>(ubis, m, sp, H, start, gs, g4, T, pcnt, psum); break;
+        case 2: k_score<2><<<blocks, kST, 0, st>>>(ubis, m, sp, H, start, gs, g4, T, pcnt, psum); break;
+        case 3: k_score<3><<<blocks, kST, 0, st>>>(ubis, m, sp, H, start, gs, g4, T, pcnt, psum); break;
+        default: k_score<4><<<blocks, kST, 0, st>>>(ubis, m, sp, H, start, gs, g4, T, pcnt, psum); break;
     }
     ID11B_CHECK_LAUNCH();
     k_score_special<<<(unsigned)((m * 32 + kGT - 1) / kGT), kGT, 0, st>>>(
         ubis, m, ntol, T, gv, (const int*)(b + L.spec), (const int*)(b + L.spos) + n, scnt,
         ssum);
     ID11B_CHECK_LAUNCH();
-    k_score_finish<<<(unsigned)((m + kGT - 1) / kGT), kGT, 0, st>>>(m, parts, ntol, pcnt, psum,
+    k_score_finish<<<(unsigned)((m + kGT - 1) / kGT), kGT, 0, st>>>(m, sp.parts(), ntol, pcnt, psum,
                                                                     scnt, ssum, counts, sums);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
@@ -985,10 +1300,11 @@ extern "C" int id11b_grid_stats(const void* gridbuf, int64_t* nregular, int64_t*
     return ID11B_OK;
 }
 
+// entries (16 bytes) and limits (4) per g
 extern "C" int64_t id11b_assign_workspace_bytes(int64_t n) {
     if (n < 0) return -1;
     const size_t nn = (size_t)(n > 0 ? n : 1);
-    return (int64_t)(al256(sizeof(unsigned long long) * nn) + al256(sizeof(int) * nn));
+    return (int64_t)(al256(sizeof(AssignEntry) * nn) + al256(sizeof(unsigned) * nn));
 }
 
 extern "C" int id11b_dev_score_and_assign_grid(const double* ubis, int64_t m,
@@ -1011,22 +1327,19 @@ extern "C" int id11b_dev_score_and_assign_grid(const double* ubis, int64_t m,
     const char* b = (const char*)gridbuf;
     const Header* H = (const Header*)b;
     const int* start = (const int*)(b + L.start);
-    const double* gs = (const double*)(b + L.g);
     const int* gidx = (const int*)(b + L.idx);
-    unsigned long long* best = (unsigned long long*)ws;
-    int* lab = (int*)((char*)ws + al256(sizeof(unsigned long long) * (size_t)n));
-    k_assign_init<<<grid_for(n, kGT), kGT, 0, st>>>(n, best, lab);
+    AssignEntry* entry = (AssignEntry*)ws;
+    unsigned* limit = (unsigned*)((char*)ws + al256(sizeof(AssignEntry) * (size_t)n));
+    k_assign_entries<<<grid_for(n, kGT), kGT, 0, st>>>(start, ncells, gidx, tol, drlv2, entry,
+                                                       limit);
     ID11B_CHECK_LAUNCH();
-    const int parts = score_parts(m);
-    const unsigned blocks = (unsigned)((m * parts + kSW - 1) / kSW);
-    k_assign<0><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, gidx, tol, drlv2, best, lab,
-                                        0);
+    const Split sp = split_for(score_parts(m), true, m, n, ncells);
+    k_assign_once<<<(unsigned)((m * sp.parts() + kSW - 1) / kSW), kST, 0, st>>>(
+        ubis, m, sp, H, start, (const double*)(b + L.g), (const float4*)(b + L.g4), tol, entry,
+        limit);
     ID11B_CHECK_LAUNCH();
-    k_assign<1><<<blocks, kST, 0, st>>>(ubis, m, parts, H, start, gs, gidx, tol, drlv2, best, lab,
-                                        0);
-    ID11B_CHECK_LAUNCH();
-    k_assign_final<<<grid_for(n, kGT), kGT, 0, st>>>(start, ncells, gidx, best, lab, grain_labels,
-                                                     m, drlv2, labels, npk);
+    k_assign_winners<<<grid_for(n, kGT), kGT, 0, st>>>(start, ncells, gidx, entry, grain_labels, m,
+                                                       drlv2, labels, npk);
     ID11B_CHECK_LAUNCH();
     k_assign_special<<<grid_for(n, kGT), kGT, 0, st>>>(ubis, m, gv, (const int*)(b + L.spec),
                                                        (const int*)(b + L.spos) + n, tol,
@@ -1058,18 +1371,21 @@ extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, 
     const Layout L = layout(n, (int64_t)nx * nx * nx * xsub);
     const char* b = (const char*)gridbuf;
     const Header* H = (const Header*)b;
-    const int parts = score_parts(m);
-    const unsigned blocks = (unsigned)((m * parts + kSW - 1) / kSW);
+    const int64_t ncells = (int64_t)nx * nx * nx * xsub;
+    const int parts = refine_parts(m, n, ncells);
+    const Split sp = split_for(parts, false, m, n, ncells);
+    const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     double* part = (double*)ws;
     for (int it = 0; it < iters; it++) {
-        k_refine<<<blocks, kST, 0, st>>>(ubis, m, parts, H, (const int*)(b + L.start),
-                                         (const double*)(b + L.g), tol, part);
+        k_refine<<<blocks, kST, 0, st>>>(ubis, m, sp, H, (const int*)(b + L.start),
+                                         (const double*)(b + L.g), (const float4*)(b + L.g4), tol,
+                                         part);
         ID11B_CHECK_LAUNCH();
         double* spart = part + m * parts * kLsqF;
         k_refine_special<<<(unsigned)((m * 32 + kGT - 1) / kGT), kGT, 0, st>>>(
             ubis, m, tol, gv, (const int*)(b + L.spec), (const int*)(b + L.spos) + n, spart);
         ID11B_CHECK_LAUNCH();
-        k_refine_finish<<<(unsigned)((m + kGT - 1) / kGT), kGT, 0, st>>>(ubis, m, parts, part,
+        k_refine_finish<<<(unsigned)((m + kGT - 1) / kGT), kGT, 0, st>>>(ubis, m, sp.parts(), part,
                                                                          spart, npk, mean);
         ID11B_CHECK_LAUNCH();
     }
@@ -1101,17 +1417,19 @@ extern "C" int id11b_dev_assign_grid_pass(const double* ubis, int64_t m, int64_t
     if (m == 0) return ID11B_OK;
     const Layout L = layout(n, (int64_t)nx * nx * nx * xsub);
     const char* b = (const char*)gridbuf;
-    const int parts = score_parts(m);
-    const unsigned blocks = (unsigned)((m * parts + kSW - 1) / kSW);
+    const Split sp = split_for(score_parts(m), true, m, n, (int64_t)nx * nx * nx * xsub);
+    const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     if (pass == 0)
-        k_assign<0><<<blocks, kST, 0, st>>>(ubis, m, parts, (const Header*)b,
+        k_assign<0><<<blocks, kST, 0, st>>>(ubis, m, sp, (const Header*)b,
                                             (const int*)(b + L.start), (const double*)(b + L.g),
-                                            (const int*)(b + L.idx), tol, drlv2,
+                                            (const float4*)(b + L.g4), (const int*)(b + L.idx),
+                                            tol, drlv2,
                                             (unsigned long long*)best, lab, index_base);
     else
-        k_assign<1><<<blocks, kST, 0, st>>>(ubis, m, parts, (const Header*)b,
+        k_assign<1><<<blocks, kST, 0, st>>>(ubis, m, sp, (const Header*)b,
                                             (const int*)(b + L.start), (const double*)(b + L.g),
-                                            (const int*)(b + L.idx), tol, drlv2,
+                                            (const float4*)(b + L.g4), (const int*)(b + L.idx),
+                                            tol, drlv2,
                                             (unsigned long long*)best, lab, index_base);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;

@@ -1,0 +1,68 @@
+"""Edges of the cell-index lookup (scoring, refinement, assignment): rows of
+cells holding more g than a warp lists at once, more rows than it lists, indexes
+split into slabs, and the starting drlv2 values of the assignment -- against the
+oracle.  Counts, labels and drlv2 must be identical; refined UBIs are FP64 sums
+in another order: 1e-11 of the UBI's largest element, as for the index's other
+refinement tests."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def scene():
+    from imaged11_b200 import synth
+    ps = synth.simulate(60, "Al", gmax=1.3, seed=91, noise_frac=0.10)
+    rng = np.random.default_rng(92)
+    u = synth.trial_ubis(ps.ubis, 60, 0.5, 0.2, rng)
+    u[3] = 0.0                      # singular: plain scan
+    u[7] = u[5]                     # a tie
+    return ps.gv, u
+
+
+# cell side, x cells per side, g kept: one row of 24,000 g (longer than the
+# marks), few long rows, many rows of few g (three boxes' rows fill the list),
+# 65M cells (eight slabs) and a ragged 1,000-g index
+@pytest.mark.parametrize("cell,xsub,n", [(10.0, 1, None), (1.0, 1, None), (0.3, 2, 20001),
+                                         (0.006, 1, None), (0.0275, 16, None), (0.05, 4, 1000)])
+@pytest.mark.parametrize("tol", [0.03, 0.25])
+def test_rows_and_slabs(scene, oracle, cell, xsub, n, tol, cuda):
+    from imaged11_b200 import batch
+    gv, u = scene
+    g = gv[:n]
+    grid = batch.GvecGrid(g, cell=cell, xsub=xsub)
+    assert np.array_equal(
+        batch.score_grid(u, grid, [tol, 0.6], method="walk").cpu().numpy(),
+        oracle.score_many(u, g, [tol, 0.6]))
+    d = np.zeros(len(g)) + 2
+    lab = np.zeros(len(g), np.int32) - 1
+    rd, rl = d.copy(), lab.copy()
+    for i, x in enumerate(u):
+        _, rd, rl = oracle.score_and_assign(x, g, tol, rd, rl, i)
+    batch.score_and_assign_grid(u, grid, tol, d, lab)
+    assert np.array_equal(lab, rl) and np.array_equal(d, rd)
+    ur, npk, mean = (t.cpu().numpy() for t in batch.refine_grid(u[4:12].copy(), grid, tol))
+    for i in range(8):
+        k, m, x = oracle.score_and_refine(u[4 + i], g, tol)
+        assert npk[i] == k and abs(mean[i] - m) <= 1e-12 * m
+        assert np.abs(ur[i] - x).max() <= 1e-11 * np.abs(x).max()
+
+
+def test_assignment_starting_values(scene, oracle, cuda):
+    """drlv2 on entry: NaN, infinities, zeros of both signs, negative, above
+    tol^2, and exactly a grain's drlv2 (not below it: the label stays)."""
+    from imaged11_b200 import batch
+    gv, u = scene
+    n = len(gv)
+    exact = np.zeros(n) + 2
+    _, exact, _ = oracle.score_and_assign(u[5], gv, 0.1, exact, np.zeros(n, np.int32), 1)
+    rng = np.random.default_rng(93)
+    d = rng.choice([np.nan, np.inf, -np.inf, 0.0, -0.0, -1.0, 0.01, 2.0, 1e-9], n)
+    d[::3] = exact[::3]
+    lab = rng.integers(-1, 70, n).astype(np.int32)
+    rd, rl = d.copy(), lab.copy()
+    for i, x in enumerate(u):
+        _, rd, rl = oracle.score_and_assign(x, gv, 0.1, rd, rl, i)
+    batch.score_and_assign_grid(u, batch.GvecGrid(gv), 0.1, d, lab)
+    assert np.array_equal(lab, rl) and np.array_equal(d, rd, equal_nan=True)
