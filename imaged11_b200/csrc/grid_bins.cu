@@ -73,9 +73,6 @@ constexpr int kEW = ID11B_ENUM_WARPS;
 constexpr int kET = 32 * kEW;
 constexpr int kJT = 256;            // threads per join CTA (one row at a time)
 constexpr int kJW = kJT / 32;
-#ifndef ID11B_JOIN_FOLD
-#define ID11B_JOIN_FOLD 1
-#endif
 #ifndef ID11B_JOIN_RANKED
 #define ID11B_JOIN_RANKED 1
 #endif
@@ -208,12 +205,6 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // FP32 form of a UBI's plan for the candidate work of the enumeration.  The
 // half widths are widened by a bound on the FP32 error of the box centre:
 // c = fma(l, ub_r2, fma(k, ub_r1, h * ub_r0)) with ub rounded to FP32 is
@@ -482,9 +473,9 @@ k_rowsplit(const uint64_t* __restrict__ tmp, const int* __restrict__ blkstart, i
     }
 }
 
-// A pair inside a band (or, with sums, any pair below hmax): the reference's
-// exact FP64 drlv2 and whether it belongs to the box's hkl, by value.  Out of
-// line: rare, and its registers would otherwise weigh on the whole join.
+// The reference's exact FP64 drlv2 of a pair and whether it belongs to the
+// box's hkl, by value.  Out of line: its registers would otherwise weigh on
+// the whole join.
 struct Exact {
     double s;   // drlv2
     bool own;   // the rounded h is the box's hkl
@@ -503,90 +494,86 @@ __device__ __noinline__ Exact exact_pair(const double* __restrict__ ubis, int64_
     return r;
 }
 
-// A pair inside a band (or, with sums, any pair below hmax), evaluated
-// exactly: counted for the tolerances its FP64 drlv2 clears under its own hkl
-// (those it cleared in FP32 by more than the band were counted already).
-//
-// AS 1 and 2 (assignment, NT 1, SUMS): the two passes of k_assign
-// (gvec_grid.cu) on the pair -- below tol^2 and below the g's drlv2 on entry,
-// pass 1 takes the smallest drlv2 bits per g, pass 2 the lowest UBI index
-// reaching them.
-template <int NT, bool SUMS, int AS>
+__device__ __forceinline__ void box_hkl(uint64_t rec, float hkf[3]) {
+    hkf[0] = (float)((int)((rec >> kHShift) & 511) - kHklOff);
+    hkf[1] = (float)((int)((rec >> kKShift) & 511) - kHklOff);
+    hkf[2] = (float)((int)((rec >> kLShift) & 511) - kHklOff);
+}
+
+// A pair inside a band of a counting join, evaluated exactly: counted for the
+// tolerances its FP64 drlv2 clears under its own hkl (those it cleared in FP32
+// by more than the band were counted already).
+template <int NT>
 __device__ __forceinline__ void rare_pair(float s, int pos, const JoinParams& P,
                                           const double* __restrict__ ubis, int64_t ubi,
                                           const double* __restrict__ gs, const float* hkf,
-                                          int cnt[NT], unsigned long long sum[NT]) {
+                                          int cnt[NT]) {
     const Exact e = exact_pair(ubis, ubi, gs, pos, hkf[0], hkf[1], hkf[2]);
     if (!e.own) return;
-    if (AS) {
-        if (!(e.s < P.t2[0])) return;
-        const int k = __ldg(P.gidx + pos);
-        if (!(e.s < __ldg(P.d0 + k))) return;
-        const unsigned long long b = (unsigned long long)__double_as_longlong(e.s);
-        if (AS == 1)
-            atomicMin(P.best + k, b);
-        else if (P.best[k] == b)
-            atomicMin(P.lab + k, (int)ubi);
-        return;
-    }
 #pragma unroll
-    for (int j = 0; j < NT; j++) {
-        if (!(e.s < P.t2[j])) continue;
-        if (SUMS) {
-            cnt[j]++;
-            sum[j] += __double2ull_rn(e.s * P.fix);  // per term: order-free
-        } else if (!(s < P.lo[j])) {
-            cnt[j]++;
-        }
-    }
+    for (int j = 0; j < NT; j++)
+        if (e.s < P.t2[j] && !(s < P.lo[j])) cnt[j]++;
 }
+
+// With sums, and for the assignment, every pair below hmax is evaluated
+// exactly.  A lane finds few of them in a run (one or two per box of 16 g
+// screened), so evaluating them where they are found leaves most lanes idle:
+// the warp's pairs of up to 32 g are listed box by box and evaluated 32 at a
+// time, one per lane, and each lane then adds the values of its own box.  At
+// three tolerances with sums the join of 5,003 UBIs x 568k g takes 0.66 ms,
+// 0.98 with each pair evaluated where it was found; all of 20,000 UBIs x 1.1M g
+// 4.2 and 5.0 ms.  (Queuing them over runs and adding each value by global atomics was slower
+// where boxes hold more pairs: 0.68 and 5.4 ms.)
+constexpr int kPend = 96;  // pairs a warp lists at a time
+union Pend {
+    struct {
+        int lane, q;  // box (lane of the run), staged g
+    } pair;
+    double s;         // its drlv2, or infinity where it is not under the box's hkl
+};
 
 struct Staged {  // the tile of staged g, structure of arrays (pairs read as 64 bits)
     const float *x, *y, *z;
     const int* pos;
 };
 
-// The box of one lane against staged g [ga, gb), two at a time with packed
-// f32x2 instructions (lane by lane the operations of drlv2_f32, so every
-// screening value is the scalar one).  The range is widened to even bounds
-// (an odd tile ends with a NaN g): testing g beyond a run's range is harmless,
-// every g of a tile being tested at most once per box.  Counting is free of
-// branches; one branch per pair of g catches the rare band cases.
+// drlv2 of one lane's box against staged g q and q + 1, with packed f32x2
+// instructions (lane by lane the scalar operations): UBI.g - hkl with the
+// subtraction folded into the first FMA (hh holds -hkl), three roundings of
+// partial sums below |hkl| + S gmax.
+__device__ __forceinline__ void screen_pair(const Staged& t, int q, const uint64_t uu[9],
+                                            const uint64_t hh[3], float& sa, float& sb) {
+    const uint64_t gx = *reinterpret_cast<const uint64_t*>(t.x + q);
+    const uint64_t gy = *reinterpret_cast<const uint64_t*>(t.y + q);
+    const uint64_t gz = *reinterpret_cast<const uint64_t*>(t.z + q);
+    const uint64_t d0 = fma2(uu[2], gz, fma2(uu[1], gy, fma2(uu[0], gx, hh[0])));
+    const uint64_t d1 = fma2(uu[5], gz, fma2(uu[4], gy, fma2(uu[3], gx, hh[1])));
+    const uint64_t d2 = fma2(uu[8], gz, fma2(uu[7], gy, fma2(uu[6], gx, hh[2])));
+    upk2(fma2(d2, d2, fma2(d1, d1, mul2(d0, d0))), sa, sb);
+}
+
+// The box of one lane against staged g [ga, gb), counting.  The range is
+// widened to even bounds (an odd tile ends with a NaN g): testing g beyond a
+// run's range is harmless, every g of a tile being tested at most once per
+// box.  Counting is free of branches; one branch per pair of g catches the
+// rare band cases.
 //
 // RANKED (lo and hi both non-decreasing in j): a value below lo_j is below
 // every later lo, so the only band it can lie in is that of the largest lo_j
 // not above it -- one select chain and one compare instead of a test per
 // tolerance.  (If s lies in band i <= J, J the largest j with lo_j <= s, then
 // s < hi_i <= hi_J.)
-template <int NT, bool SUMS, bool RANKED, int AS>
+template <int NT, bool RANKED>
 __device__ __forceinline__ void test_range(const Staged& t, int ga, int gb, const uint64_t uu[9],
                                            const uint64_t hh[3], const float* hkf,
                                            const JoinParams& P, const double* __restrict__ ubis,
                                            int64_t ubi, const double* __restrict__ gs, int cnt[NT],
-                                           unsigned long long sum[NT], unsigned& ntest) {
+                                           unsigned& ntest) {
     for (int q = ga & ~1; q < gb; q += 2) {
-        const uint64_t gx = *reinterpret_cast<const uint64_t*>(t.x + q);
-        const uint64_t gy = *reinterpret_cast<const uint64_t*>(t.y + q);
-        const uint64_t gz = *reinterpret_cast<const uint64_t*>(t.z + q);
-#if ID11B_JOIN_FOLD
-        // UBI.g - hkl with the subtraction folded into the first FMA (hh holds
-        // -hkl): three roundings of partial sums below |hkl| + S gmax
-        const uint64_t d0 = fma2(uu[2], gz, fma2(uu[1], gy, fma2(uu[0], gx, hh[0])));
-        const uint64_t d1 = fma2(uu[5], gz, fma2(uu[4], gy, fma2(uu[3], gx, hh[1])));
-        const uint64_t d2 = fma2(uu[8], gz, fma2(uu[7], gy, fma2(uu[6], gx, hh[2])));
-#else
-        const uint64_t h0 = fma2(uu[2], gz, fma2(uu[1], gy, mul2(uu[0], gx)));
-        const uint64_t h1 = fma2(uu[5], gz, fma2(uu[4], gy, mul2(uu[3], gx)));
-        const uint64_t h2 = fma2(uu[8], gz, fma2(uu[7], gy, mul2(uu[6], gx)));
-        const uint64_t d0 = sub2(h0, hh[0]), d1 = sub2(h1, hh[1]), d2 = sub2(h2, hh[2]);
-#endif
         float sa, sb;
-        upk2(fma2(d2, d2, fma2(d1, d1, mul2(d0, d0))), sa, sb);
+        screen_pair(t, q, uu, hh, sa, sb);
         bool ra, rb;
-        if (SUMS) {
-            ra = sa < P.hmax;
-            rb = sb < P.hmax;
-        } else if (RANKED) {
+        if (RANKED) {
             bool ia[NT], ib[NT];
 #pragma unroll
             for (int j = 0; j < NT; j++) {
@@ -614,10 +601,100 @@ __device__ __forceinline__ void test_range(const Staged& t, int ga, int gb, cons
         }
         if (ra || rb) {
             ntest += (unsigned)ra + (unsigned)rb;
-            if (ra) rare_pair<NT, SUMS, AS>(sa, t.pos[q], P, ubis, ubi, gs, hkf, cnt, sum);
-            if (rb) rare_pair<NT, SUMS, AS>(sb, t.pos[q + 1], P, ubis, ubi, gs, hkf, cnt, sum);
+            if (ra) rare_pair<NT>(sa, t.pos[q], P, ubis, ubi, gs, hkf, cnt);
+            if (rb) rare_pair<NT>(sb, t.pos[q + 1], P, ubis, ubi, gs, hkf, cnt);
         }
     }
+}
+
+// The same range with every pair below hmax evaluated exactly.  Called by the
+// whole warp; a lane without a box has hmax < 0.  recs: the run's boxes.
+//
+// Sums: the pairs' counts and fixed-point sums in cnt and sum of the box's lane.
+// AS 1 and 2 (assignment, NT 1): the two passes of k_assign (gvec_grid.cu) on
+// the pair -- below tol^2 and below the g's drlv2 on entry, pass 1 takes the
+// smallest drlv2 bits per g, pass 2 the lowest UBI index reaching them.
+template <int NT, int AS>
+__device__ __forceinline__ void exact_range(const Staged& t, int ga, int gb, const uint64_t uu[9],
+                                            const uint64_t hh[3], float hmax, int lane,
+                                            const uint64_t* recs, Pend* pend,
+                                            const JoinParams& P, const double* __restrict__ ubis,
+                                            const double* __restrict__ gs, int cnt[NT],
+                                            unsigned long long sum[NT], unsigned& ntest) {
+    for (int q0 = ga & ~1; q0 < gb; q0 += 32) {
+        const int qe = min(q0 + 32, gb);
+        unsigned mask = 0;
+        int left = 32;
+        for (int q = q0; q < qe; q += 2) {
+            float sa, sb;
+            screen_pair(t, q, uu, hh, sa, sb);
+            mask = (mask >> 2) | (sa < hmax ? 0x40000000u : 0u) | (sb < hmax ? 0x80000000u : 0u);
+            left -= 2;
+        }
+        mask >>= left;  // bit b: staged g q0 + b (left < 32)
+        const int mine = __popc(mask);
+        ntest += mine;
+        int total;
+        int at = warp_excl_scan(mine, lane, total);  // the lane's next pair to list
+        for (int base = 0; base < total; base += kPend) {
+            const int e0 = at;
+            for (; mask && at < base + kPend; at++) {
+                pend[at - base].pair = {lane, q0 + __ffs(mask) - 1};
+                mask &= mask - 1;
+            }
+            __syncwarp();
+            const int n = min(kPend, total - base);
+            for (int e = lane; e < n; e += 32) {
+                const uint64_t rec = recs[pend[e].pair.lane];
+                const int pos = t.pos[pend[e].pair.q];
+                const int64_t ubi = P.i0 + (int64_t)(rec >> kUShift);
+                float hkf[3];
+                box_hkl(rec, hkf);
+                const Exact x = exact_pair(ubis, ubi, gs, pos, hkf[0], hkf[1], hkf[2]);
+                if (!AS) {
+                    pend[e].s = x.own ? x.s : INFINITY;
+                } else if (x.own && x.s < P.t2[0]) {
+                    const int k = __ldg(P.gidx + pos);
+                    if (x.s < __ldg(P.d0 + k)) {
+                        const unsigned long long b =
+                            (unsigned long long)__double_as_longlong(x.s);
+                        if (AS == 1)
+                            atomicMin(P.best + k, b);
+                        else if (P.best[k] == b)
+                            atomicMin(P.lab + k, (int)ubi);
+                    }
+                }
+            }
+            __syncwarp();
+            if (!AS) {
+                for (int e = e0; e < at; e++) {
+                    const double x = pend[e - base].s;
+                    const unsigned long long f =
+                        x < P.t2[NT - 1] ? __double2ull_rn(x * P.fix) : 0ull;  // per term: order-free
+#pragma unroll
+                    for (int j = 0; j < NT; j++)
+                        if (x < P.t2[j]) {
+                            cnt[j]++;
+                            sum[j] += f;
+                        }
+                }
+                __syncwarp();
+            }
+        }
+    }
+}
+
+// A UBI's FP32 elements and -hkl, each duplicated into a packed pair.
+__device__ __forceinline__ void load_pack(const float4* __restrict__ packs, int64_t ubi,
+                                          const float hkf[3], uint64_t uu[9], uint64_t hh[3]) {
+    const float4 p0 = __ldg(packs + 3 * ubi);
+    const float4 p1 = __ldg(packs + 3 * ubi + 1);
+    const float4 p2 = __ldg(packs + 3 * ubi + 2);
+    const float u[9] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x};
+#pragma unroll
+    for (int e = 0; e < 9; e++) uu[e] = pk2(u[e], u[e]);
+#pragma unroll
+    for (int e = 0; e < 3; e++) hh[e] = pk2(-hkf[e], -hkf[e]);
 }
 
 // Exclusive scan of a[0 .. len) into b (block-wide; ends with a barrier).
@@ -659,7 +736,8 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
        int* __restrict__ counts, double* __restrict__ sums) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* s_box = reinterpret_cast<uint64_t*>(smem);        // kBMax sorted boxes
-    float* s_gx = reinterpret_cast<float*>(s_box + kBMax);      // kGMax staged g
+    Pend* pend = reinterpret_cast<Pend*>(s_box + kBMax) + kPend * (threadIdx.x >> 5);  // SUMS
+    float* s_gx = reinterpret_cast<float*>(s_box + kBMax + (SUMS ? kPend * kJW : 0));  // kGMax staged g
     float* s_gy = s_gx + kGMax;
     float* s_gz = s_gy + kGMax;
     int* s_gp = reinterpret_cast<int*>(s_gz + kGMax);
@@ -822,22 +900,14 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                     const int gb = s_gs[min(box_fx(s_box[k0 + nrun - 1]) + P.Rx, gxb) - gxa + 1];
                     if (lane == 0 && ga < gb)
                         npairs += (unsigned long long)nrun * (unsigned)(((gb + 1) & ~1) - (ga & ~1));
-                    if (lane < nrun && ga < gb) {
-                        const uint64_t rec = s_box[k0 + lane];
+                    if (SUMS) {
+                        if (ga >= gb) continue;  // uniform over the warp
+                        const uint64_t rec = s_box[k0 + min(lane, nrun - 1)];
                         const int64_t ubi = P.i0 + (int64_t)(rec >> kUShift);
-                        const float hkf[3] = {(float)((int)((rec >> kHShift) & 511) - kHklOff),
-                                              (float)((int)((rec >> kKShift) & 511) - kHklOff),
-                                              (float)((int)((rec >> kLShift) & 511) - kHklOff)};
-                        const float4 p0 = __ldg(packs + 3 * ubi);
-                        const float4 p1 = __ldg(packs + 3 * ubi + 1);
-                        const float4 p2 = __ldg(packs + 3 * ubi + 2);
-                        const float u[9] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x};
+                        float hkf[3];
+                        box_hkl(rec, hkf);
                         uint64_t uu[9], hh[3];
-#pragma unroll
-                        for (int e = 0; e < 9; e++) uu[e] = pk2(u[e], u[e]);
-#pragma unroll
-                        for (int e = 0; e < 3; e++)
-                            hh[e] = ID11B_JOIN_FOLD ? pk2(-hkf[e], -hkf[e]) : pk2(hkf[e], hkf[e]);
+                        load_pack(packs, ubi, hkf, uu, hh);
                         int cnt[NT];
                         unsigned long long sum[NT];
 #pragma unroll
@@ -845,15 +915,30 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                             cnt[j] = 0;
                             sum[j] = 0ull;
                         }
-                        test_range<NT, SUMS, RANKED, AS>(T, ga, gb, uu, hh, hkf, P, ubis, ubi,
-                                                         gs, cnt, sum, ntest);
+                        exact_range<NT, AS>(T, ga, gb, uu, hh, lane < nrun ? P.hmax : -1.f, lane,
+                                            s_box + k0, pend, P, ubis, gs, cnt, sum, ntest);
 #pragma unroll
                         for (int j = 0; j < NT && !AS; j++) {
                             if (cnt[j]) atomicAdd(counts + ubi * NT + P.ord[j], cnt[j]);
-                            if (SUMS && sum[j])
+                            if (sum[j])
                                 atomicAdd(reinterpret_cast<unsigned long long*>(
                                               sums + ubi * NT + P.ord[j]), sum[j]);
                         }
+                    } else if (lane < nrun && ga < gb) {
+                        const uint64_t rec = s_box[k0 + lane];
+                        const int64_t ubi = P.i0 + (int64_t)(rec >> kUShift);
+                        float hkf[3];
+                        box_hkl(rec, hkf);
+                        uint64_t uu[9], hh[3];
+                        load_pack(packs, ubi, hkf, uu, hh);
+                        int cnt[NT];
+#pragma unroll
+                        for (int j = 0; j < NT; j++) cnt[j] = 0;
+                        test_range<NT, RANKED>(T, ga, gb, uu, hh, hkf, P, ubis, ubi, gs, cnt,
+                                               ntest);
+#pragma unroll
+                        for (int j = 0; j < NT; j++)
+                            if (cnt[j]) atomicAdd(counts + ubi * NT + P.ord[j], cnt[j]);
                     }
                 }
                 __syncthreads();
@@ -1130,8 +1215,8 @@ struct JoinLaunch {
 template <class Ctas, class Join, class After>
 static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, int32_t xsub,
                          const void* gridbuf, const Tols& T, int ntol, double tmax, void* ws,
-                         int64_t ws_bytes, cudaStream_t st, int passes, const JoinParams& P0,
-                         Ctas ctas, Join join, After after) {
+                         int64_t ws_bytes, cudaStream_t st, int passes, bool exact,
+                         const JoinParams& P0, Ctas ctas, Join join, After after) {
     const int nrows = nx * nx;
     const int nxx = nx * xsub;
     const int nblk = (nrows + kRowBlock - 1) / kRowBlock;
@@ -1217,13 +1302,10 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
         double W;
         memcpy(&W, &bi.wmax_bits, sizeof(W));
         // the FP32 error of the screened UBI.g - hkl per component: inputs
-        // rounded (2 eps S G) and three roundings, of partial sums below S G
-        // (h; the subtraction of hkl is then exact where it matters) or, folded,
-        // below |hkl| + S G <= S (2 G + W) (a box's centre c lies within G + W of
-        // the origin in every component, and hkl = UBI.c)
-        const double E = ID11B_JOIN_FOLD
-                             ? kEps32 * (double)smax * (8.0 * G + 3.0 * W) * (1. + 1e-6)
-                             : 6.0 * kEps32 * (double)smax * G;
+        // rounded (2 eps S G) and three roundings, of partial sums below
+        // |hkl| + S G <= S (2 G + W) (a box's centre c lies within G + W of the
+        // origin in every component, and hkl = UBI.c)
+        const double E = kEps32 * (double)smax * (8.0 * G + 3.0 * W) * (1. + 1e-6);
         P.hmax = 0.f;
         // ascending order of tolerance (stable), unused slots last
         int ord[ID11B_MAX_TOLS];
@@ -1258,7 +1340,8 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     if (bi.total > 0 && nhalo > kMaxHalo) return ID11B_ERR_SIZE;  // cells far smaller than W
     const size_t jsmem = sizeof(uint64_t) * kBMax + 4 * sizeof(float) * kGMax +
                          4 * sizeof(int) * (size_t)(std::max(nxx, nhalo) + 1) +
-                         2 * sizeof(int) * (size_t)(nhalo + 1);
+                         2 * sizeof(int) * (size_t)(nhalo + 1) +
+                         (exact ? sizeof(Pend) * kPend * kJW : 0);
     const int jgrid = num_sms() * ctas(jsmem, ranked);
     cudaEvent_t ev0 = t_join_start, ev1 = t_join_stop;
     t_join_start = t_join_stop = nullptr;
@@ -1331,7 +1414,7 @@ extern "C" int id11b_dev_score_grid_bins(const double* ubis, int64_t m, const do
     }
     JoinParams P0 = {};
     const int rc = bins_pipeline(
-        ubis, m, n, nx, xsub, gridbuf, T, ntol, tmax, ws, ws_bytes, st, 1, P0,
+        ubis, m, n, nx, xsub, gridbuf, T, ntol, tmax, ws, ws_bytes, st, 1, sums != nullptr, P0,
         [&](size_t smem, bool ranked) { return ID11B_BINS_DISPATCH(join_ctas, smem, ranked); },
         [&](int, const JoinLaunch& J) {
             return ID11B_BINS_DISPATCH(launch_join, J.grid, J.smem, J.ranked, J.recs, J.rstart,
@@ -1378,7 +1461,7 @@ extern "C" int id11b_dev_assign_grid_bins(const double* ubis, int64_t m, const d
     P0.best = bst;
     P0.lab = lab;
     return bins_pipeline(
-        ubis, m, n, nx, xsub, gridbuf, T, 1, tol, ws, ws_bytes, st, 2, P0,
+        ubis, m, n, nx, xsub, gridbuf, T, 1, tol, ws, ws_bytes, st, 2, true, P0,
         [&](size_t smem, bool) { return ctas_per_sm(k_join<1, true, false, 1>, kJT, smem); },
         [&](int pass, const JoinLaunch& J) {
             if (pass == 0)

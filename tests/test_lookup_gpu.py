@@ -66,3 +66,26 @@ def test_assignment_starting_values(scene, oracle, cuda):
         _, rd, rl = oracle.score_and_assign(x, gv, 0.1, rd, rl, i)
     batch.score_and_assign_grid(u, batch.GvecGrid(gv), 0.1, d, lab)
     assert np.array_equal(lab, rl) and np.array_equal(d, rd, equal_nan=True)
+
+
+@pytest.mark.parametrize("copies", [1, 3, 33, 70])
+@pytest.mark.parametrize("ntol", [1, 3, 4])
+def test_binned_sums_of_dense_boxes(oracle, copies, ntol, cuda):
+    """Every g of a run inside every box (up to 32 x 32 pairs of one step, many
+    more than a warp lists at once) and odd tiles: counts identical, sums equal
+    to FP64 rounding and the fixed-point step of each term."""
+    from imaged11_b200 import batch
+    rng = np.random.default_rng(94 + copies)
+    a = 4.0
+    hkl = np.stack(np.meshgrid(*[np.arange(-3, 4)] * 3), -1).reshape(-1, 3)[1:].astype(float)
+    g = np.repeat(hkl / a, copies, 0) + rng.normal(size=(len(hkl) * copies, 3)) * 1e-3
+    u = a * np.eye(3)[None] * (1 + rng.normal(size=(101, 1, 1)) * 1e-3)
+    tols = [0.3, 0.01, 0.1, 0.03][:ntol]
+    c, s = batch.score_grid(u, batch.GvecGrid(g), tols, sums=True, method="bins")
+    assert np.array_equal(c.cpu().numpy(), oracle.score_many(u, g, tols))
+    step = 2.0 ** -(62 - np.ceil(np.log2(len(g) * max(tols) ** 2)))
+    s = s.cpu().numpy()
+    for i in range(0, len(u), 7):
+        for j, t in enumerate(tols):
+            n, mean, _ = oracle.score_and_refine(u[i], g, t)
+            assert abs(s[i, j] - n * mean) <= 1e-12 * n * mean + n * step
