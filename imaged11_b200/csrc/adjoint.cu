@@ -31,9 +31,11 @@
 // and dr/d(tilts), the centre and distance terms with r and the pixel sizes
 // (k_finish).
 //
-// One CTA per grain accumulates its peaks' terms in registers and reduces
-// them in a fixed tree into a per-grain row; one CTA then sums the rows in
-// grain order.  Every result is deterministic.
+// One CTA (one to four warps, by the number of grains) takes grains in a fixed
+// stride, accumulates a grain's peaks in registers and reduces them in a fixed
+// tree; the geometry's sums stay one per lane from grain to grain and go out as
+// one row per CTA, and one CTA then sums the rows in order.  Every result is
+// deterministic.
 //
 // Variable projection (MODE 3): each grain's UBI is first solved in closed
 // form for the current g (UBI = (sum h g^T)(sum g g^T)^-1, the least-squares
@@ -46,10 +48,12 @@
 
 namespace id11b {
 
-constexpr int kAT = 64;         // threads per CTA
+constexpr int kAT = 64;         // threads per CTA of k_bragg
 constexpr int kNP = 12;         // geometry parameters
-constexpr int kGlob = 22;       // dM(9) dlam(1) dt(3) sum_axyz(3) dR1(3) dR2(3)
+constexpr int kGlob = 22;       // dM(9) -dlam*wavelength(1) dt(3) sum_axyz(3) dR1(3) dR2(3)
 constexpr int kPart = kGlob + 1;  // + sum of squared residuals
+constexpr int kRow = 32;        // doubles per CTA row of sums
+constexpr int kMaxRows = 4096;  // CTAs of a launch that sums rows
 
 struct AdjDet {
     double y_size, z_size, omegasign, o11, o12, o21, o22;
@@ -59,7 +63,7 @@ struct AdjGeom {
     double r[9];        // detector rotation . flip (row-major)
     double M[9];        // chi.wedge
     double t[3];        // grain-origin translation
-    double wavelength, distance, y_center, z_center, y_size, z_size, omegasign;
+    double wavelength, inv_wavelength, distance, y_center, z_center, y_size, z_size, omegasign;
 };
 
 struct PeakState {
@@ -81,14 +85,26 @@ struct RotFactors {
     double R[3][9], dR[3][9], F[9], W[9], C[9], dW[9], dC[9];
 };
 
-__device__ void rot_factors(const double* p, const AdjDet& D, RotFactors& f) {
-    double sx, cx, sy, cy, sz, cz, sw, cw, sc, cc;
-    sincos(p[3], &sx, &cx);
-    sincos(p[4], &sy, &cy);
-    sincos(p[5], &sz, &cz);
+// sin and cos of the five angles, each taken by its own lane (a warp; the
+// chain of five would be most of the kernels' start-up): sc = sin, cos of
+// tilt_x, tilt_y, tilt_z, wedge, chi
+__device__ __forceinline__ void angle_sincos(const double* __restrict__ p, double sc[10]) {
+    const int lane = threadIdx.x & 31;
     const double rad = 3.14159265358979323846 / 180.0;
-    sincos(p[7] * rad, &sw, &cw);
-    sincos(p[8] * rad, &sc, &cc);
+    double a = 0., s, c;
+    if (lane < 3) a = p[3 + lane];
+    if (lane == 3 || lane == 4) a = p[4 + lane] * rad;
+    sincos(a, &s, &c);
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        sc[2 * k] = __shfl_sync(0xffffffffu, s, k);
+        sc[2 * k + 1] = __shfl_sync(0xffffffffu, c, k);
+    }
+}
+
+__device__ void rot_factors(const double sc[10], const AdjDet& D, RotFactors& f) {
+    const double sx = sc[0], cx = sc[1], sy = sc[2], cy = sc[3], sz = sc[4], cz = sc[5],
+                 sw = sc[6], cw = sc[7], sk = sc[8], ck = sc[9];
     const double R3[9] = {1, 0, 0, 0, cx, -sx, 0, sx, cx};
     const double R2[9] = {cy, 0, sy, 0, 1, 0, -sy, 0, cy};
     const double R1[9] = {cz, -sz, 0, sz, cz, 0, 0, 0, 1};
@@ -97,9 +113,9 @@ __device__ void rot_factors(const double* p, const AdjDet& D, RotFactors& f) {
     const double dR1[9] = {-sz, -cz, 0, cz, -sz, 0, 0, 0, 0};
     const double F[9] = {1, 0, 0, 0, D.o22, D.o21, 0, D.o12, D.o11};
     const double W[9] = {cw, 0, -sw, 0, 1, 0, sw, 0, cw};
-    const double C[9] = {1, 0, 0, 0, cc, -sc, 0, sc, cc};
+    const double C[9] = {1, 0, 0, 0, ck, -sk, 0, sk, ck};
     const double dW[9] = {-sw, 0, -cw, 0, 0, 0, cw, 0, -sw};
-    const double dC[9] = {0, 0, 0, 0, -sc, -cc, 0, cc, -sc};
+    const double dC[9] = {0, 0, 0, 0, -sk, -ck, 0, ck, -sk};
 #pragma unroll
     for (int e = 0; e < 9; e++) {
         f.R[0][e] = R3[e];
@@ -125,15 +141,16 @@ __device__ void rot_product(const RotFactors& f, int which, double out[9]) {
     mat3mul(abc, f.F, out);
 }
 
-__device__ void make_geom(const double* p, const AdjDet& D, AdjGeom& P) {
+__device__ void make_geom(const double* p, const double sc[10], const AdjDet& D, AdjGeom& P) {
     RotFactors f;
-    rot_factors(p, D, f);
+    rot_factors(sc, D, f);
     rot_product(f, -1, P.r);
     mat3mul(f.W, f.C, P.M);
     P.t[0] = p[9];
     P.t[1] = p[10];
     P.t[2] = p[11];
     P.wavelength = p[6];
+    P.inv_wavelength = 1.0 / p[6];
     P.distance = p[0];
     P.y_center = p[1];
     P.z_center = p[2];
@@ -157,6 +174,13 @@ __device__ __forceinline__ void peak_sincos(const AdjGeom& P, const double* __re
     }
 }
 
+// a / y given ry = 1 / y rounded: the quotient's remainder corrects the product
+// (three operations; the rounding is that of a division but for rare last bits)
+__device__ __forceinline__ double div_by(double a, double y, double ry) {
+    const double q = a * ry;
+    return fma(fma(-q, y, a), ry, q);
+}
+
 __device__ __forceinline__ void forward_peak(const AdjGeom& P, double s, double f, double so,
                                              double co, PeakState& q) {
     q.so = so;
@@ -174,14 +198,14 @@ __device__ __forceinline__ void forward_peak(const AdjGeom& P, double s, double 
 #pragma unroll
     for (int i = 0; i < 3; i++)
         d[i] = xyz[i] - (P.M[3 * i] * q.u[0] + P.M[3 * i + 1] * q.u[1] + P.M[3 * i + 2] * q.u[2]);
-    q.rn = 1.0 / sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    q.rn = rsqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
 #pragma unroll
     for (int i = 0; i < 3; i++) q.dh[i] = d[i] * q.rn;
     // divided, not multiplied by a rounded 1/wavelength: the rounding then
     // stays independent from peak to peak as wavelength varies
-    q.k[0] = (q.dh[0] - 1.0) / P.wavelength;
-    q.k[1] = q.dh[1] / P.wavelength;
-    q.k[2] = q.dh[2] / P.wavelength;
+    q.k[0] = div_by(q.dh[0] - 1.0, P.wavelength, P.inv_wavelength);
+    q.k[1] = div_by(q.dh[1], P.wavelength, P.inv_wavelength);
+    q.k[2] = div_by(q.dh[2], P.wavelength, P.inv_wavelength);
     double v[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) v[i] = P.M[i] * q.k[0] + P.M[3 + i] * q.k[1] + P.M[6 + i] * q.k[2];
@@ -214,15 +238,13 @@ __device__ __forceinline__ void adjoint_peak(const AdjGeom& P, const PeakState& 
     for (int j = 0; j < 3; j++)
 #pragma unroll
         for (int i = 0; i < 3; i++) gl[3 * j + i] += q.k[j] * av[i];
-    const double akk = ak[0] * q.k[0] + ak[1] * q.k[1] + ak[2] * q.k[2];
-    gl[9] += -akk / P.wavelength;
-    double adh[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) adh[i] = ak[i] / P.wavelength;
-    const double dd = q.dh[0] * adh[0] + q.dh[1] * adh[1] + q.dh[2] * adh[2];
+    // dL/dwavelength = -(sum of ak.k) / wavelength, divided once at the end
+    gl[9] += ak[0] * q.k[0] + ak[1] * q.k[1] + ak[2] * q.k[2];
+    const double dd = q.dh[0] * ak[0] + q.dh[1] * ak[1] + q.dh[2] * ak[2];
+    const double rl = q.rn * P.inv_wavelength;
     double ad[3];
 #pragma unroll
-    for (int i = 0; i < 3; i++) ad[i] = (adh[i] - q.dh[i] * dd) * q.rn;
+    for (int i = 0; i < 3; i++) ad[i] = (ak[i] - q.dh[i] * dd) * rl;
     // o = M u: dM[i][j] += a_o_i u_j with a_o = -a_d
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -261,14 +283,120 @@ __device__ __forceinline__ void cta_reduce(double* acc, double (*red)[NA]) {
     __syncthreads();
 }
 
+// Sums over the warp of v[0 .. N), one per lane: at each step a lane keeps half
+// of its values and adds the partner's copies of them, so N - 1 exchanges do
+// what N full butterflies (5 N) would.  Returns the lane's sum; slot_of<N>
+// says which (-1: none; lanes may share one).
+template <int N, int O>
+struct ScatterSum {
+    static __device__ __forceinline__ double run(double* v, int lane) {
+        if constexpr (O == 0) {
+            return v[0];
+        } else if constexpr (N == 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+            return ScatterSum<1, O / 2>::run(v, lane);
+        } else {
+            constexpr int K = (N + 1) / 2;
+            const bool up = lane & O;
+#pragma unroll
+            for (int i = 0; i < K; i++) {
+                const double hi = i + K < N ? v[i + K] : 0.;
+                const double got = __shfl_xor_sync(0xffffffffu, up ? v[i] : hi, O);
+                v[i] = (up ? hi : v[i]) + got;
+            }
+            return ScatterSum<K, O / 2>::run(v, lane);
+        }
+    }
+};
+
+template <int N>
+__device__ __forceinline__ int slot_of(int lane) {
+    int at = 0, n = N, have = N;  // first value kept, values per lane, of them real ones
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n == 1) continue;
+        const int k = (n + 1) / 2;
+        if (lane & o) {
+            at += k;
+            have -= k;
+        } else {
+            have = min(have, k);
+        }
+        n = k;
+    }
+    return have > 0 ? at : -1;
+}
+
+// The grain's least-squares UBI from the sums A = sum h g^T (9) and
+// B = sum g g^T (6, upper triangle): UBI = A B^-1, element `lane` of it, by one
+// warp (each lane one cofactor and one division).  B is positive
+// semi-definite; fewer than three independent g leave it singular up to
+// rounding, so the test is relative: det <= 1e-10 trace^3 counts as singular
+// (UBI 0).
+// ab, B: shared memory (B: nine doubles of scratch).
+__device__ __forceinline__ double best_ubi(const double* ab, double* B, int lane) {
+    const int e = lane < 9 ? lane : 0, i = e / 3, j = e - 3 * i;
+    const int lo = min(i, j), hi = max(i, j);
+    if (lane < 9) B[e] = ab[9 + hi + lo + (lo > 0)];  // 00 01 02 11 12 22
+    __syncwarp();
+    const double tr = B[0] + B[4] + B[8];
+    const double det = B[0] * (B[4] * B[8] - B[5] * B[7]) - B[1] * (B[3] * B[8] - B[5] * B[6]) +
+                       B[2] * (B[3] * B[7] - B[4] * B[6]);
+    const double dx = det3_exact(B);
+    const bool ok = det > 1e-10 * tr * tr * tr && dx != 0.;
+    const double bi = ok ? inv3_elem(B, dx, e) : 0.;
+    double x = 0.;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        x += ab[3 * i + k] * __shfl_sync(0xffffffffu, bi, 3 * k + j);
+    return x;
+}
+
+// What the kernels read of a peak (H: its hkl too)
+struct PeakIn {
+    double s, f, so, co, h[3];
+};
+
+template <bool H>
+__device__ __forceinline__ void load_peak(const AdjGeom& P, const double* __restrict__ sc,
+                                          const double* __restrict__ fc,
+                                          const double* __restrict__ omega,
+                                          const double* __restrict__ osc,
+                                          const double* __restrict__ hkl, int64_t kk, PeakIn& x) {
+    x.s = __ldg(sc + kk);
+    x.f = __ldg(fc + kk);
+    peak_sincos(P, omega, osc, kk, x.so, x.co);
+    if (H)
+#pragma unroll
+        for (int i = 0; i < 3; i++) x.h[i] = __ldg(hkl + 3 * kk + i);
+}
+
 // MODE 0: residuals (+ g, + per-grain sum of squares); ubis == nullptr
 //         gives g only.
 // MODE 1: adjoint of given dL/dres.
 // MODE 2: loss 0.5 sum res^2 and its gradient (a_res = res) in one pass.
 // MODE 3: variable projection: least-squares UBI per grain, then MODE 2 at it.
 // MODE 4: least-squares UBI per grain only.
+//
+// T threads per CTA, one grain at a time.  Bound: the FP64 pipe (80 operations a
+// peak for a forward pass and its normal-equation sums, 170 with the reverse
+// pass) at the 43 % of its rate that 10 or 12 resident warps reach (the sums and
+// the peak's state are 168 registers); the next peak's loads are in flight while
+// one is computed.  Projected loss of 20,000 grains, 7.8M peaks: 0.23 ms and 0.012
+// for k_finish, from 0.52 and 0.12 ms with 64 threads a grain, full butterflies
+// (19,000 shuffles a grain), one thread's 3x3 solve, a division for each of 1/|d|
+// and /wavelength, and a row of sums per grain.  Gradient of 500 grains, 245k
+// peaks: 15.2 + 6.3 -> 7.9 + 4.5 us.
 template <int MODE>
-__global__ void __launch_bounds__(kAT)
+__host__ __device__ constexpr int residual_warps() {
+    // resident warps per SM compiled for: 12 (168 registers) for the projected
+    // loss, 0.23 ms against 0.29 at 10; the gradient spills at 12 (500 grains: 9.4 us
+    // against 7.9)
+    return MODE == 3 ? 12 : MODE == 1 || MODE == 2 ? 8 : 16;
+}
+
+template <int MODE, int T>
+__global__ void __launch_bounds__(T, residual_warps<MODE>() * 32 / T)
 k_residual(const double* __restrict__ params, AdjDet D, const double* __restrict__ sc,
            const double* __restrict__ fc, const double* __restrict__ omega,
            const double* __restrict__ osc,
@@ -276,31 +404,42 @@ k_residual(const double* __restrict__ params, AdjDet D, const double* __restrict
            const double* __restrict__ ubis, int ngrains, double* __restrict__ res,
            double* __restrict__ gout, double* __restrict__ ssq,
            const double* __restrict__ ares, double* __restrict__ dubi,
-           double* __restrict__ partial, double* __restrict__ ubis_out) {
+           double* __restrict__ rows, double* __restrict__ ubis_out) {
     constexpr bool kAdj = MODE == 1 || MODE == 2 || MODE == 3;
-    constexpr int NA = MODE == 0 ? 1 : (MODE == 4 ? 15 : 9 + kPart);
-    constexpr int NR = NA > 15 ? NA : 15;
+    constexpr int kU = MODE == 1 || MODE == 2 ? 9 : 0;  // dL/dUBI beside the geometry's sums
+    constexpr int W = T / 32;
     __shared__ AdjGeom sP;
-    __shared__ double s_red[kAT / 32][NR];
+    __shared__ double s_red[W][32];
+    __shared__ double s_ab[15], s_B[9];
     __shared__ double s_U[9];
-    const int tid = threadIdx.x;
-    if (tid == 0) make_geom(params, D, sP);
-    __syncthreads();
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (w == 0) {
+        double a[10];
+        angle_sincos(params, a);
+        if (lane == 0) make_geom(params, a, D, sP);
+    }
+    auto sync = [] {  // one warp needs no barrier of the CTA
+        if (T == 32) __syncwarp(); else __syncthreads();
+    };
+    sync();
     const AdjGeom& P = sP;
+    const int slot = slot_of<kU + kPart>(lane);
+    double total = 0.;  // the lane's geometry sum, over the CTA's grains
     for (int G = blockIdx.x; G < ngrains; G += gridDim.x) {
         const int64_t k0 = off[G], k1 = off[G + 1];
         double U[9];
         if (MODE == 3 || MODE == 4) {
-            // pass 1: A = sum h g^T (9), B = sum g g^T (6, upper triangle)
             double a[15];
 #pragma unroll
             for (int e = 0; e < 15; e++) a[e] = 0.;
-            for (int64_t kk = k0 + tid; kk < k1; kk += kAT) {
+            PeakIn in;
+            if (k0 + tid < k1) load_peak<true>(P, sc, fc, omega, osc, hkl, k0 + tid, in);
+            for (int64_t kk = k0 + tid; kk < k1; kk += T) {
+                const PeakIn x = in;  // the next peak's loads are in flight meanwhile
+                if (kk + T < k1) load_peak<true>(P, sc, fc, omega, osc, hkl, kk + T, in);
                 PeakState q;
-                double so, co;
-                peak_sincos(P, omega, osc, kk, so, co);
-                forward_peak(P, sc[kk], fc[kk], so, co, q);
-                const double h[3] = {hkl[3 * kk], hkl[3 * kk + 1], hkl[3 * kk + 2]};
+                forward_peak(P, x.s, x.f, x.so, x.co, q);
+                const double* h = x.h;
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
@@ -312,35 +451,27 @@ k_residual(const double* __restrict__ params, AdjDet D, const double* __restrict
                 a[13] += q.g[1] * q.g[2];
                 a[14] += q.g[2] * q.g[2];
             }
-            cta_reduce<15>(a, reinterpret_cast<double(*)[15]>(&s_red[0][0]));
-            if (tid == 0) {
-                const double* r = s_red[0];
-                double B[9] = {r[9], r[10], r[11], r[10], r[12], r[13], r[11], r[13], r[14]};
-                // B is positive semi-definite; fewer than three independent
-                // g leave it singular up to rounding, so the test is
-                // relative: det <= 1e-10 trace^3 counts as singular
-                const double tr = B[0] + B[4] + B[8];
-                const double det = B[0] * (B[4] * B[8] - B[5] * B[7]) -
-                                   B[1] * (B[3] * B[8] - B[5] * B[6]) +
-                                   B[2] * (B[3] * B[7] - B[4] * B[6]);
-                double X[9];
-                if (det > 1e-10 * tr * tr * tr && inverse3x3_exact(B) == 0) {
-                    mat3mul(r, B, X);   // UBI = A B^-1
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 9; e++) X[e] = 0.;   // singular: UBI 0
+            const int at = slot_of<15>(lane);
+            const double v = ScatterSum<15, 16>::run(a, lane);
+            if (at >= 0) s_red[w][at] = v;
+            sync();
+            if (w == 0) {
+                if (lane < 15) {
+                    double t = s_red[0][lane];
+                    for (int q = 1; q < W; q++) t += s_red[q][lane];
+                    s_ab[lane] = t;
                 }
-#pragma unroll
-                for (int e = 0; e < 9; e++) s_U[e] = X[e];
+                __syncwarp();
+                const double x = best_ubi(s_ab, s_B, lane);
+                if (lane < 9) {
+                    s_U[lane] = x;
+                    if (ubis_out) ubis_out[9 * (int64_t)G + lane] = x;
+                }
             }
-            __syncthreads();
+            sync();
+            if (MODE == 4) continue;
 #pragma unroll
             for (int e = 0; e < 9; e++) U[e] = s_U[e];
-            if (ubis_out && tid < 9) ubis_out[9 * (int64_t)G + tid] = s_U[tid];
-            if (MODE == 4) {
-                __syncthreads();
-                continue;
-            }
         } else if (ubis) {
 #pragma unroll
             for (int e = 0; e < 9; e++) U[e] = ubis[9 * (int64_t)G + e];
@@ -348,14 +479,17 @@ k_residual(const double* __restrict__ params, AdjDet D, const double* __restrict
 #pragma unroll
             for (int e = 0; e < 9; e++) U[e] = 0.;
         }
-        double acc[NA];
+        double acc[kU + kPart];
 #pragma unroll
-        for (int e = 0; e < NA; e++) acc[e] = 0.;
-        for (int64_t kk = k0 + tid; kk < k1; kk += kAT) {
+        for (int e = 0; e < kU + kPart; e++) acc[e] = 0.;
+        PeakIn in;
+        constexpr bool kH = MODE == 2 || MODE == 3;
+        if (k0 + tid < k1) load_peak<kH>(P, sc, fc, omega, osc, hkl, k0 + tid, in);
+        for (int64_t kk = k0 + tid; kk < k1; kk += T) {
+            const PeakIn x = in;
+            if (kk + T < k1) load_peak<kH>(P, sc, fc, omega, osc, hkl, kk + T, in);
             PeakState q;
-            double so, co;
-            peak_sincos(P, omega, osc, kk, so, co);
-            forward_peak(P, sc[kk], fc[kk], so, co, q);
+            forward_peak(P, x.s, x.f, x.so, x.co, q);
             if (MODE == 0) {
                 if (gout) {
 #pragma unroll
@@ -381,76 +515,113 @@ k_residual(const double* __restrict__ params, AdjDet D, const double* __restrict
 #pragma unroll
                     for (int i = 0; i < 3; i++)
                         ar[i] = U[3 * i] * q.g[0] + U[3 * i + 1] * q.g[1] + U[3 * i + 2] * q.g[2] -
-                                hkl[3 * kk + i];
-                    acc[9 + kGlob] += ar[0] * ar[0] + ar[1] * ar[1] + ar[2] * ar[2];
+                                x.h[i];
+                    acc[kU + kGlob] += ar[0] * ar[0] + ar[1] * ar[1] + ar[2] * ar[2];
                 }
-                adjoint_peak(P, q, U, ar, MODE == 3 ? nullptr : acc, acc + 9);
+                adjoint_peak(P, q, U, ar, kU ? acc : nullptr, acc + kU);
             }
         }
-        cta_reduce<NA>(acc, reinterpret_cast<double(*)[NA]>(&s_red[0][0]));
-        for (int e = tid; e < NA; e += kAT) {
-            const double t = s_red[0][e];
-            if (MODE == 0) {
-                if (ssq) ssq[G] = t;
-            } else if (e < 9) {
-                if (dubi) dubi[9 * (int64_t)G + e] = t;
+        if (MODE == 0) {
+            if (ssq) {
+                const double v = warp_sum(acc[0]);
+                if (lane == 0) s_red[w][0] = v;
+                sync();
+                if (tid == 0) {
+                    double t = s_red[0][0];
+                    for (int q = 1; q < W; q++) t += s_red[q][0];
+                    ssq[G] = t;
+                }
+                sync();
+            }
+            continue;
+        }
+        const double v = ScatterSum<kU + kPart, 16>::run(acc, lane);
+        if (slot >= kU) total += v;
+        if (kU && dubi) {
+            if (T == 32) {
+                if (slot >= 0 && slot < kU) dubi[9 * (int64_t)G + slot] = v;
             } else {
-                partial[(int64_t)G * kPart + (e - 9)] = t;
+                if (slot >= 0 && slot < kU) s_red[w][slot] = v;
+                sync();
+                if (tid < kU) {
+                    double t = s_red[0][tid];
+                    for (int q = 1; q < W; q++) t += s_red[q][tid];
+                    dubi[9 * (int64_t)G + tid] = t;
+                }
+                sync();
             }
         }
-        __syncthreads();
+    }
+    if (!kAdj) return;
+    if (slot >= kU) s_red[w][slot - kU] = total;
+    sync();
+    if (tid < kPart) {
+        double t = s_red[0][tid];
+        for (int q = 1; q < W; q++) t += s_red[q][tid];
+        rows[(int64_t)blockIdx.x * kRow + tid] = t;
     }
 }
 
-// Sums the per-grain rows (rows x kPart) in grain order (one warp per
-// column: lane l sums rows l, l+32, ..., then a fixed butterfly) and maps the
-// sums onto the 12 geometry parameters; loss = 0.5 * sum of squares.
-__global__ void __launch_bounds__(32 * kPart)
-k_finish(const double* __restrict__ partial, int rows, const double* __restrict__ params,
+// Sums the CTAs' rows in order (warp w takes rows w, w + 32, ..., a lane per
+// column; then the warps in order) and maps the sums onto the 12 geometry
+// parameters; loss = 0.5 * sum of squares.
+__global__ void __launch_bounds__(1024)
+k_finish(const double* __restrict__ rows, int nrows, const double* __restrict__ params,
          AdjDet D, double* __restrict__ grad, double* __restrict__ loss) {
-    __shared__ double col[kPart];
-    const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+    __shared__ double s_w[32][kRow + 1];
+    __shared__ double col[kRow];
+    __shared__ double s_dr[4][9], s_dm[2][9];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double t = 0.;
-    for (int r = lane; r < rows; r += 32) t += partial[(int64_t)r * kPart + c];
-    t = warp_sum(t);
-    if (lane == 0) col[c] = t;
+    if (lane < kPart) {
+#pragma unroll 14
+        for (int r = w; r < nrows; r += 32) t += rows[(int64_t)r * kRow + lane];
+    }
+    s_w[w][lane] = t;
+    if (w == 0) {  // r and its derivatives by the tilts, M's by wedge and chi
+        double a[10];
+        angle_sincos(params, a);
+        if (lane < 4) {
+            RotFactors f;
+            rot_factors(a, D, f);
+            rot_product(f, lane - 1, s_dr[lane]);
+            if (lane < 2) mat3mul(lane == 0 ? f.dW : f.W, lane == 0 ? f.C : f.dC, s_dm[lane]);
+        }
+    }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    if (loss) *loss = 0.5 * col[kGlob];
-    if (!grad) return;
-    RotFactors f;
-    rot_factors(params, D, f);
-    double r[9];
-    rot_product(f, -1, r);
+    if (w < kPart) {  // warp w: column w over the 32 warps
+        const double v = warp_sum(s_w[lane][w]);
+        if (lane == 0) col[w] = v;
+    }
+    __syncthreads();
+    const int e = threadIdx.x;
+    if (e == 31 && loss) *loss = 0.5 * col[kGlob];
+    if (!grad || e >= kNP) return;
     const double* dM = col;          // dL/dM (row-major)
     const double* A = col + 13;      // sum of dL/dxyz
     const double* dR1 = col + 16;    // dL/dr[:,1]
     const double* dR2 = col + 19;    // dL/dr[:,2]
-    grad[0] = A[0];
-    grad[1] = -D.y_size * (r[1] * A[0] + r[4] * A[1] + r[7] * A[2]);
-    grad[2] = -D.z_size * (r[2] * A[0] + r[5] * A[1] + r[8] * A[2]);
-    for (int k = 0; k < 3; k++) {    // tilt_x, tilt_y, tilt_z
-        double dr[9];
-        rot_product(f, k, dr);
-        double s = 0.;
-        for (int i = 0; i < 3; i++) s += dr[3 * i + 1] * dR1[i] + dr[3 * i + 2] * dR2[i];
-        grad[3 + k] = s;
+    const double* r = s_dr[0];
+    double g;
+    if (e == 0) {
+        g = A[0];
+    } else if (e <= 2) {
+        g = -(e == 1 ? D.y_size : D.z_size) * (r[e] * A[0] + r[3 + e] * A[1] + r[6 + e] * A[2]);
+    } else if (e <= 5) {             // tilt_x, tilt_y, tilt_z
+        const double* dr = s_dr[e - 2];
+        g = 0.;
+        for (int i = 0; i < 3; i++) g += dr[3 * i + 1] * dR1[i] + dr[3 * i + 2] * dR2[i];
+    } else if (e == 6) {
+        g = -col[9] / params[6];
+    } else if (e <= 8) {
+        const double* dm = s_dm[e - 7];
+        g = 0.;
+        for (int i = 0; i < 9; i++) g += dM[i] * dm[i];
+        g *= 3.14159265358979323846 / 180.0;
+    } else {
+        g = col[e + 1];
     }
-    grad[6] = col[9];
-    const double rad = 3.14159265358979323846 / 180.0;
-    double dMw[9], dMc[9];
-    mat3mul(f.dW, f.C, dMw);
-    mat3mul(f.W, f.dC, dMc);
-    double sw = 0., sc = 0.;
-    for (int e = 0; e < 9; e++) {
-        sw += dM[e] * dMw[e];
-        sc += dM[e] * dMc[e];
-    }
-    grad[7] = sw * rad;
-    grad[8] = sc * rad;
-    grad[9] = col[10];
-    grad[10] = col[11];
-    grad[11] = col[12];
+    grad[e] = g;
 }
 
 // Bragg angle of each assigned reflection computed from its grain's UB and
@@ -526,6 +697,43 @@ static int adj_grid(int ngrains) {
     return ngrains < cap ? ngrains : cap;
 }
 
+template <int MODE, int T>
+static int residual_slots() {  // resident CTAs of k_residual<MODE, T> on the GPU
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_residual<MODE, T>, T, 0) !=
+            cudaSuccess || per < 1)
+        per = 1;
+    return (sms > 0 ? sms : 148) * per;
+}
+
+// k_residual's launch: the widest CTA for which every grain has one of its own
+// resident, so that few grains still fill the GPU (100 grains' gradient: 5.0 us
+// with 128 threads, 6.3 with 64, 9.6 with 32), one warp each where there are more
+// grains than that (20,000 projected: 0.23 ms with 32, 0.25 with 64, 0.30 with 128).
+template <int MODE, class... A>
+static int launch_residual(int ngrains, int* rows, cudaStream_t st, A... args) {
+    // best_ubis takes the projected loss's width, and so gives its UBIs bit for bit
+    constexpr int kAs = MODE == 4 ? 3 : MODE;
+    static const int wide = residual_slots<kAs, 128>(), half = residual_slots<kAs, 64>(),
+                     slots32 = residual_slots<MODE, 32>();
+    int grid;
+    if (ngrains <= wide) {
+        grid = std::min(ngrains, kMaxRows);
+        k_residual<MODE, 128><<<grid, 128, 0, st>>>(args...);
+    } else if (ngrains <= half) {
+        grid = std::min(ngrains, kMaxRows);
+        k_residual<MODE, 64><<<grid, 64, 0, st>>>(args...);
+    } else {
+        grid = std::min(ngrains, std::min(slots32, kMaxRows));
+        k_residual<MODE, 32><<<grid, 32, 0, st>>>(args...);
+    }
+    ID11B_CHECK_LAUNCH();
+    if (rows) *rows = grid;
+    return ID11B_OK;
+}
+
 static int adj_det(const double* d, AdjDet& D) {
     if (!d) return ID11B_ERR_ARG;
     D.y_size = d[0];
@@ -543,7 +751,8 @@ static int adj_det(const double* d, AdjDet& D) {
 using namespace id11b;
 
 extern "C" int64_t id11b_adjoint_workspace_bytes(int32_t ngrains) {
-    return (int64_t)sizeof(double) * kPart * (ngrains > 0 ? ngrains : 1);
+    return (int64_t)sizeof(double) * kRow *
+           (ngrains > 0 ? (ngrains < kMaxRows ? ngrains : kMaxRows) : 1);
 }
 
 // omega_sincos (optional, 16-byte aligned): the table id11b_dev_omega_sincos
@@ -562,11 +771,10 @@ extern "C" int id11b_dev_residuals(const double* params, const double* detector,
     if (!offsets || !sc || !fc || !omega) return ID11B_ERR_ARG;
     if (ubis && (!hkl || !res)) return ID11B_ERR_ARG;
     if (!ubis && !gvec) return ID11B_ERR_ARG;
-    k_residual<0><<<adj_grid(ngrains), kAT, 0, (cudaStream_t)stream>>>(
-        params, D, sc, fc, omega, omega_sincos, hkl, offsets, ubis, ngrains, res, gvec,
-        ubis ? ssq : nullptr, nullptr, nullptr, nullptr, nullptr);
-    ID11B_CHECK_LAUNCH();
-    return ID11B_OK;
+    double* const none = nullptr;
+    return launch_residual<0>(ngrains, nullptr, (cudaStream_t)stream, params, D, sc, fc, omega,
+                              omega_sincos, hkl, offsets, ubis, ngrains, res, gvec,
+                              ubis ? ssq : none, (const double*)none, none, none, none);
 }
 
 extern "C" int id11b_dev_residuals_adjoint(const double* params, const double* detector,
@@ -588,13 +796,14 @@ extern "C" int id11b_dev_residuals_adjoint(const double* params, const double* d
     if (!offsets || !sc || !fc || !omega || !hkl || !ubis || !grad_res || !workspace)
         return ID11B_ERR_ARG;
     if (ws_bytes < id11b_adjoint_workspace_bytes(ngrains)) return ID11B_ERR_SIZE;
-    double* partial = (double*)workspace;
-    k_residual<1><<<adj_grid(ngrains), kAT, 0, st>>>(params, D, sc, fc, omega, omega_sincos, hkl,
-                                                     offsets, ubis, ngrains, nullptr, nullptr,
-                                                     nullptr, grad_res, grad_ubis, partial,
-                                                     nullptr);
-    ID11B_CHECK_LAUNCH();
-    k_finish<<<1, 32 * kPart, 0, st>>>(partial, ngrains, params, D, grad_params, nullptr);
+    double* rows = (double*)workspace;
+    double* const none = nullptr;
+    int nrows = 0;
+    const int rc = launch_residual<1>(ngrains, &nrows, st, params, D, sc, fc, omega, omega_sincos,
+                                      hkl, offsets, ubis, ngrains, none, none, none, grad_res,
+                                      grad_ubis, rows, none);
+    if (rc) return rc;
+    k_finish<<<1, 1024, 0, st>>>(rows, nrows, params, D, grad_params, nullptr);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
 }
@@ -618,18 +827,18 @@ extern "C" int id11b_dev_residual_loss(const double* params, const double* detec
     }
     if (!offsets || !sc || !fc || !omega || !hkl || !workspace) return ID11B_ERR_ARG;
     if (ws_bytes < id11b_adjoint_workspace_bytes(ngrains)) return ID11B_ERR_SIZE;
-    double* partial = (double*)workspace;
-    const int grid = adj_grid(ngrains);
-    if (ubis)
-        k_residual<2><<<grid, kAT, 0, st>>>(params, D, sc, fc, omega, omega_sincos, hkl, offsets,
-                                            ubis, ngrains, nullptr, nullptr, nullptr, nullptr,
-                                            grad_ubis, partial, nullptr);
-    else
-        k_residual<3><<<grid, kAT, 0, st>>>(params, D, sc, fc, omega, omega_sincos, hkl, offsets,
-                                            nullptr, ngrains, nullptr, nullptr, nullptr, nullptr,
-                                            nullptr, partial, ubis_out);
-    ID11B_CHECK_LAUNCH();
-    k_finish<<<1, 32 * kPart, 0, st>>>(partial, ngrains, params, D, grad_params, loss);
+    double* rows = (double*)workspace;
+    double* const none = nullptr;
+    int nrows = 0;
+    const int rc =
+        ubis ? launch_residual<2>(ngrains, &nrows, st, params, D, sc, fc, omega, omega_sincos, hkl,
+                                  offsets, ubis, ngrains, none, none, none, (const double*)none,
+                                  grad_ubis, rows, none)
+             : launch_residual<3>(ngrains, &nrows, st, params, D, sc, fc, omega, omega_sincos, hkl,
+                                  offsets, (const double*)none, ngrains, none, none, none,
+                                  (const double*)none, none, rows, ubis_out);
+    if (rc) return rc;
+    k_finish<<<1, 1024, 0, st>>>(rows, nrows, params, D, grad_params, loss);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
 }
@@ -644,11 +853,10 @@ extern "C" int id11b_dev_best_ubis(const double* params, const double* detector,
     if (osc_misaligned(omega_sincos)) return ID11B_ERR_ALIGN;
     if (ngrains == 0) return ID11B_OK;
     if (!offsets || !sc || !fc || !omega || !hkl || !ubis_out) return ID11B_ERR_ARG;
-    k_residual<4><<<adj_grid(ngrains), kAT, 0, (cudaStream_t)stream>>>(
-        params, D, sc, fc, omega, omega_sincos, hkl, offsets, nullptr, ngrains, nullptr,
-        nullptr, nullptr, nullptr, nullptr, nullptr, ubis_out);
-    ID11B_CHECK_LAUNCH();
-    return ID11B_OK;
+    double* const none = nullptr;
+    return launch_residual<4>(ngrains, nullptr, (cudaStream_t)stream, params, D, sc, fc, omega,
+                              omega_sincos, hkl, offsets, (const double*)none, ngrains, none, none,
+                              none, (const double*)none, none, none, ubis_out);
 }
 
 extern "C" int id11b_dev_bragg_theta(const double* ubs, const double* hkl,

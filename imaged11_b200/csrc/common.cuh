@@ -68,6 +68,28 @@ __device__ __forceinline__ int inverse3x3_exact(double m[9]) {
     return 0;
 }
 
+// The determinant of inverse3x3_exact.
+__device__ __forceinline__ double det3_exact(const double* a) {
+    return dadd(dsub(dmul(a[0], dsub(dmul(a[8], a[4]), dmul(a[7], a[5]))),
+                     dmul(a[3], dsub(dmul(a[8], a[1]), dmul(a[7], a[2])))),
+                dmul(a[6], dsub(dmul(a[5], a[1]), dmul(a[4], a[2]))));
+}
+
+// Element idx of the cofactor inverse with the same expressions, for nine lanes
+// that take one element each: the four factors are picked by index, so the lanes
+// share one path and one division (a switch over the nine expressions ran nine
+// divisions one after another).
+__device__ __forceinline__ double inv3_elem(const double* a, double det, int idx) {
+    // element idx = +-(a[p] a[q] - a[r] a[s]): p, q, r, s as the digits of pqrs
+    constexpr unsigned long long kP = 0x477588588ull, kQ = 0x003003114ull,
+                                 kR = 0x366366477ull, kS = 0x114225225ull;
+    const int sh = 4 * idx;
+    const int p = (int)(kP >> sh) & 15, q = (int)(kQ >> sh) & 15, r = (int)(kR >> sh) & 15,
+              s = (int)(kS >> sh) & 15;
+    const double t = dsub(dmul(a[p], a[q]), dmul(a[r], a[s]));
+    return ddiv(idx & 1 ? -t : t, det);
+}
+
 // UB = R.inv(H), UBI = inv(UB); ubi is replaced only when both inverses exist
 // (ImageD11 src/closest.c:326-340).  UB(i,j) sums l = 0,1,2 starting from 0.
 __device__ __forceinline__ void lsq_update_exact(double R[9], double H[9], double ubi[9]) {

@@ -25,29 +25,6 @@
 
 namespace id11b {
 
-// Element idx of the cofactor inverse, as inverse3x3 (src/closest.c:38-76).
-__device__ __forceinline__ double inv3_elem(const double* a, double det, int idx) {
-    const double a00 = a[0], a01 = a[1], a02 = a[2], a10 = a[3], a11 = a[4], a12 = a[5],
-                 a20 = a[6], a21 = a[7], a22 = a[8];
-    switch (idx) {
-        case 0: return ddiv(dsub(dmul(a22, a11), dmul(a21, a12)), det);
-        case 1: return ddiv(-dsub(dmul(a22, a01), dmul(a21, a02)), det);
-        case 2: return ddiv(dsub(dmul(a12, a01), dmul(a11, a02)), det);
-        case 3: return ddiv(-dsub(dmul(a22, a10), dmul(a20, a12)), det);
-        case 4: return ddiv(dsub(dmul(a22, a00), dmul(a20, a02)), det);
-        case 5: return ddiv(-dsub(dmul(a12, a00), dmul(a10, a02)), det);
-        case 6: return ddiv(dsub(dmul(a21, a10), dmul(a20, a11)), det);
-        case 7: return ddiv(-dsub(dmul(a21, a00), dmul(a20, a01)), det);
-        default: return ddiv(dsub(dmul(a11, a00), dmul(a10, a01)), det);
-    }
-}
-
-__device__ __forceinline__ double det3_exact(const double* a) {
-    return dadd(dsub(dmul(a[0], dsub(dmul(a[8], a[4]), dmul(a[7], a[5]))),
-                     dmul(a[3], dsub(dmul(a[8], a[1]), dmul(a[7], a[2])))),
-                dmul(a[6], dsub(dmul(a[5], a[1]), dmul(a[4], a[2]))));
-}
-
 template <int NT>
 struct RefineSmem {
     double red[NT / 32][17];  // per-warp partial sums

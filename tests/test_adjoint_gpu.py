@@ -272,3 +272,82 @@ def test_singular_grain_gets_zero_ubi(cuda):
     L = adjoint.projected_loss(p, peaks)
     L.backward()
     assert np.isfinite(float(L)) and np.all(np.isfinite(p.grad.cpu().numpy()))
+
+
+@pytest.mark.parametrize("ngrains", [1, 3, 299, 400, 700, 1000, 2500])
+def test_launch_widths_match_autograd(ngrains, cuda):
+    """Grain counts on both sides of each CTA width (and more grains than
+    resident CTAs), grains of 0 to 70 peaks (fewer than the CTA's threads, not a
+    multiple of them): loss, gradients and best UBIs against torch autograd of
+    the same model in FP64.  Sums of n terms differ by rounding in their order:
+    1e-12 of the largest element."""
+    import math
+    import torch
+    from imaged11_b200 import adjoint, synth
+    rng = np.random.default_rng(ngrains)
+    truth = synth.default_geometry(distance=152300., y_center=1027.7, z_center=1021.9,
+                                   tilt_x=0.004, tilt_y=-0.002, tilt_z=0.006, wedge=0.01,
+                                   chi=0.02, t_x=5., t_y=-3., t_z=2.)
+    count = rng.integers(8, 71, ngrains)
+    count[ngrains // 2:] = np.where(rng.random(ngrains - ngrains // 2) < 0.1, 0,
+                                    count[ngrains // 2:])
+    off = np.concatenate([[0], np.cumsum(count)])
+    n = int(off[-1])
+    s, f, om = rng.uniform(0, 2048, n), rng.uniform(0, 2048, n), rng.uniform(0, 360, n)
+    u = 4.05 * synth.random_rotations(ngrains, rng)
+    grain = torch.tensor(np.repeat(np.arange(ngrains), count), device=cuda)
+    t = {k: torch.tensor(v, device=cuda) for k, v in (("s", s), ("f", f), ("om", om))}
+    p = adjoint.params_tensor(truth).requires_grad_(True)
+    ut = torch.tensor(u, device=cuda).requires_grad_(True)
+    q = dict(zip(adjoint.PARAMS, p))
+
+    def mat(rows):
+        return torch.stack([torch.stack([torch.as_tensor(v, dtype=torch.float64, device=cuda)
+                                         for v in r]) for r in rows])
+
+    def rot(a):
+        return torch.sin(a), torch.cos(a)
+    (sx, cx), (sy, cy), (sz, cz) = rot(q["tilt_x"]), rot(q["tilt_y"]), rot(q["tilt_z"])
+    (sw, cw), (sk, ck) = rot(q["wedge"] * math.pi / 180), rot(q["chi"] * math.pi / 180)
+    r = mat([[1, 0, 0], [0, cx, -sx], [0, sx, cx]]) @ mat([[cy, 0, sy], [0, 1, 0], [-sy, 0, cy]]) \
+        @ mat([[cz, -sz, 0], [sz, cz, 0], [0, 0, 1]]) @ mat([[1, 0, 0], [0, -1, 0], [0, 0, 1]])
+    M = mat([[cw, 0, -sw], [0, 1, 0], [sw, 0, cw]]) @ mat([[1, 0, 0], [0, ck, -sk], [0, sk, ck]])
+    v1, v2 = (t["f"] - q["y_center"]) * 75., (t["s"] - q["z_center"]) * 75.
+    xyz = v1[:, None] * r[:, 1] + v2[:, None] * r[:, 2]
+    xyz = torch.stack([xyz[:, 0] + q["distance"], xyz[:, 1], xyz[:, 2]], 1)
+    so, co = rot(t["om"] * math.pi / 180)
+    o = torch.stack([co * q["t_x"] - so * q["t_y"], so * q["t_x"] + co * q["t_y"],
+                     q["t_z"].expand(n)], 1) @ M.T
+    d = xyz - o
+    k = (d / d.norm(dim=1, keepdim=True) -
+         torch.tensor([1., 0., 0.], dtype=torch.float64, device=cuda)) / q["wavelength"]
+    v = k @ M
+    g = torch.stack([co * v[:, 0] + so * v[:, 1], co * v[:, 1] - so * v[:, 0], v[:, 2]], 1)
+    h = torch.round(torch.einsum("nij,nj->ni", ut.detach()[grain], g.detach()))
+    h = h + 0.01 * torch.tensor(rng.normal(size=(n, 3)), device=cuda)
+    geo = dict(y_size=75., z_size=75., omegasign=1., o11=1., o12=0., o21=0., o22=-1.)
+    peaks = adjoint.PeakTable(s, f, om, h.cpu().numpy(), off, geo)
+
+    def close(a, b, tol=1e-12):
+        return bool((a - b).abs().max() <= tol * b.abs().max())
+    L = 0.5 * ((torch.einsum("nij,nj->ni", ut[grain], g) - h) ** 2).sum()
+    gp, gu = torch.autograd.grad(L, (p, ut), retain_graph=True)
+    L2, gp2, gu2 = _grad(p.detach(), ut.detach(), peaks)
+    assert abs(L2 - float(L.detach())) <= 1e-12 * float(L.detach())
+    # each parameter's gradient is a sum of n terms that may cancel: its bound
+    # scales with the loss's terms, so each is held to 1e-9 of itself
+    assert np.all(np.abs(gp2 - gp.cpu().numpy()) <= 1e-9 * np.abs(gp.cpu().numpy()))
+    assert close(torch.tensor(gu2, device=cuda), gu)
+    pr = p.detach().clone().requires_grad_(True)
+    ub = torch.full((ngrains, 3, 3), 7., dtype=torch.float64, device=cuda)
+    Lp = adjoint.projected_loss(pr, peaks, ub)
+    Lp.backward()
+    assert torch.equal(adjoint.best_ubis(p.detach(), peaks)[count > 0], ub[count > 0])
+    assert bool((ub[count == 0] == 0).all())
+    Lu = 0.5 * ((torch.einsum("nij,nj->ni", ub[grain], g) - h) ** 2).sum()
+    gq, = torch.autograd.grad(Lu, (p,))
+    assert abs(float(Lp.detach()) - float(Lu.detach())) <= 1e-12 * float(Lu.detach())
+    # the wavelength is a flat direction of the projected loss (its gradient is
+    # zero but for rounding): nothing to compare there
+    some = [i for i, k in enumerate(adjoint.PARAMS) if k != "wavelength"]
+    assert np.all((pr.grad - gq).abs()[some].cpu().numpy() <= 1e-8 * gq.abs()[some].cpu().numpy())
