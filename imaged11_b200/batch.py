@@ -457,10 +457,10 @@ class GrainSet:
     is copied to the GPU once; grains are processed largest first.
 
     threads: CTA size of the persistent launch; None takes the size
-    tune.tune_refine found for this many grains and peaks, else 64.  Measured
-    on B200 with 2,000 grains of 20..1,500 peaks: 64 threads 53 us for 5
-    rounds, 128 -> 87 us, 256 -> 147 us -- many small CTAs keep more grains in
-    flight, which matters more than the longest grain's share of lanes."""
+    tune.tune_refine found for this many grains and peaks, else 128.  Measured
+    on B200 with 2,000 grains of 20..2,000 peaks, 5 rounds: 128 threads 37 us,
+    64 -> 42 us, 256 -> 54 us; with 500 grains 17, 22 and 24 us -- the large
+    grains want several warps each, the small ones are refined by one warp."""
 
     def __init__(self, gv, offsets, ubis, threads=None):
         torch = _torch()
@@ -482,7 +482,7 @@ class GrainSet:
         self.peaks = int(off[-1] - off[0]) if len(off) else 0
         if threads is None:
             from . import tune
-            threads = tune.refine_threads(self.ngrains, self.peaks) or 64
+            threads = tune.refine_threads(self.ngrains, self.peaks) or 128
         self.threads = int(threads)
 
     def refine(self, tol, iters, persistent=True, precision="fp64"):

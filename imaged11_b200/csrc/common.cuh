@@ -148,6 +148,50 @@ __device__ __forceinline__ long long warp_sum(long long v) {
     return v;
 }
 
+// Sums over the warp of v[0 .. N), one per lane: at each step a lane keeps half
+// of its values and adds the partner's copies of them, so N - 1 exchanges do
+// what N full butterflies (5 N) would.  Returns the lane's sum; slot_of<N>
+// says which (-1: none; lanes may share one).
+template <int N, int O>
+struct ScatterSum {
+    static __device__ __forceinline__ double run(double* v, int lane) {
+        if constexpr (O == 0) {
+            return v[0];
+        } else if constexpr (N == 1) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+            return ScatterSum<1, O / 2>::run(v, lane);
+        } else {
+            constexpr int K = (N + 1) / 2;
+            const bool up = lane & O;
+#pragma unroll
+            for (int i = 0; i < K; i++) {
+                const double hi = i + K < N ? v[i + K] : 0.;
+                const double got = __shfl_xor_sync(0xffffffffu, up ? v[i] : hi, O);
+                v[i] = (up ? hi : v[i]) + got;
+            }
+            return ScatterSum<K, O / 2>::run(v, lane);
+        }
+    }
+};
+
+template <int N>
+__device__ __forceinline__ int slot_of(int lane) {
+    int at = 0, n = N, have = N;  // first value kept, values per lane, of them real ones
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n == 1) continue;
+        const int k = (n + 1) / 2;
+        if (lane & o) {
+            at += k;
+            have -= k;
+        } else {
+            have = min(have, k);
+        }
+        n = k;
+    }
+    return have > 0 ? at : -1;
+}
+
 }  // namespace id11b
 
 // Status from a launch: 0, or ID11B_ERR_CUDA with the CUDA code recorded.

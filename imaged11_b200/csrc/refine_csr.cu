@@ -6,14 +6,15 @@
 // 256 or 512 threads, chosen from the largest grain) refines one grain at a
 // time and runs all rounds itself: per round, every thread tests its peaks
 // with the reference's exact FP64 arithmetic and accumulates the accepted
-// peaks' normal-equation terms, the CTA reduces them in a fixed tree (warp
-// butterfly, then warps in order),
-// and nine threads apply the reference's update (one cofactor / one UB element
-// each; the same expressions as inverse3x3, so the result equals the
-// single-thread update bit for bit).
+// peaks' normal-equation terms, the CTA reduces them in a fixed tree (exchanges
+// that leave one sum per lane, then the warps in order), and nine lanes of the
+// first warp apply the reference's update (one cofactor / one UB element each;
+// the same expressions as inverse3x3, so the result equals the single-thread
+// update bit for bit).
 //
-// Persistent mode (queue != null): a grid sized to the GPU pulls grains from
-// an atomic work counter in the caller's order -- largest grains first (LPT)
+// Persistent mode (queue != null): a grid sized to the GPU, each CTA's first
+// grain its own index, the others from an atomic work counter read while the
+// grain before is refined, in the caller's order -- largest grains first (LPT)
 // keeps the tail short.  No CTA ever waits on another, so there is nothing to
 // time out.  Plain mode (queue == null): CTA b refines grain order[b]; used
 // one launch per round as the straightforward baseline.
@@ -25,19 +26,15 @@
 
 namespace id11b {
 
-template <int NT>
 struct RefineSmem {
-    double red[NT / 32][17];  // per-warp partial sums
-    double R[9], H[9], Hi[9], UB[9], UBI[9], ubi[9];
-    long long n;
-    double ss;
-    int ok, ok2;
-    int grain;
+    double R[9], H[9], UB[9], ubi[9];
 };
 
-// H upper-triangle slot (00 01 02 11 12 22) -> row, column
-__constant__ int c_hrow[6] = {0, 0, 0, 1, 1, 2};
-__constant__ int c_hcol[6] = {0, 1, 2, 1, 2, 2};
+// H upper-triangle slot (00 01 02 11 12 22) of element e of H
+__device__ __forceinline__ int h_slot(int e) {
+    const int i = e / 3, j = e - 3 * i, lo = min(i, j);
+    return i + j + (lo > 0);
+}
 
 // Compensated FP32 accumulation (the F32C variant): a sum kept as s + c with
 // every addition's rounding error recovered exactly (TwoSum) and every
@@ -51,203 +48,282 @@ __device__ __forceinline__ void comp_add(float& s, float& c, float x) {
     s = t;
 }
 
+// One round's pass over the grain's peaks (tid, tid + N, ...), in the reference's
+// FP64 arithmetic: the accepted peaks' normal-equation terms.  Two peaks a step,
+// their tests side by side (each is a chain of dependent operations) and the
+// next two's loads in flight; the segment is read-only and re-read every round,
+// so later rounds hit L1.  The terms use fused multiply-adds: H (products of
+// integers) is exact either way; each R term is rounded once instead of twice --
+// R is order-dependent against the reference's sequential sum in any case.
+__device__ __forceinline__ void add_peak(const double ih[3], const double g[3], double s,
+                                         double acc[17], int& nacc) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) acc[3 * i + j] = fma(ih[j], g[i], acc[3 * i + j]);
+    acc[9] = fma(ih[0], ih[0], acc[9]);
+    acc[10] = fma(ih[1], ih[0], acc[10]);
+    acc[11] = fma(ih[2], ih[0], acc[11]);
+    acc[12] = fma(ih[1], ih[1], acc[12]);
+    acc[13] = fma(ih[2], ih[1], acc[13]);
+    acc[14] = fma(ih[2], ih[2], acc[14]);
+    acc[15] = dadd(acc[15], s);
+    nacc++;
+}
+
+template <int N>
+__device__ __forceinline__ void refine_peaks(const double u[9], const double* __restrict__ first,
+                                             int tid, int n, double tolsq, double acc[17],
+                                             int& nacc) {
+    double nxt[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            nxt[q][i] = tid + q * N < n ? __ldg(first + 3 * q * N + i) : 0.;
+    const double* p = first;
+    for (int k = tid; k < n; k += 2 * N) {
+        double g[2][3], ih[2][3];
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int i = 0; i < 3; i++) g[q][i] = nxt[q][i];
+        p += 6 * N;
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (k + (2 + q) * N < n)
+#pragma unroll
+                for (int i = 0; i < 3; i++) nxt[q][i] = __ldg(p + 3 * q * N + i);
+        const double s0 = drlv2_exact(u, g[0][0], g[0][1], g[0][2], ih[0]);
+        const double s1 = drlv2_exact(u, g[1][0], g[1][1], g[1][2], ih[1]);
+        if (s0 < tolsq) add_peak(ih[0], g[0], s0, acc, nacc);
+        if (k + N < n && s1 < tolsq) add_peak(ih[1], g[1], s1, acc, nacc);
+    }
+}
+
+// The same in the F32C variant: FP32 screening with the proven band
+// (score_batch.cu) for this UBI, compensated R and drlv2 sums, exact integer H.
+template <int N>
+__device__ __forceinline__ void refine_peaks_f32c(const double u[9],
+                                                  const double* __restrict__ first, int tid, int n,
+                                                  double tolsq, double gmax, double acc[17],
+                                                  int& nacc) {
+    float u32[9], rs[9], rc[9], ss32 = 0.f, sc32 = 0.f;
+    int hint[6] = {0, 0, 0, 0, 0, 0};
+    double S = 0.;
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+        S = fmax(S, fabs(u[3 * r]) + fabs(u[3 * r + 1]) + fabs(u[3 * r + 2]));
+    const double E = 6.0 * 5.9604644775390625e-08 * S * (1. + 1e-15) * gmax;
+    const double t = sqrt(tolsq);
+    const double band = 1.25 * (3.0 * E * (2.0 * (t + 1e-3) + E) +
+                                4.0 * 5.9604644775390625e-08 * (tolsq + 0.01));
+    const float lo32 = __double2float_rd(tolsq - band), hi32 = __double2float_ru(tolsq + band);
+#pragma unroll
+    for (int e = 0; e < 9; e++) {
+        u32[e] = __double2float_rn(u[e]);
+        rs[e] = rc[e] = 0.f;
+    }
+    // kU peaks per lane per step: all their loads are issued before any is used
+    constexpr int kU = 4;
+    const double* p = first;
+    for (int k = tid; k < n; k += kU * N, p += 3 * kU * N) {
+        double gg[kU][3];
+#pragma unroll
+        for (int q = 0; q < kU; q++)
+            if (k + q * N < n)
+#pragma unroll
+                for (int i = 0; i < 3; i++) gg[q][i] = __ldg(p + 3 * q * N + i);
+#pragma unroll
+        for (int q = 0; q < kU; q++) {
+            if (k + q * N >= n) break;
+            // g split exactly enough into hi + lo floats
+            float gh[3], gl[3], ihf[3], d[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                gh[i] = __double2float_rn(gg[q][i]);
+                gl[i] = __double2float_rn(gg[q][i] - (double)gh[i]);
+            }
+            const float M = 12582912.0f;  // 1.5 * 2^23
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const float h = fmaf(u32[3 * r + 2], gh[2],
+                                     fmaf(u32[3 * r + 1], gh[1], u32[3 * r] * gh[0]));
+                ihf[r] = __fsub_rn(__fadd_rn(h, M), M);
+                d[r] = h - ihf[r];
+            }
+            float s32 = fmaf(d[2], d[2], fmaf(d[1], d[1], d[0] * d[0]));
+            if (!(s32 < hi32)) continue;
+            if (!(s32 < lo32)) {  // inside the band: the exact decision
+                double ih[3];
+                const double s = drlv2_exact(u, gg[q][0], gg[q][1], gg[q][2], ih);
+                if (!(s < tolsq)) continue;
+#pragma unroll
+                for (int r = 0; r < 3; r++) ihf[r] = (float)ih[r];
+                s32 = (float)s;
+            }
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    // ih_j * g_i = ih_j * gh_i (TwoProduct) + ih_j * gl_i
+                    const float pr = ihf[j] * gh[i];
+                    const float pe = fmaf(ihf[j], gh[i], -pr);
+                    comp_add(rs[3 * i + j], rc[3 * i + j], pr);
+                    rc[3 * i + j] += pe + ihf[j] * gl[i];
+                }
+            const int a = (int)ihf[0], b = (int)ihf[1], c = (int)ihf[2];
+            hint[0] += a * a;
+            hint[1] += b * a;
+            hint[2] += c * a;
+            hint[3] += b * b;
+            hint[4] += c * b;
+            hint[5] += c * c;
+            comp_add(ss32, sc32, s32);
+            nacc++;
+        }
+    }
+    // to FP64 for the fixed reduction: s + c, exact integers
+#pragma unroll
+    for (int e = 0; e < 9; e++) acc[e] = (double)rs[e] + (double)rc[e];
+#pragma unroll
+    for (int e = 0; e < 6; e++) acc[9 + e] = (double)hint[e];
+    acc[15] = (double)ss32 + (double)sc32;
+}
+
+// `iters` rounds of one grain by N threads (tid of them; N == 32: one warp of the
+// CTA by itself).  red: N / 32 rows of per-warp partial sums.  V > 1 (N == 32):
+// the warp does the work of V warps in turn, peak by peak and sum by sum as they
+// would, so the result has the same bits.
+template <int N, bool F32C, int V = 1>
+__device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], int tid, int g,
+                                             double* __restrict__ ubis,
+                                             const double* __restrict__ gv, int64_t k0, int n,
+                                             double tolsq, int iters, int* __restrict__ npk,
+                                             double* __restrict__ mean, double gmax) {
+    const int lane = tid & 31, w = tid >> 5;
+    auto sync = [] {
+        if (N == 32) __syncwarp(); else __syncthreads();
+    };
+    const int field = slot_of<17>(lane);
+    if (tid < 9) sm.ubi[tid] = ubis[9 * (int64_t)g + tid];
+    sync();
+    for (int it = 0; it < iters; it++) {
+        double u[9];
+#pragma unroll
+        for (int e = 0; e < 9; e++) u[e] = sm.ubi[e];
+        double part = 0.;
+#pragma unroll 1
+        for (int v = 0; v < V; v++) {
+            const int first = tid + 32 * v;
+            double acc[17];
+#pragma unroll
+            for (int f = 0; f < 17; f++) acc[f] = 0.;
+            int nacc = 0;
+            if (F32C)
+                refine_peaks_f32c<N * V>(u, gv + 3 * (k0 + first), first, n, tolsq, gmax, acc, nacc);
+            else
+                refine_peaks<N * V>(u, gv + 3 * (k0 + first), first, n, tolsq, acc, nacc);
+            acc[16] = (double)nacc;
+            part += ScatterSum<17, 16>::run(acc, lane);
+        }
+        if (field >= 0) red[w][field] = part;
+        sync();
+        if (w == 0) {
+            double t = 0.;
+            if (lane < 17)
+                for (int q = 0; q < N / 32; q++) t += red[q][lane];
+            // t: R in lanes 0 .. 8, H's upper triangle 9 .. 14, sum, n
+            if (lane < 9) sm.R[lane] = t;
+            const int e = lane < 9 ? lane : 0;
+            const double h = __shfl_sync(0xffffffffu, t, 9 + h_slot(e));
+            if (lane < 9) sm.H[lane] = h;
+            const double ss = __shfl_sync(0xffffffffu, t, 15);
+            const long long np = (long long)__shfl_sync(0xffffffffu, t, 16);
+            __syncwarp();
+            // UB = R . inv(H); UBI = inv(UB); keep ubi unless both inverses exist
+            const double det = det3_exact(sm.H);
+            const double hi = det != 0. ? inv3_elem(sm.H, det, e) : 0.;
+            const int i = e / 3, j = e - 3 * i;
+            double s = 0.;
+#pragma unroll
+            for (int l = 0; l < 3; l++)
+                s = dadd(s, dmul(sm.R[3 * i + l], __shfl_sync(0xffffffffu, hi, 3 * l + j)));
+            if (lane < 9) sm.UB[lane] = s;
+            __syncwarp();
+            const double det2 = det3_exact(sm.UB);
+            if (lane < 9 && det != 0. && det2 != 0.) sm.ubi[lane] = inv3_elem(sm.UB, det2, e);
+            if (lane == 0 && it == iters - 1) {
+                if (npk) npk[g] = (int)np;
+                if (mean) mean[g] = np > 0 ? ddiv(ss, (double)np) : 0.;
+            }
+        }
+        sync();
+    }
+    if (tid < 9) ubis[9 * (int64_t)g + tid] = sm.ubi[tid];
+    sync();
+}
+
+// Persistent mode with more grains than CTAs: CTAs of NT threads take grains of
+// more than kSolo peaks whole; from the first smaller one on, each of a CTA's
+// warps takes grains by itself, so that the rounds' fixed part (the reduction
+// and the 3x3 solves, which one warp does) of several grains overlap.  A larger
+// grain met after that (an order that is not by size) is done by one warp as the
+// CTA would, so a grain's result depends on its size alone.
+//
+// Bound: instruction issue and FP64 latency at 16 resident warps (123
+// registers), then the largest grains' own five rounds.  2,000 grains of 20 ..
+// 2,000 peaks (859k), five rounds: 36.6 us with 128 threads, 42 with 64; 55.9 (64)
+// and 80.2 (128) with a CTA for every grain, 17 warp sums and five barriers a
+// round.  500 such grains 36.0 -> 17.0, 8,000 of up to 400 peaks, three rounds, 86
+// -> 35 us.  kSolo at 128 threads: 256 43.0, 512 43.2, 768 36.6, 1,024 41.9 us.
+constexpr int kSolo = 768;
+
 template <int NT, bool F32C = false>
 __global__ void __launch_bounds__(NT)
 k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
              const int64_t* __restrict__ off, const int* __restrict__ order, int ngrains,
              double tolsq, int iters, int* __restrict__ queue, int* __restrict__ npk,
              double* __restrict__ mean, double gmax) {
-    __shared__ RefineSmem<NT> sm;
+    __shared__ RefineSmem sm[NT / 32];
+    __shared__ double s_red[NT / 32][17];
+    __shared__ int s_next;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    for (int slot = blockIdx.x;; slot += gridDim.x) {
-        if (queue) {
-            if (tid == 0) sm.grain = atomicAdd(queue, 1);
-            __syncthreads();
-            slot = sm.grain;
-        }
-        if (slot >= ngrains) break;
+    int slot = blockIdx.x;
+    while (slot < ngrains) {
         const int g = order ? order[slot] : slot;
-        const int64_t k0 = off[g], k1 = off[g + 1];
-        if (tid < 9) sm.ubi[tid] = ubis[9 * (int64_t)g + tid];
-        __syncthreads();
-        for (int it = 0; it < iters; it++) {
-            double u[9];
-#pragma unroll
-            for (int e = 0; e < 9; e++) u[e] = sm.ubi[e];
-            double acc[17];
-#pragma unroll
-            for (int f = 0; f < 17; f++) acc[f] = 0.;
-            // F32C: screening thresholds of the proven band (score_batch.cu) for
-            // this UBI, FP32 copy of the UBI, compensated R and drlv2 sums,
-            // exact integer H
-            float lo32 = 0.f, hi32 = 0.f, u32[9], rs[9], rc[9], ss32 = 0.f, sc32 = 0.f;
-            int hint[6] = {0, 0, 0, 0, 0, 0}, nacc = 0;
-            if (F32C) {
-                double S = 0.;
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-                    S = fmax(S, fabs(u[3 * r]) + fabs(u[3 * r + 1]) + fabs(u[3 * r + 2]));
-                const double E = 6.0 * 5.9604644775390625e-08 * S * (1. + 1e-15) * gmax;
-                const double t = sqrt(tolsq);
-                const double band = 1.25 * (3.0 * E * (2.0 * (t + 1e-3) + E) +
-                                            4.0 * 5.9604644775390625e-08 * (tolsq + 0.01));
-                lo32 = __double2float_rd(tolsq - band);
-                hi32 = __double2float_ru(tolsq + band);
-#pragma unroll
-                for (int e = 0; e < 9; e++) {
-                    u32[e] = __double2float_rn(u[e]);
-                    rs[e] = rc[e] = 0.f;
-                }
-            }
-            // kU peaks per lane per step: all their loads are issued before any
-            // is used, so one memory latency covers kU peaks (the segment is
-            // read-only and re-read every round, so later rounds hit L1)
-            constexpr int kU = 4;
-            for (int64_t kb = k0 + tid; kb < k1; kb += kU * NT) {
-                double gg[kU][3];
-#pragma unroll
-                for (int q = 0; q < kU; q++) {
-                    const int64_t k = kb + (int64_t)q * NT;
-                    if (k < k1) {
-                        gg[q][0] = __ldg(gv + 3 * k);
-                        gg[q][1] = __ldg(gv + 3 * k + 1);
-                        gg[q][2] = __ldg(gv + 3 * k + 2);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kU; q++) {
-                    if (kb + (int64_t)q * NT >= k1) break;
-                    if (F32C) {
-                        // g split exactly enough into hi + lo floats
-                        float gh[3], gl[3], ihf[3], t[3];
-#pragma unroll
-                        for (int i = 0; i < 3; i++) {
-                            gh[i] = __double2float_rn(gg[q][i]);
-                            gl[i] = __double2float_rn(gg[q][i] - (double)gh[i]);
-                        }
-                        const float M = 12582912.0f;  // 1.5 * 2^23
-#pragma unroll
-                        for (int r = 0; r < 3; r++) {
-                            const float h = fmaf(u32[3 * r + 2], gh[2],
-                                                 fmaf(u32[3 * r + 1], gh[1], u32[3 * r] * gh[0]));
-                            ihf[r] = __fsub_rn(__fadd_rn(h, M), M);
-                            t[r] = h - ihf[r];
-                        }
-                        float s32 = fmaf(t[2], t[2], fmaf(t[1], t[1], t[0] * t[0]));
-                        if (!(s32 < hi32)) continue;
-                        if (!(s32 < lo32)) {  // inside the band: the exact decision
-                            double ih[3];
-                            const double s = drlv2_exact(u, gg[q][0], gg[q][1], gg[q][2], ih);
-                            if (!(s < tolsq)) continue;
-#pragma unroll
-                            for (int r = 0; r < 3; r++) ihf[r] = (float)ih[r];
-                            s32 = (float)s;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 3; i++)
-#pragma unroll
-                            for (int j = 0; j < 3; j++) {
-                                // ih_j * g_i = ih_j * gh_i (TwoProduct) + ih_j * gl_i
-                                const float p = ihf[j] * gh[i];
-                                const float pe = fmaf(ihf[j], gh[i], -p);
-                                comp_add(rs[3 * i + j], rc[3 * i + j], p);
-                                rc[3 * i + j] += pe + ihf[j] * gl[i];
-                            }
-                        const int a = (int)ihf[0], b = (int)ihf[1], c = (int)ihf[2];
-                        hint[0] += a * a;
-                        hint[1] += b * a;
-                        hint[2] += c * a;
-                        hint[3] += b * b;
-                        hint[4] += c * b;
-                        hint[5] += c * c;
-                        comp_add(ss32, sc32, s32);
-                        nacc++;
-                        continue;
-                    }
-                    double ih[3];
-                    const double s = drlv2_exact(u, gg[q][0], gg[q][1], gg[q][2], ih);
-                    if (!(s < tolsq)) continue;
-                    // normal equations with fused multiply-adds: H (products of
-                    // integers) is exact either way; each R term is rounded once
-                    // instead of twice -- R is order-dependent against the
-                    // reference's sequential sum in any case
-#pragma unroll
-                    for (int i = 0; i < 3; i++)
-#pragma unroll
-                        for (int j = 0; j < 3; j++)
-                            acc[3 * i + j] = fma(ih[j], gg[q][i], acc[3 * i + j]);
-                    acc[9] = fma(ih[0], ih[0], acc[9]);
-                    acc[10] = fma(ih[1], ih[0], acc[10]);
-                    acc[11] = fma(ih[2], ih[0], acc[11]);
-                    acc[12] = fma(ih[1], ih[1], acc[12]);
-                    acc[13] = fma(ih[2], ih[1], acc[13]);
-                    acc[14] = fma(ih[2], ih[2], acc[14]);
-                    acc[15] = dadd(acc[15], s);
-                    acc[16] += 1.0;
-                }
-            }
-            if (F32C) {  // to FP64 for the fixed reduction: s + c, exact integers
-#pragma unroll
-                for (int e = 0; e < 9; e++) acc[e] = (double)rs[e] + (double)rc[e];
-#pragma unroll
-                for (int e = 0; e < 6; e++) acc[9 + e] = (double)hint[e];
-                acc[15] = (double)ss32 + (double)sc32;
-                acc[16] = (double)nacc;
-            }
-#pragma unroll
-            for (int f = 0; f < 17; f++) acc[f] = warp_sum(acc[f]);
-            if (lane == 0)
-#pragma unroll
-                for (int f = 0; f < 17; f++) sm.red[w][f] = acc[f];
-            __syncthreads();
-            if (tid < 17) {
-                double t = 0.;
-                for (int q = 0; q < NT / 32; q++) t += sm.red[q][tid];
-                if (tid < 9) {
-                    sm.R[tid] = t;
-                } else if (tid < 15) {
-                    const int i = c_hrow[tid - 9], j = c_hcol[tid - 9];
-                    sm.H[3 * i + j] = t;  // identical sums for (i,j) and (j,i)
-                    sm.H[3 * j + i] = t;
-                } else if (tid == 15) {
-                    sm.ss = t;
-                } else {
-                    sm.n = (long long)t;
-                }
-            }
-            __syncthreads();
-            // UB = R . inv(H); UBI = inv(UB); keep ubi unless both inverses exist
-            if (tid < 9) {
-                const double det = det3_exact(sm.H);
-                if (tid == 0) sm.ok = det != 0.;
-                if (det != 0.) sm.Hi[tid] = inv3_elem(sm.H, det, tid);
-            }
-            __syncthreads();
-            if (tid < 9 && sm.ok) {
-                const int i = tid / 3, j = tid % 3;
-                double s = 0.;
-                s = dadd(s, dmul(sm.R[3 * i + 0], sm.Hi[0 + j]));
-                s = dadd(s, dmul(sm.R[3 * i + 1], sm.Hi[3 + j]));
-                s = dadd(s, dmul(sm.R[3 * i + 2], sm.Hi[6 + j]));
-                sm.UB[tid] = s;
-            }
-            __syncthreads();
-            if (tid < 9 && sm.ok) {
-                const double det = det3_exact(sm.UB);
-                if (tid == 0) sm.ok2 = det != 0.;
-                if (det != 0.) sm.UBI[tid] = inv3_elem(sm.UB, det, tid);
-            }
-            __syncthreads();
-            if (tid < 9 && sm.ok && sm.ok2) sm.ubi[tid] = sm.UBI[tid];
-            if (tid == 0 && it == iters - 1) {
-                if (npk) npk[g] = (int)sm.n;
-                if (mean) mean[g] = sm.n > 0 ? ddiv(sm.ss, (double)sm.n) : 0.;
-            }
-            __syncthreads();
+        const int64_t k0 = off[g];
+        const int n = (int)(off[g + 1] - k0);
+        if (NT > 32 && queue && ngrains > (int)gridDim.x && n <= kSolo) break;
+        if (tid == 0) s_next = queue ? (int)gridDim.x + atomicAdd(queue, 1) : ngrains;
+        refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
+                               gmax);
+        slot = s_next;
+        if (NT == 32) __syncwarp(); else __syncthreads();
+    }
+    if (NT == 32) return;
+    // one warp per grain: warp 0 begins with the CTA's
+    int mine = slot;
+    if (w > 0) {
+        mine = ngrains;
+        if (slot < ngrains) {
+            if (lane == 0) mine = (int)gridDim.x + atomicAdd(queue, 1);
+            mine = __shfl_sync(0xffffffffu, mine, 0);
         }
-        if (tid < 9) ubis[9 * (int64_t)g + tid] = sm.ubi[tid];
-        __syncthreads();
-        if (!queue && slot + (int)gridDim.x >= ngrains) break;  // plain: one grain per CTA
+    }
+    while (mine < ngrains) {
+        const int g = order ? order[mine] : mine;
+        const int64_t k0 = off[g];
+        const int n = (int)(off[g + 1] - k0);
+        int next = 0;
+        if (lane == 0) next = (int)gridDim.x + atomicAdd(queue, 1);
+        if (n <= kSolo)
+            refine_grain<32, F32C>(sm[w], s_red + w, lane, g, ubis, gv, k0, n, tolsq, iters, npk,
+                                   mean, gmax);
+        else
+            refine_grain<32, F32C, NT / 32>(sm[w], s_red + w, lane, g, ubis, gv, k0, n, tolsq,
+                                            iters, npk, mean, gmax);
+        mine = __shfl_sync(0xffffffffu, next, 0);
     }
 }
 

@@ -379,9 +379,11 @@ int id11b_dev_refine_batch(double *ubis, int64_t m, const double *gv, const floa
  * grains from a work counter in `workspace` (id11b_refine_csr_workspace_bytes());
  * persistent == 0: one CTA per grain, the plain baseline (call once per round).
  * npk / mean_drlv2 (optional, ngrains) receive the last round's count and mean
- * drlv2.  threads: CTA size 32, 64, 128, 256 or 512 (0 = 128); small CTAs keep
- * more grains in flight (64 is fastest for 2,000 grains of 20..1,500 peaks).  Exact FP64 per pair; the persistent launch (counter reset + kernel)
- * can be captured in a CUDA graph and replayed. */
+ * drlv2.  threads: CTA size 32, 64, 128, 256 or 512 (0 = 128, the fastest for
+ * 2,000 grains of 20..2,000 peaks); with more grains than resident CTAs, grains
+ * of up to 768 peaks are refined by one warp each.  Exact FP64 per pair; the
+ * persistent launch (counter reset + kernel) can be captured in a CUDA graph and
+ * replayed. */
 int64_t id11b_refine_csr_workspace_bytes(void);
 int id11b_dev_refine_csr(double *ubis, const double *gv, const int64_t *offsets,
                          const int32_t *order, int32_t ngrains, double tol, int iters,

@@ -89,3 +89,36 @@ def test_refine_csr_compensated_fp32(grains, oracle, cuda):
     # the mean drlv2 is a sum of FP32 per-peak values (each within the
     # screening band of the exact one): about 1e-6 relative here
     assert np.all(np.abs(mean - ref_m) <= 1e-4 * np.abs(ref_m) + 1e-18)
+
+
+@pytest.mark.parametrize("threads", [32, 64, 128, 256, 512])
+@pytest.mark.parametrize("ordered", [True, False])
+def test_refine_csr_more_grains_than_ctas(oracle, threads, ordered, cuda):
+    """More grains than resident CTAs: grains on both sides of the size one warp
+    takes, empty and tiny ones, in order of size and not (a large grain met by a
+    warp working alone): the oracle's rounds, and the same bits in both orders."""
+    import torch
+    from imaged11_b200 import batch, synth
+    from imaged11_b200._lib import lib, check
+    rng = np.random.default_rng(43)
+    counts = rng.integers(20, 41, 5200)
+    counts[:12] = [0, 1, 2, 31, 32, 33, 767, 768, 769, 1537, 2000, 770]
+    rng.shuffle(counts)
+    gv, off, ubis = synth.grain_gvectors(counts, "Ti_hcp", rng)
+    u0 = synth.perturb_ubis(ubis, 0.2, 0.002, rng)
+    ref_u, ref_n, ref_m = oracle.refine_csr(u0, gv, off, 0.05, 3)
+    gs = batch.GrainSet(gv, off, u0, threads=threads)
+    u, npk, mean = gs.refine(0.05, 3)
+    u = u.cpu().numpy()
+    if not ordered:
+        other = torch.tensor(u0, device=cuda).contiguous()
+        check(lib.id11b_dev_refine_csr(other.data_ptr(), gs.gv.data_ptr(), gs.offsets.data_ptr(),
+                                       None, gs.ngrains, 0.05, 3, 1, threads, npk.data_ptr(),
+                                       mean.data_ptr(), gs.ws.data_ptr(), gs.ws.numel(), None),
+              "refine_csr")
+        torch.cuda.synchronize()
+        assert np.array_equal(other.cpu().numpy(), u)
+    big = ref_n > 3     # (up to three peaks the normal matrix is singular to rounding)
+    _check(u[big], npk.cpu().numpy()[big], mean.cpu().numpy()[big], ref_u[big], ref_n[big],
+           ref_m[big])
+    assert np.array_equal(npk.cpu().numpy(), ref_n)
