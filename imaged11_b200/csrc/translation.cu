@@ -22,7 +22,9 @@
 // derivative of the cost through U1 vanishes.  The sums J^T J, J^T r and the
 // cost are reduced in a fixed order and a Levenberg-Marquardt step is taken;
 // a step that raises the cost is undone and the damping raised.  One CTA per
-// grain, every iteration in one launch.
+// grain, every iteration in one launch; sin and cos of a peak's omega, and the
+// 1 / |d| that the second pass shares with the first, are kept in shared memory
+// by the thread that owns the peak.
 #include <math.h>
 
 #include "common.cuh"
@@ -30,12 +32,10 @@
 namespace id11b {
 namespace trans {
 
-// threads per grain (500 grains of ~650 peaks, 30 iterations on B200: 64 and 128
-// threads 0.44 ms, 256 threads 0.53 ms, the call's host work included)
-#ifndef ID11B_TRANS_THREADS
-#define ID11B_TRANS_THREADS 64
-#endif
-constexpr int kTT = ID11B_TRANS_THREADS;
+constexpr int kTT = 64;  // threads per grain
+// peaks per thread kept in shared memory (three doubles each: 24 KB a CTA); the
+// peaks of a larger grain beyond 64 x 16 are computed in each pass
+constexpr int kKeep = 16;
 constexpr double kRad = 3.14159265358979323846 / 180.0;
 
 struct Geo {
@@ -49,14 +49,17 @@ struct Acc {
     double a[11];
 };
 
-// g of one peak at translation t, with what its tangents need
+// g of one peak at translation t, with what its tangents need; so and co (and inv
+// when HAVE) given.  Near the minimum a step is taken or refused by the last bits
+// of the cost, so the passes compute g each in its own way, as they always did:
+// taking the first pass's g in the second moves t by 1e-8 of itself.
 struct PeakG {
     double so, co, n0, n1, n2, inv, g[3];
 };
 
+template <bool HAVE>
 __device__ __forceinline__ void peak_g(const Geo& P, const double t[3], double x0, double x1,
-                                       double x2, double om, PeakG& q) {
-    sincos(kRad * om * P.omegasign, &q.so, &q.co);
+                                       double x2, PeakG& q) {
     const double* M = P.m;
     const double so = q.so, co = q.co;
     // o = M.A.t, A = [[co,-so,0],[so,co,0],[0,0,1]]
@@ -64,7 +67,7 @@ __device__ __forceinline__ void peak_g(const Geo& P, const double t[3], double x
     const double d0 = x0 - (M[0] * at0 + M[1] * at1 + M[2] * at2);
     const double d1 = x1 - (M[3] * at0 + M[4] * at1 + M[5] * at2);
     const double d2 = x2 - (M[6] * at0 + M[7] * at1 + M[8] * at2);
-    q.inv = 1.0 / sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+    if (!HAVE) q.inv = 1.0 / sqrt(d0 * d0 + d1 * d1 + d2 * d2);
     q.n0 = d0 * q.inv;
     q.n1 = d1 * q.inv;
     q.n2 = d2 * q.inv;
@@ -79,11 +82,8 @@ __device__ __forceinline__ void peak_g(const Geo& P, const double t[3], double x
 
 // first pass: R (9, R[i][j] = sum h_j g_i) and H (6, upper) of the peaks
 // with drlv2(u0) < tol^2, as score_and_refine sums them
-__device__ __forceinline__ void refit_terms(const Geo& P, const double u[9], const double t[3],
-                                            double x0, double x1, double x2, double om,
+__device__ __forceinline__ void refit_terms(const Geo& P, const double u[9], const PeakG& q,
                                             double* a) {
-    PeakG q;
-    peak_g(P, t, x0, x1, x2, om, q);
     double ih[3], r[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -106,11 +106,8 @@ __device__ __forceinline__ void refit_terms(const Geo& P, const double u[9], con
 }
 
 // second pass: cost and Gauss-Newton sums at u
-__device__ __forceinline__ void peak_terms(const Geo& P, const double u[9], const double t[3],
-                                           double x0, double x1, double x2, double om,
+__device__ __forceinline__ void peak_terms(const Geo& P, const double u[9], const PeakG& q,
                                            Acc& acc) {
-    PeakG q;
-    peak_g(P, t, x0, x1, x2, om, q);
     const double* M = P.m;
     const double so = q.so, co = q.co, n0 = q.n0, n1 = q.n1, n2 = q.n2, inv = q.inv;
     double r[3];
@@ -172,25 +169,33 @@ __device__ __forceinline__ bool solve3(const double h[6], const double b[3], dou
     return isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]);
 }
 
-// U1 = (R H^-1)^-1 from the first pass's sums; false (U1 left as u0) when
-// H or R H^-1 is singular, as score_and_refine leaves its UBI
-__device__ bool refit_ubi(const double* a, const double u0[9], double u1[9]) {
-    double H[9] = {a[9], a[10], a[11], a[10], a[12], a[13], a[11], a[13], a[14]};
+// U1 = (R H^-1)^-1 from the first pass's sums (a: lane q < 15 holds the q-th), one
+// element per lane, by one warp; u0 when H or R H^-1 is singular, as
+// score_and_refine leaves its UBI.  m: nine doubles of scratch in shared memory.
+__device__ __forceinline__ double refit_ubi(double a, double u0, double* m, int lane) {
+    const int e = lane < 9 ? lane : 0, i = e / 3, j = e - 3 * i;
+    const double h = __shfl_sync(0xffffffffu, a, 9 + (i + j + (min(i, j) > 0)));
+    if (lane < 9) m[e] = h;
+    __syncwarp();
+    const double det = det3_exact(m);
+    const double hi = det != 0. ? inv3_elem(m, det, e) : 0.;
+    double r[3], c[3];
 #pragma unroll
-    for (int e = 0; e < 9; e++) u1[e] = u0[e];
-    if (inverse3x3_exact(H) != 0) return false;
-    double UB[9];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            UB[3 * i + j] = a[3 * i] * H[j] + a[3 * i + 1] * H[3 + j] + a[3 * i + 2] * H[6 + j];
-    if (inverse3x3_exact(UB) != 0) return false;
-#pragma unroll
-    for (int e = 0; e < 9; e++) u1[e] = UB[e];
-    return true;
+    for (int l = 0; l < 3; l++) {
+        r[l] = __shfl_sync(0xffffffffu, a, 3 * i + l);
+        c[l] = __shfl_sync(0xffffffffu, hi, 3 * l + j);
+    }
+    __syncwarp();
+    if (lane < 9) m[e] = r[0] * c[0] + r[1] * c[1] + r[2] * c[2];
+    __syncwarp();
+    const double det2 = det3_exact(m);
+    return det != 0. && det2 != 0. ? inv3_elem(m, det2, e) : u0;
 }
 
+// Bound: the FP64 pipe of the SMs that hold four grains (500 grains are 3.4 CTAs
+// per SM), at two warps per scheduler.  500 grains of 420 .. 560 peaks, 30
+// iterations: 0.31 ms; 0.43 with sin, cos and 1 / |d| taken in every pass, full
+// butterflies and one thread's 3x3 solves.  Two or four peaks at a time: 0.32, 0.35.
 __global__ void __launch_bounds__(kTT)
 k_refine_translations(const double* __restrict__ xyz, const double* __restrict__ omega,
                       const int64_t* __restrict__ offsets, int32_t ngrains,
@@ -198,15 +203,28 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
                       double* __restrict__ cost_out, int32_t* __restrict__ npk_out,
                       double* __restrict__ ubi_out) {
     __shared__ double s_red[kTT / 32][15];
-    __shared__ double s_t[3];
-    __shared__ double s_u[9];
+    __shared__ double s_t[3], s_u[9], s_m[9];
+    extern __shared__ double s_keep[];  // [field][peak of the thread][thread]
     const int gi = blockIdx.x;
     if (gi >= ngrains) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int64_t p0 = offsets[gi], p1 = offsets[gi + 1];
+    const int64_t p0 = offsets[gi];
+    const int np = (int)(offsets[gi + 1] - p0);
+    double* const keep = s_keep + tid;
+    constexpr int kF = kKeep * kTT;  // doubles per field
+    auto angles = [&](int k, PeakG& q) {
+        sincos(kRad * omega[p0 + k] * P.omegasign, &q.so, &q.co);
+    };
+    for (int i = 0, k = tid; k < np && i < kKeep; i++, k += kTT) {
+        PeakG q;
+        angles(k, q);
+        keep[i * kTT] = q.so;
+        keep[kF + i * kTT] = q.co;
+    }
     double u0[9];
 #pragma unroll
     for (int e = 0; e < 9; e++) u0[e] = ubis[9 * gi + e];
+    const double u0e = ubis[9 * gi + (lane < 9 ? lane : 0)];
     double tacc[3] = {tr[3 * gi], tr[3 * gi + 1], tr[3 * gi + 2]};
     double hacc[6] = {0, 0, 0, 0, 0, 0}, bacc[3] = {0, 0, 0}, cacc = 0., nacc = 0.;
     double uacc[9];
@@ -225,23 +243,31 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         double a[15];
 #pragma unroll
         for (int q = 0; q < 15; q++) a[q] = 0.;
-        for (int64_t k = p0 + tid; k < p1; k += kTT)
-            refit_terms(P, u0, t, xyz[3 * k], xyz[3 * k + 1], xyz[3 * k + 2], omega[k], a);
-#pragma unroll
-        for (int q = 0; q < 15; q++) {
-            const double v = warp_sum(a[q]);
-            if (lane == 0) s_red[wid][q] = v;
+        for (int i = 0, k = tid; k < np; i++, k += kTT) {
+            const double* x = xyz + 3 * (p0 + k);
+            PeakG q;
+            if (i < kKeep) {
+                q.so = keep[i * kTT];
+                q.co = keep[kF + i * kTT];
+            } else {
+                angles(k, q);
+            }
+            peak_g<false>(P, t, x[0], x[1], x[2], q);
+            if (i < kKeep) keep[2 * kF + i * kTT] = q.inv;
+            refit_terms(P, u0, q, a);
+        }
+        {
+            const int f = slot_of<15>(lane);
+            const double v = ScatterSum<15, 16>::run(a, lane);
+            if (f >= 0) s_red[wid][f] = v;
         }
         __syncthreads();
-        if (tid == 0) {
-            double r[15];
-            for (int q = 0; q < 15; q++) {
-                r[q] = 0.;
-                for (int w = 0; w < kTT / 32; w++) r[q] += s_red[w][q];  // fixed order
-            }
-            double u1[9];
-            refit_ubi(r, u0, u1);
-            for (int e = 0; e < 9; e++) s_u[e] = u1[e];
+        if (wid == 0) {
+            double v = 0.;
+            if (lane < 15)
+                for (int w = 0; w < kTT / 32; w++) v += s_red[w][lane];  // fixed order
+            v = refit_ubi(v, u0e, s_m, lane);
+            if (lane < 9) s_u[lane] = v;
         }
         __syncthreads();
         double u1[9];
@@ -251,12 +277,24 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         Acc acc;
 #pragma unroll
         for (int q = 0; q < 11; q++) acc.a[q] = 0.;
-        for (int64_t k = p0 + tid; k < p1; k += kTT)
-            peak_terms(P, u1, t, xyz[3 * k], xyz[3 * k + 1], xyz[3 * k + 2], omega[k], acc);
-#pragma unroll
-        for (int q = 0; q < 11; q++) {
-            const double v = warp_sum(acc.a[q]);
-            if (lane == 0) s_red[wid][q] = v;
+        for (int i = 0, k = tid; k < np; i++, k += kTT) {
+            PeakG q;
+            const double* x = xyz + 3 * (p0 + k);
+            if (i < kKeep) {
+                q.so = keep[i * kTT];
+                q.co = keep[kF + i * kTT];
+                q.inv = keep[2 * kF + i * kTT];
+                peak_g<true>(P, t, x[0], x[1], x[2], q);
+            } else {
+                angles(k, q);
+                peak_g<false>(P, t, x[0], x[1], x[2], q);
+            }
+            peak_terms(P, u1, q, acc);
+        }
+        {
+            const int f = slot_of<11>(lane);
+            const double v = ScatterSum<11, 16>::run(acc.a, lane);
+            if (f >= 0) s_red[wid][f] = v;
         }
         __syncthreads();
         if (tid == 0) {
@@ -334,7 +372,8 @@ extern "C" int id11b_dev_refine_translations(const double* xyz, const double* om
     P.omegasign = omegasign;
     P.ds = 1.0 / wvln;
     P.tol2 = tol * tol;
-    k_refine_translations<<<(unsigned)ngrains, kTT, 0, (cudaStream_t)stream>>>(
+    k_refine_translations<<<(unsigned)ngrains, kTT, sizeof(double) * 3 * kKeep * kTT,
+                            (cudaStream_t)stream>>>(
         xyz, omega, offsets, ngrains, ubis, translations, P, iters, cost, npk, ubis_refit);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;

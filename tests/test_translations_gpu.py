@@ -72,3 +72,31 @@ def test_recovers_translations(scene, oracle, cuda):
                        options={"xatol": 1e-3, "fatol": 1e-12, "maxiter": 2000})
         c_gn, _ = oracle_cost(oracle, xyz[a:b], om[a:b], ps.ubis[g], t[g], geo)
         assert c_gn <= res.fun * (1 + 1e-6) + 1e-12, (g, c_gn, res.fun)
+
+
+def test_grain_sizes(oracle, cuda):
+    """Grains of a few peaks, around one CTA's threads and around what a thread
+    keeps in shared memory (64 x 16 peaks): the objective at each grain's own
+    translation (1e-9 relative, as above) and a cost that does not rise."""
+    from imaged11_b200 import batch, synth
+    geo = synth.default_geometry(distance=152300.0, tilt_x=0.004, wedge=0.01, chi=0.02)
+    sizes = [4, 5, 63, 64, 65, 129, 1023, 1024, 1025, 1150]
+    ps = synth.simulate(len(sizes), "Ti_hcp", gmax=1.75, seed=83, geo=geo, noise_frac=0.0,
+                        translations_um=60.0)
+    idx, off = ps.grain_offsets()
+    assert np.diff(off).min() >= max(sizes)
+    keep = np.concatenate([idx[off[g]:off[g] + k] for g, k in enumerate(sizes)])
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    p, r, dist = synth.xlylzl_params(geo)
+    xyz = oracle.compute_xlylzl(ps.s[keep], ps.f[keep], p, r, dist)
+    om = ps.omega[keep]
+    t0 = np.random.default_rng(84).uniform(-40, 40, (len(sizes), 3))
+    args = (geo["omegasign"], geo["wavelength"], geo["wedge"], geo["chi"])
+    _, cost, npk = batch.refine_translations(xyz, om, off, ps.ubis, t0, *args, iters=0)
+    for g in range(len(sizes)):
+        a, b = off[g], off[g + 1]
+        c, n = oracle_cost(oracle, xyz[a:b], om[a:b], ps.ubis[g], t0[g], geo)
+        assert int(npk[g]) == n
+        assert abs(float(cost[g]) - c) <= 1e-9 * c + 1e-15
+    _, after, _ = batch.refine_translations(xyz, om, off, ps.ubis, t0, *args, iters=5)
+    assert bool((after <= cost).all()) and bool((after[2:] < cost[2:]).all())
