@@ -749,22 +749,36 @@ k_refine(const double* __restrict__ ubis, int64_t m, Split sp, const Header* __r
     }
 }
 
-// The g-vectors outside the regular range, one warp per UBI: normal-equation
-// terms of the pairs below tol^2 (lanes stride the list, fixed-tree sums).
+// One warp per UBI: the items' partials in item order (lane f takes field f), then
+// the normal-equation terms of the g outside the regular range (lanes stride the
+// list, fixed-tree sums), then the reference's update; n and mean drlv2 of the UBI
+// as it was on entry.  Seventeen lanes load an item's row at once: 2,000 UBIs x 10
+// items take 5.5 us; 14.5 with one thread per UBI, and 4 for a kernel of its own
+// for the list.
 __global__ void __launch_bounds__(kGT)
-k_refine_special(const double* __restrict__ ubis, int64_t m, double tol,
-                 const double* __restrict__ gv, const int* __restrict__ special,
-                 const int* __restrict__ nspecial, double* __restrict__ spart) {
+k_refine_finish(double* __restrict__ ubis, int64_t m, int parts,
+                const double* __restrict__ part_in, double tol, const double* __restrict__ gv,
+                const int* __restrict__ special, const int* __restrict__ nspecial,
+                int* __restrict__ npk, double* __restrict__ mean) {
     __shared__ double s_lsq[kGT / 32][kLsqF * 32];
+    __shared__ double s_t[kGT / 32][kLsqF];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t i = ((int64_t)blockIdx.x * kGT + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
     if (i >= m) return;  // uniform per warp
-    double* acc = s_lsq[threadIdx.x >> 5] + lane;
-    for (int f = 0; f < kLsqF; f++) acc[f * 32] = 0.;
+    double t = 0.;
+    if (lane < kLsqF) {
+        const double* p = part_in + i * parts * kLsqF + lane;
+#pragma unroll 4
+        for (int q = 0; q < parts; q++) t += p[(int64_t)q * kLsqF];
+        s_t[w][lane] = t;
+    }
+    __syncwarp();
+    double u[9];
+    for (int e = 0; e < 9; e++) u[e] = ubis[9 * i + e];
     const int ns = *nspecial;
     if (ns) {
-        double u[9];
-        for (int e = 0; e < 9; e++) u[e] = ubis[9 * i + e];
+        double* acc = s_lsq[w] + lane;
+        for (int f = 0; f < kLsqF; f++) acc[f * 32] = 0.;
         for (int q = lane; q < ns; q += 32) {
             const int64_t k = special[q];
             double ih[3];
@@ -772,40 +786,25 @@ k_refine_special(const double* __restrict__ ubis, int64_t m, double tol,
             const double sv = drlv2_exact(u, g[0], g[1], g[2], ih);
             if (sv < tol * tol) lsq_add(acc, sv, g, ih);
         }
+        __syncwarp();
+        for (int f = 0; f < kLsqF; f++) {
+            const double v = warp_sum(acc[f * 32]);
+            if (lane == 0) s_t[w][f] += v;
+        }
+        __syncwarp();
     }
-    __syncwarp();
-    for (int f = 0; f < kLsqF; f++) {
-        const double v = warp_sum(acc[f * 32]);
-        if (lane == 0) spart[i * kLsqF + f] = v;
-    }
-}
-
-// One thread per UBI: partials in part order, then the slot of the g outside
-// the regular range, then the reference's update; n and mean drlv2 of the UBI
-// as it was on entry.
-__global__ void __launch_bounds__(kGT)
-k_refine_finish(double* __restrict__ ubis, int64_t m, int parts,
-                const double* __restrict__ part_in, const double* __restrict__ spart,
-                int* __restrict__ npk, double* __restrict__ mean) {
-    const int64_t i = (int64_t)blockIdx.x * kGT + threadIdx.x;
-    if (i >= m) return;
-    double t[kLsqF];
-    for (int f = 0; f < kLsqF; f++) t[f] = 0.;
-    for (int p = 0; p < parts; p++)
-        for (int f = 0; f < kLsqF; f++) t[f] += part_in[(i * parts + p) * kLsqF + f];
-    for (int f = 0; f < kLsqF; f++) t[f] += spart[i * kLsqF + f];
-    double u[9];
-    for (int e = 0; e < 9; e++) u[e] = ubis[9 * i + e];
+    if (lane != 0) return;
+    const double* z = s_t[w];
     double R[9], Hm[9];
-    for (int f = 0; f < 9; f++) R[f] = t[f];
-    Hm[0] = t[9];  Hm[1] = t[10]; Hm[2] = t[11];
-    Hm[3] = t[10]; Hm[4] = t[12]; Hm[5] = t[13];
-    Hm[6] = t[11]; Hm[7] = t[13]; Hm[8] = t[14];
+    for (int f = 0; f < 9; f++) R[f] = z[f];
+    Hm[0] = z[9];  Hm[1] = z[10]; Hm[2] = z[11];
+    Hm[3] = z[10]; Hm[4] = z[12]; Hm[5] = z[13];
+    Hm[6] = z[11]; Hm[7] = z[13]; Hm[8] = z[14];
     lsq_update_exact(R, Hm, u);
     for (int e = 0; e < 9; e++) ubis[9 * i + e] = u[e];
-    const long long n = (long long)t[16];
+    const long long n = (long long)z[16];
     if (npk) npk[i] = (int)n;
-    if (mean) mean[i] = n > 0 ? t[15] / (double)n : 0.;
+    if (mean) mean[i] = n > 0 ? z[15] / (double)n : 0.;
 }
 
 // ------------------------------------------------------------ assignment --
@@ -1348,12 +1347,11 @@ extern "C" int id11b_dev_score_and_assign_grid(const double* ubis, int64_t m,
     return ID11B_OK;
 }
 
-// partials: m * parts + m slots of 17 doubles (the last m: the g outside the
-// regular range)
+// partials: 17 doubles per work item
 extern "C" int64_t id11b_grid_refine_workspace_bytes(int64_t m) {
     if (m < 0) return -1;
     const size_t mm = (size_t)(m > 0 ? m : 1);
-    return (int64_t)al256(sizeof(double) * kLsqF * (mm * score_parts(m) + mm));
+    return (int64_t)al256(sizeof(double) * kLsqF * mm * score_parts(m));
 }
 
 extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, int64_t n,
@@ -1381,12 +1379,9 @@ extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, 
                                          (const double*)(b + L.g), (const float4*)(b + L.g4), tol,
                                          part);
         ID11B_CHECK_LAUNCH();
-        double* spart = part + m * parts * kLsqF;
-        k_refine_special<<<(unsigned)((m * 32 + kGT - 1) / kGT), kGT, 0, st>>>(
-            ubis, m, tol, gv, (const int*)(b + L.spec), (const int*)(b + L.spos) + n, spart);
-        ID11B_CHECK_LAUNCH();
-        k_refine_finish<<<(unsigned)((m + kGT - 1) / kGT), kGT, 0, st>>>(ubis, m, sp.parts(), part,
-                                                                         spart, npk, mean);
+        k_refine_finish<<<(unsigned)((m * 32 + kGT - 1) / kGT), kGT, 0, st>>>(
+            ubis, m, sp.parts(), part, tol, gv, (const int*)(b + L.spec),
+            (const int*)(b + L.spos) + n, npk, mean);
         ID11B_CHECK_LAUNCH();
     }
     return ID11B_OK;
