@@ -192,6 +192,37 @@ __device__ __forceinline__ int slot_of(int lane) {
     return have > 0 ? at : -1;
 }
 
+// Elements of a symmetric 3x3 matrix from its upper triangle (00 01 02 11 12 22).
+__device__ __forceinline__ int h_slot(int e) {
+    const int i = e / 3, j = e - 3 * i, lo = min(i, j);
+    return i + j + (lo > 0);
+}
+
+// lsq_update_exact by one warp: lane f of t holds field f of the sums (R 9, H's
+// upper triangle 6); u is the lane's UBI element (lanes 0 .. 8).  Returns the new
+// one (u unless both inverses exist).  Each lane takes one cofactor and one UB
+// element with the same expressions, so the result has the same bits.  m: 27
+// doubles of scratch in shared memory.
+__device__ __forceinline__ double lsq_update_warp(double t, double u, double* m, int lane) {
+    const int e = lane < 9 ? lane : 0, i = e / 3, j = e - 3 * i;
+    const double h = __shfl_sync(0xffffffffu, t, 9 + h_slot(e));
+    if (lane < 9) {
+        m[lane] = t;       // R
+        m[9 + lane] = h;   // H
+    }
+    __syncwarp();
+    const double det = det3_exact(m + 9);
+    const double hi = det != 0. ? inv3_elem(m + 9, det, e) : 0.;
+    double s = 0.;
+#pragma unroll
+    for (int l = 0; l < 3; l++)
+        s = dadd(s, dmul(m[3 * i + l], __shfl_sync(0xffffffffu, hi, 3 * l + j)));
+    if (lane < 9) m[18 + lane] = s;  // UB
+    __syncwarp();
+    const double det2 = det3_exact(m + 18);
+    return det != 0. && det2 != 0. ? inv3_elem(m + 18, det2, e) : u;
+}
+
 }  // namespace id11b
 
 // Status from a launch: 0, or ID11B_ERR_CUDA with the CUDA code recorded.

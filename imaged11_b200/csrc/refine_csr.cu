@@ -27,14 +27,8 @@
 namespace id11b {
 
 struct RefineSmem {
-    double R[9], H[9], UB[9], ubi[9];
+    double m[27], ubi[9];
 };
-
-// H upper-triangle slot (00 01 02 11 12 22) of element e of H
-__device__ __forceinline__ int h_slot(int e) {
-    const int i = e / 3, j = e - 3 * i, lo = min(i, j);
-    return i + j + (lo > 0);
-}
 
 // Compensated FP32 accumulation (the F32C variant): a sum kept as s + c with
 // every addition's rounding error recovered exactly (TwoSum) and every
@@ -234,25 +228,10 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
             if (lane < 17)
                 for (int q = 0; q < N / 32; q++) t += red[q][lane];
             // t: R in lanes 0 .. 8, H's upper triangle 9 .. 14, sum, n
-            if (lane < 9) sm.R[lane] = t;
-            const int e = lane < 9 ? lane : 0;
-            const double h = __shfl_sync(0xffffffffu, t, 9 + h_slot(e));
-            if (lane < 9) sm.H[lane] = h;
             const double ss = __shfl_sync(0xffffffffu, t, 15);
             const long long np = (long long)__shfl_sync(0xffffffffu, t, 16);
-            __syncwarp();
-            // UB = R . inv(H); UBI = inv(UB); keep ubi unless both inverses exist
-            const double det = det3_exact(sm.H);
-            const double hi = det != 0. ? inv3_elem(sm.H, det, e) : 0.;
-            const int i = e / 3, j = e - 3 * i;
-            double s = 0.;
-#pragma unroll
-            for (int l = 0; l < 3; l++)
-                s = dadd(s, dmul(sm.R[3 * i + l], __shfl_sync(0xffffffffu, hi, 3 * l + j)));
-            if (lane < 9) sm.UB[lane] = s;
-            __syncwarp();
-            const double det2 = det3_exact(sm.UB);
-            if (lane < 9 && det != 0. && det2 != 0.) sm.ubi[lane] = inv3_elem(sm.UB, det2, e);
+            const double v = lsq_update_warp(t, lane < 9 ? sm.ubi[lane] : 0., sm.m, lane);
+            if (lane < 9) sm.ubi[lane] = v;
             if (lane == 0 && it == iters - 1) {
                 if (npk) npk[g] = (int)np;
                 if (mean) mean[g] = np > 0 ? ddiv(ss, (double)np) : 0.;

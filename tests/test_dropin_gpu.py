@@ -248,3 +248,37 @@ def test_host_calls_small_large_and_threads(cim, oracle, cuda):
             n2, m2, u2 = oracle.score_and_refine(ubis[(k + rep) % len(ubis)], ps.gv, 0.05)
             assert n == n2 and abs(m - m2) <= 1e-12 * abs(m2)
             assert np.abs(u - u2).max() <= 1e-12 * np.abs(u2).max()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 511, 513, 1535, 2047, 2049, 8191, 8192,
+                               8193, 16383, 16384, 16385])
+def test_least_squares_sizes(oracle, n, cuda):
+    """Sizes around the CTAs, shares and tiles of the one-cluster launch and past
+    it, from host arrays, device arrays and a device array that is not 16-byte
+    aligned: counts exact, UBI and mean drlv2 to the rounding of sums in another
+    order (1e-12)."""
+    import torch
+    from imaged11_b200 import cImageD11 as cim
+    rng = np.random.default_rng(n)
+    ubi = 4.05 * np.linalg.qr(rng.normal(size=(3, 3)))[0]
+    gv = rng.integers(-5, 6, size=(n, 3)) @ np.linalg.inv(ubi).T + rng.normal(size=(n, 3)) * 4e-3
+    labels = rng.integers(0, 3, n).astype(np.int32)
+    labels[-1] = 1
+    kept = gv[labels == 1]
+    want = (oracle.score_and_refine(ubi, gv, 0.05), oracle.score_and_refine(ubi, kept, 1.0))
+    dev = torch.tensor(np.concatenate([gv[:1], gv]), device=cuda)
+    forms = ((gv, labels), (dev[1:].clone(), torch.tensor(labels, device=cuda)),
+             (dev[1:], torch.tensor(labels, device=cuda)))
+    assert forms[2][0].data_ptr() % 16 == 8
+    for g, lab in forms:
+        for mode, (rn, rmean, ru) in enumerate(want):
+            host = isinstance(g, np.ndarray)
+            u = ubi.copy() if host else torch.tensor(ubi, device=cuda)
+            k, mean = cim.score_and_refine(u, g, 0.05) if mode == 0 else \
+                cim.refine_assigned(u, g, lab, 1)
+            u = u if host else u.cpu().numpy()
+            assert k == rn
+            if k > 3:       # (up to three peaks the normal matrix is singular to rounding)
+                assert abs(mean - rmean) <= 1e-12 * rmean
+                assert np.abs(u - np.asarray(ru)).max() <= 1e-12 * np.abs(ru).max() * \
+                    max(1.0, 1e3 / k)
