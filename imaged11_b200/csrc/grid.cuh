@@ -40,15 +40,19 @@ struct Tols {
 __host__ __device__ inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Grid buffer: header | cnt[ncells+1] | start[ncells+1] | g[n][3] | gidx[n] |
-// flag[n+1] | spos[n+1] | spec[n] | scan totals
+// flag[n+1] (then the g of each cell, unordered) | spos[n+1] | spec[n] | totals of
+// both scans | g4[n] (at first each g's place in its cell)
 struct Layout {
     size_t header, cnt, start, g, idx, flag, spos, spec, tot, g4, bytes;
 };
 
+__host__ __device__ inline int64_t scan_blocks(int64_t len) {
+    return (len + kScanPer - 1) / kScanPer;
+}
+
 __host__ __device__ inline Layout layout(int64_t n, int64_t ncells) {
     Layout L;
     const size_t nn = (size_t)(n > 0 ? n : 1);
-    const int64_t big = ncells + 1 > n + 1 ? ncells + 1 : n + 1;
     size_t o = 0;
     L.header = o; o = al256(o + sizeof(Header));
     L.cnt = o;    o = al256(o + sizeof(int) * (size_t)(ncells + 1));
@@ -58,7 +62,7 @@ __host__ __device__ inline Layout layout(int64_t n, int64_t ncells) {
     L.flag = o;   o = al256(o + sizeof(int) * (nn + 1));
     L.spos = o;   o = al256(o + sizeof(int) * (nn + 1));
     L.spec = o;   o = al256(o + sizeof(int) * nn);
-    L.tot = o;    o = al256(o + sizeof(int) * (size_t)((big + kScanPer - 1) / kScanPer + 1));
+    L.tot = o;    o = al256(o + sizeof(int) * (size_t)(scan_blocks(ncells + 1) + scan_blocks(n + 1)));
     L.g4 = o;     o = al256(o + sizeof(float) * 4 * nn);  // FP32 copy of the sorted g
     L.bytes = o;
     return L;

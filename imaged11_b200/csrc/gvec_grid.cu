@@ -67,164 +67,181 @@ k_bounds(const double* __restrict__ gv, int64_t n, unsigned int* __restrict__ ou
     }
 }
 
+// Each g's cell counted, and its place among the cell's g in the order the
+// atomics ran; flag: 1 for a g that no cell holds.  Writes the header.
 __global__ void __launch_bounds__(kGT)
-k_count(const double* __restrict__ gv, int64_t n, const Header* __restrict__ Hp,
-        int* __restrict__ cnt, int* __restrict__ flag) {
-    const Header H = *Hp;
+k_count(const double* __restrict__ gv, int64_t n, const Header H, Header* __restrict__ Hp,
+        int* __restrict__ cnt, int* __restrict__ flag, int* __restrict__ place) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *Hp = H;
+        flag[n] = 0;
+    }
     for (int64_t k = (int64_t)blockIdx.x * kGT + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * kGT) {
         double a = gv[3 * k], b = gv[3 * k + 1], c = gv[3 * k + 2];
         const bool reg = indexed(a, b, c, H);
         flag[k] = reg ? 0 : 1;
-        if (reg) atomicAdd(cnt + cell_of(a, b, c, H), 1);
+        if (reg) place[k] = atomicAdd(cnt + cell_of(a, b, c, H), 1);
     }
 }
 
-// exclusive scan of x[0..len) into y, CTA totals into tot (pass 1)
-__global__ void __launch_bounds__(kScanT)
-k_scan_local(const int* __restrict__ x, int64_t len, int* __restrict__ y, int* __restrict__ tot) {
+// Exclusive scans of one or two arrays x[0 .. len) into y (16-byte aligned), the
+// CTAs' totals in tot: blocks 0 .. nb - 1 of the first, then the second's.
+struct ScanJob {
+    const int* x;
+    int64_t len;
+    int* y;
+    int* tot;
+    int nb;
+};
+
+__device__ __forceinline__ void scan_load(const int* __restrict__ x, int64_t base, int64_t len,
+                                          int v[4]) {
+    if (base + 3 < len) {
+        const int4 q = *reinterpret_cast<const int4*>(x + base);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = base + q < len ? x[base + q] : 0;
+    }
+}
+
+__device__ __forceinline__ void scan_store(int* __restrict__ y, int64_t base, int64_t len,
+                                           const int v[4]) {
+    if (base + 3 < len) {
+        *reinterpret_cast<int4*>(y + base) = make_int4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (base + q < len) y[base + q] = v[q];
+    }
+}
+
+// pass 1: each CTA's kScanPer entries, from zero
+__global__ void __launch_bounds__(kScanT) k_scan_local(ScanJob first, ScanJob second) {
     __shared__ int s_w[kScanT / 32];
-    const int64_t base = (int64_t)blockIdx.x * kScanPer + 4 * threadIdx.x;
-    int v[4], sum = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        v[q] = base + q < len ? x[base + q] : 0;
-        sum += v[q];
-    }
+    const bool two = (int)blockIdx.x >= first.nb;
+    const ScanJob J = two ? second : first;
+    const int blk = (int)blockIdx.x - (two ? first.nb : 0);
+    const int64_t base = (int64_t)blk * kScanPer + 4 * threadIdx.x;
+    int v[4];
+    scan_load(J.x, base, J.len, v);
+    const int sum = v[0] + v[1] + v[2] + v[3];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_w[wid] = incl;
+    int total;
+    const int excl = warp_excl_scan(sum, lane, total);
+    if (lane == 31) s_w[wid] = total;
     __syncthreads();
     if (wid == 0) {
-        int w = s_w[lane];
-        int wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += t;
-        }
-        s_w[lane] = wi - w;  // exclusive over warps
-        if (lane == 31) tot[blockIdx.x] = wi;
+        int all;
+        const int we = warp_excl_scan(s_w[lane], lane, all);
+        s_w[lane] = we;  // exclusive over warps
+        if (lane == 31) J.tot[blk] = all;
     }
     __syncthreads();
-    int run = s_w[wid] + incl - sum;
+    int run = s_w[wid] + excl, out[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        if (base + q < len) y[base + q] = run;
+        out[q] = run;
         run += v[q];
     }
+    scan_store(J.y, base, J.len, out);
 }
 
-// exclusive scan of the CTA totals in place (one CTA, sequential chunks)
-__global__ void __launch_bounds__(kScanT) k_scan_totals(int* __restrict__ tot, int nb) {
+// pass 2: the totals in place (one CTA per array, sequential chunks)
+__global__ void __launch_bounds__(kScanT) k_scan_totals(ScanJob first, ScanJob second) {
     __shared__ int s_w[kScanT / 32];
     __shared__ int s_carry;
+    const ScanJob J = blockIdx.x ? second : first;
+    int* __restrict__ tot = J.tot;
     if (threadIdx.x == 0) s_carry = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int b0 = 0; b0 < nb; b0 += kScanT) {
+    for (int b0 = 0; b0 < J.nb; b0 += kScanT) {
         const int i = b0 + threadIdx.x;
-        const int v = i < nb ? tot[i] : 0;
-        int incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) s_w[wid] = incl;
+        const int v = i < J.nb ? tot[i] : 0;
+        int total;
+        const int excl = warp_excl_scan(v, lane, total);
+        if (lane == 31) s_w[wid] = total;
         __syncthreads();
         if (wid == 0) {
-            int w = s_w[lane], wi = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += t;
-            }
-            s_w[lane] = wi - w;
+            int all;
+            const int we = warp_excl_scan(s_w[lane], lane, all);
+            s_w[lane] = we;
         }
         __syncthreads();
         const int carry = s_carry;
-        if (i < nb) tot[i] = carry + s_w[wid] + incl - v;
+        if (i < J.nb) tot[i] = carry + s_w[wid] + excl;
         __syncthreads();
-        if (threadIdx.x == kScanT - 1) s_carry = carry + s_w[wid] + incl;
+        if (threadIdx.x == kScanT - 1) s_carry = carry + s_w[wid] + excl + v;
         __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(kScanT)
-k_scan_add(int* __restrict__ y, int64_t len, const int* __restrict__ tot) {
-    const int64_t base = (int64_t)blockIdx.x * kScanPer + 4 * threadIdx.x;
-    const int add = tot[blockIdx.x];
+// pass 3
+__global__ void __launch_bounds__(kScanT) k_scan_add(ScanJob first, ScanJob second) {
+    const bool two = (int)blockIdx.x >= first.nb;
+    const ScanJob J = two ? second : first;
+    const int blk = (int)blockIdx.x - (two ? first.nb : 0);
+    const int64_t base = (int64_t)blk * kScanPer + 4 * threadIdx.x;
+    const int add = J.tot[blk];
+    int v[4];
+    scan_load(J.y, base, J.len, v);
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-        if (base + q < len) y[base + q] += add;
+    for (int q = 0; q < 4; q++) v[q] += add;
+    scan_store(J.y, base, J.len, v);
 }
 
+// The g of each cell listed where the cell begins, in the order of their places;
+// the g that no cell holds in their own list, by index.
 __global__ void __launch_bounds__(kGT)
-k_scatter(const double* __restrict__ gv, int64_t n, const Header* __restrict__ Hp,
-          const int* __restrict__ start, int* __restrict__ cursor, double* __restrict__ gs,
-          int* __restrict__ gidx, const int* __restrict__ spos, int* __restrict__ spec) {
+k_list_cells(const double* __restrict__ gv, int64_t n, const Header* __restrict__ Hp,
+             const int* __restrict__ start, const int* __restrict__ place,
+             int* __restrict__ list, const int* __restrict__ spos, int* __restrict__ spec) {
     const Header H = *Hp;
     for (int64_t k = (int64_t)blockIdx.x * kGT + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * kGT) {
         double a = gv[3 * k], b = gv[3 * k + 1], c = gv[3 * k + 2];
-        if (!indexed(a, b, c, H)) {
+        if (!indexed(a, b, c, H))
             spec[spos[k]] = (int)k;
-            continue;
-        }
-        const int64_t cid = cell_of(a, b, c, H);
-        const int p = start[cid] + atomicAdd(cursor + cid, 1);
-        gs[3 * (int64_t)p] = a;
-        gs[3 * (int64_t)p + 1] = b;
-        gs[3 * (int64_t)p + 2] = c;
-        gidx[p] = (int)k;
+        else
+            list[start[cell_of(a, b, c, H)] + place[k]] = (int)k;
     }
 }
 
-// Each cell's entries ordered by original index (the layout, and so every
-// result, does not depend on the order the scatter's atomics ran in) and the
-// FP32 (round to nearest) copy of the sorted g for staging, with the g's x cell
-// (as int bits) in w.  One thread per position; the thread at a cell's first
-// position sorts the cell and writes its copies.  Threads at the cell's other
-// positions may read coordinates the sort is moving, but every value there is
-// a coordinate of a g of that cell, so they find the same cell and skip it.
+// Each listed g to its sorted position: within a cell by index (the layout, and so
+// every result, does not depend on the order the atomics ran in) -- its rank among
+// the cell's list, mostly of one to three -- with its FP64 coordinates, its index,
+// and the FP32 (round to nearest) copy for screening and staging, the x cell (as
+// int bits) in w.  One thread per place of the list: neighbours are in the same or
+// the next cells, so everything but the read of the g itself is coalesced.
+//
+// Bound: the random 24-byte reads, and the counts' passes over the cells.  The
+// build of 61k g (512k cells), 1.1M (8.1M) and 10.2M (10.2M): 32, 101 and 687 us;
+// scattering every g by atomics and sorting each cell by one thread took 68, 232 and
+// 4,173 us, and 20.6 ms where cells hold a hundred g and more (now 0.08).
 __global__ void __launch_bounds__(kGT)
-k_sort_cells_f32(const int* __restrict__ start, const Header* __restrict__ Hp, double* gs,
-                 int* gidx, float4* __restrict__ g4) {
+k_place(const double* __restrict__ gv, const Header* __restrict__ Hp,
+        const int* __restrict__ start, const int* __restrict__ list, double* __restrict__ gs,
+        int* __restrict__ gidx, float4* __restrict__ g4) {
     const Header H = *Hp;
     const int64_t nreg = start[H.ncells];
-    for (int64_t p = (int64_t)blockIdx.x * kGT + threadIdx.x; p < nreg;
-         p += (int64_t)gridDim.x * kGT) {
-        const int64_t c = cell_of(gs[3 * p], gs[3 * p + 1], gs[3 * p + 2], H);
-        const int a = start[c];
-        if (a != p) continue;
-        const int b = start[c + 1];
-        for (int i = a + 1; i < b; i++) {
-            const int key = gidx[i];
-            const double x = gs[3 * (int64_t)i], y = gs[3 * (int64_t)i + 1],
-                         z = gs[3 * (int64_t)i + 2];
-            int j = i - 1;
-            while (j >= a && gidx[j] > key) {
-                gidx[j + 1] = gidx[j];
-                gs[3 * (int64_t)j + 3] = gs[3 * (int64_t)j];
-                gs[3 * (int64_t)j + 4] = gs[3 * (int64_t)j + 1];
-                gs[3 * (int64_t)j + 5] = gs[3 * (int64_t)j + 2];
-                j--;
-            }
-            gidx[j + 1] = key;
-            gs[3 * (int64_t)j + 3] = x;
-            gs[3 * (int64_t)j + 4] = y;
-            gs[3 * (int64_t)j + 5] = z;
-        }
-        for (int64_t q = a; q < b; q++)
-            g4[q] = make_float4(__double2float_rn(gs[3 * q]), __double2float_rn(gs[3 * q + 1]),
-                                __double2float_rn(gs[3 * q + 2]),
-                                __int_as_float(coord_x(gs[3 * q], H)));
+    for (int64_t at = (int64_t)blockIdx.x * kGT + threadIdx.x; at < nreg;
+         at += (int64_t)gridDim.x * kGT) {
+        const int k = list[at];
+        const double a = gv[3 * (int64_t)k], b = gv[3 * (int64_t)k + 1],
+                     c = gv[3 * (int64_t)k + 2];
+        const int64_t cid = cell_of(a, b, c, H);
+        const int p0 = start[cid], p1 = start[cid + 1];
+        int p = p0;
+        if (p1 - p0 > 1)
+            for (int q = p0; q < p1; q++) p += list[q] < k;
+        gs[3 * (int64_t)p] = a;
+        gs[3 * (int64_t)p + 1] = b;
+        gs[3 * (int64_t)p + 2] = c;
+        gidx[p] = k;
+        g4[p] = make_float4(__double2float_rn(a), __double2float_rn(b), __double2float_rn(c),
+                            __int_as_float(coord_x(a, H)));
     }
 }
 
@@ -1069,16 +1086,21 @@ unsigned grid_for(int64_t items, int per) {
     return (unsigned)(b > 0 ? b : 1);
 }
 
-// exclusive scan of x[0..len) into y (len >= 1), tot: scratch
-int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st) {
-    const int64_t nb = (len + kScanPer - 1) / kScanPer;
-    k_scan_local<<<(unsigned)nb, kScanT, 0, st>>>(x, len, y, tot);
+static int scan_jobs(const ScanJob& a, const ScanJob& b, cudaStream_t st) {
+    const unsigned nb = (unsigned)(a.nb + b.nb);
+    k_scan_local<<<nb, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
-    k_scan_totals<<<1, kScanT, 0, st>>>(tot, (int)nb);
+    k_scan_totals<<<b.nb ? 2 : 1, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
-    k_scan_add<<<(unsigned)nb, kScanT, 0, st>>>(y, len, tot);
+    k_scan_add<<<nb, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
+}
+
+// exclusive scan of x[0..len) into y (len >= 1; both 16-byte aligned), tot: scratch
+int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st) {
+    return scan_jobs(ScanJob{x, len, y, tot, (int)scan_blocks(len)},
+                     ScanJob{nullptr, 0, nullptr, nullptr, 0}, st);
 }
 
 // work items (warps) per UBI: about two waves of the resident warps, and two
@@ -1185,35 +1207,27 @@ extern "C" int id11b_dev_build_grid(const double* gv, int64_t n, float gmax, flo
     h.nx = nx;
     h.nxx = nx * xsub;
     static_assert(sizeof(Header) <= 256, "header");
-    // a copy from pageable memory returns once the source has been staged,
-    // so the stack value may go out of scope
-    ID11B_CHECK(cudaMemcpyAsync(b + L.header, &h, sizeof(h), cudaMemcpyHostToDevice, st));
     int* cnt = (int*)(b + L.cnt);
     int* start = (int*)(b + L.start);
     int* flag = (int*)(b + L.flag);
     int* spos = (int*)(b + L.spos);
     int* tot = (int*)(b + L.tot);
+    int* place = (int*)(b + L.g4);  // until k_place writes g4
+    Header* H = (Header*)(b + L.header);
     ID11B_CHECK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)(ncells + 1), st));
-    ID11B_CHECK(cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)(n + 1), st));
-    const Header* H = (const Header*)(b + L.header);
-    if (n > 0) {
-        k_count<<<grid_for(n, kGT), kGT, 0, st>>>(gv, n, H, cnt, flag);
-        ID11B_CHECK_LAUNCH();
-    }
-    int rc = scan(cnt, ncells + 1, start, tot, st);
-    if (rc) return rc;
-    rc = scan(flag, n + 1, spos, tot, st);
-    if (rc) return rc;
-    ID11B_CHECK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)(ncells + 1), st));  // cursors
-    if (n > 0) {
-        k_scatter<<<grid_for(n, kGT), kGT, 0, st>>>(gv, n, H, start, cnt, (double*)(b + L.g),
-                                                    (int*)(b + L.idx), spos, (int*)(b + L.spec));
-        ID11B_CHECK_LAUNCH();
-        k_sort_cells_f32<<<grid_for(n, kGT), kGT, 0, st>>>(start, H, (double*)(b + L.g),
-                                                            (int*)(b + L.idx),
-                                                            (float4*)(b + L.g4));
-        ID11B_CHECK_LAUNCH();
-    }
+    k_count<<<grid_for(n, kGT), kGT, 0, st>>>(gv, n, h, H, cnt, flag, place);
+    ID11B_CHECK_LAUNCH();
+    const int cb = (int)scan_blocks(ncells + 1);
+    const int rc = scan_jobs(ScanJob{cnt, ncells + 1, start, tot, cb},
+                             ScanJob{flag, n + 1, spos, tot + cb, (int)scan_blocks(n + 1)}, st);
+    if (rc || n == 0) return rc;
+    int* list = flag;  // the flags are done with
+    k_list_cells<<<grid_for(n, kGT), kGT, 0, st>>>(gv, n, H, start, place, list, spos,
+                                                   (int*)(b + L.spec));
+    ID11B_CHECK_LAUNCH();
+    k_place<<<grid_for(n, kGT), kGT, 0, st>>>(gv, H, start, list, (double*)(b + L.g),
+                                              (int*)(b + L.idx), (float4*)(b + L.g4));
+    ID11B_CHECK_LAUNCH();
     return ID11B_OK;
 }
 

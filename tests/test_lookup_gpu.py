@@ -89,3 +89,26 @@ def test_binned_sums_of_dense_boxes(oracle, copies, ntol, cuda):
         for j, t in enumerate(tols):
             n, mean, _ = oracle.score_and_refine(u[i], g, t)
             assert abs(s[i, j] - n * mean) <= 1e-12 * n * mean + n * step
+
+
+@pytest.mark.parametrize("n", [0, 1, 4095, 4096, 4097, 30000])
+@pytest.mark.parametrize("cell", [None, 0.6])
+def test_build_is_repeatable(scene, n, cell, cuda):
+    """The index's layout depends on the g alone, whatever order the build's
+    atomics ran in: two builds and a rebuild refine to the same bits (g repeated,
+    outside the regular range, and cells of one and of hundreds of g)."""
+    import torch
+    from imaged11_b200 import batch
+    gv, u = scene
+    g = gv[:n].copy()
+    g[5:n:7] = g[4:n - 1:7][:len(g[5:n:7])]
+    g[3:n:101] = np.nan
+    grids = [batch.GvecGrid(g, cell=cell), batch.GvecGrid(g, cell=cell)]
+    out = [batch.refine_grid(u.copy(), x, 0.1) for x in grids]
+    grids[0].refresh()
+    out.append(batch.refine_grid(u.copy(), grids[0], 0.1))
+    st = grids[0].stats()
+    assert st["special"] == int(np.isnan(g[:, 0]).sum())
+    assert st["regular"] + st["special"] == len(g)
+    for o in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(o, out[0]))
