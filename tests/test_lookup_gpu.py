@@ -112,3 +112,27 @@ def test_build_is_repeatable(scene, n, cell, cuda):
     assert st["regular"] + st["special"] == len(g)
     for o in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(o, out[0]))
+
+
+@pytest.mark.parametrize("grains", [1, 6, 12, 60])
+@pytest.mark.parametrize("m", [1, 37, 3000])
+def test_binned_join_of_crowded_trials(scene, oracle, grains, m, cuda):
+    """Trials that crowd around a few orientations: streams that are counted
+    first, that overflow the room they are given, and that fit; one to several
+    work items a UBI; a UBI the join does not take among them."""
+    from imaged11_b200 import batch, synth
+    gv, _ = scene
+    rng = np.random.default_rng(95)
+    base = np.linalg.inv(synth.random_rotations(grains, rng) / 4.05)
+    u = synth.perturb_ubis(base[np.arange(m) % grains], 0.3, 0.001, rng)
+    if m > 20:
+        u[11] = 0.0
+    grid = batch.GvecGrid(gv)
+    tols = [0.05, 0.15]
+    c, s = batch.score_grid(u, grid, tols, sums=True, method="bins")
+    ref = oracle.score_many(u, gv, tols)
+    assert np.array_equal(c.cpu().numpy(), ref)
+    assert np.array_equal(batch.score_grid(u, grid, tols, method="bins").cpu().numpy(), ref)
+    w = batch.score_grid(u, grid, tols, sums=True, method="walk")[1]
+    step = 2.0 ** -(62 - np.ceil(np.log2(len(gv) * max(tols) ** 2)))
+    assert np.all((s - w).abs().cpu().numpy() <= 1e-12 * w.cpu().numpy() + ref * step)
