@@ -149,7 +149,7 @@ class GvecGrid:
         self.gv = g.contiguous()
         self.n = self.gv.shape[0]
         dev = self.gv.device
-        bounds = torch.zeros(2, dtype=torch.int32, device=dev)
+        bounds = torch.empty(2, dtype=torch.int32, device=dev)
         check(lib.id11b_dev_gvec_bounds(self.gv.data_ptr(), self.n, bounds.data_ptr(),
                                         _stream()), "gvec_bounds")
         b = bounds.cpu().numpy().view(np.float32)
@@ -212,20 +212,15 @@ def bins_box_estimate(ubis, grid, tmax):
     boxes the binned join enumerates for these UBIs: the lattice points of
     each UBI within rmax + |w| of the origin.  Reads one number back."""
     torch = _torch()
-    u = _dev(ubis, torch.float64).reshape(-1, 3, 3)
+    u = _dev(ubis, torch.float64).reshape(-1, 9)
     if u.shape[0] == 0:
         return 0
-    det = torch.nan_to_num(torch.linalg.det(u).abs(), nan=0.0, posinf=0.0)
-    ok = det > 0
-    ub = torch.linalg.inv(torch.where(ok[:, None, None], u, torch.eye(3, dtype=u.dtype,
-                                                                    device=u.device)))
-    w = (tmax + 1e-6) * ub.norm(dim=2).norm(dim=1)
-    r = grid.rmax + torch.nan_to_num(w, nan=0.0, posinf=0.0)
-    est = (4.0 / 3.0 * np.pi) * (r ** 3) * det * ok
+    est = torch.empty(1, dtype=torch.float64, device=u.device)
     # a UBI with more candidate hkl than g-vectors, or a large row sum, is
     # scanned plainly and enumerates no boxes
-    est = torch.where(est <= grid.n, est, torch.zeros_like(est))
-    total = 1.25 * float(est.sum().item()) + 64 * u.shape[0]
+    check(lib.id11b_dev_bins_box_estimate(u.data_ptr(), u.shape[0], grid.rmax, float(tmax), grid.n,
+                                          est.data_ptr(), _stream()), "bins_box_estimate")
+    total = 1.25 * float(est.item()) + 64 * u.shape[0]
     return int(min(total, BINS_MAX_BOXES))
 
 

@@ -295,6 +295,11 @@ int id11b_grid_stats(const void *gridbuf, int64_t *nregular, int64_t *nspecial,
  * 2^-(62 - ceil(log2(n tmax^2))), 2^-49 for 1.1M g at tol 0.1) so that they
  * repeat bit for bit; counts are exact. */
 int64_t id11b_grid_bins_workspace_bytes(int64_t m, int32_t nx, int32_t xsub, int64_t boxes);
+/* The sum over m UBIs of the lattice points expected within rmax + w of the
+ * origin (w for tolerance tmax), to *sum (device): what a box capacity is sized
+ * from.  UBIs that are singular, non-finite or have more points than n count 0. */
+int id11b_dev_bins_box_estimate(const double *ubis, int64_t m, double rmax, double tmax, int64_t n,
+                                double *sum, void *stream);
 /* Measurement hook: the calling thread's next id11b_dev_score_grid_bins call
  * records start_event before its first join launch and stop_event after its
  * last (both cudaEvent_t, created by the caller; NULL, NULL clears). */

@@ -136,3 +136,30 @@ def test_binned_join_of_crowded_trials(scene, oracle, grains, m, cuda):
     w = batch.score_grid(u, grid, tols, sums=True, method="walk")[1]
     step = 2.0 ** -(62 - np.ceil(np.log2(len(gv) * max(tols) ** 2)))
     assert np.all((s - w).abs().cpu().numpy() <= 1e-12 * w.cpu().numpy() + ref * step)
+
+
+@pytest.mark.parametrize("m", [1, 33, 1025])
+def test_box_estimate(m, cuda):
+    """The expected number of boxes against numpy, with UBIs that count none:
+    singular, NaN, infinite, and more points than g.  Near singular UBIs lose digits in
+    numpy's inverse: 1e-9."""
+    import torch
+    from imaged11_b200 import batch
+    rng = np.random.default_rng(m)
+    g = batch.GvecGrid(torch.from_numpy(rng.uniform(-1, 1, (4000, 3))).cuda())
+    u = rng.normal(size=(m, 3, 3)) * 4
+    if m > 8:
+        u[1] = 0
+        u[2, 1, 1] = np.nan
+        u[3, 0, 0] = np.inf
+        u[4] *= 1e3
+    tol = 0.05
+    want = 0.0
+    for k in range(m):
+        det = abs(np.linalg.det(u[k])) if np.isfinite(u[k]).all() else 0.0
+        if det > 0:
+            r = g.rmax + (tol + 1e-6) * np.linalg.norm(np.linalg.inv(u[k]))
+            est = 4 / 3 * np.pi * r ** 3 * det
+            want += est if est <= g.n else 0.0
+    got = batch.bins_box_estimate(torch.from_numpy(u).cuda(), g, tol)
+    assert abs(got - (1.25 * want + 64 * m)) <= 1 + 1e-9 * want
