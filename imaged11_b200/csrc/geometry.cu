@@ -1,7 +1,8 @@
 // Detector geometry kernels: compute_gv, compute_geometry, compute_xlylzl (FP64).
 //
-// Streaming, HBM-bound.  One CTA of 256 threads owns a tile of 256 peaks at a
-// time (grid-stride over tiles, grid = a multiple of the SM count).  The AoS
+// Streaming, bound by HBM (and by the FP64 pipe where angles are asked for).  One
+// CTA of 256 threads owns a tile of 256 peaks at a time (grid-stride over tiles,
+// grid = a multiple of the SM count).  The AoS
 // (n,3) inputs and outputs are staged through shared memory so that every
 // global access is a fully coalesced 8-byte-per-lane sweep of the tile's
 // 6 KB, instead of three 24-byte-strided accesses per lane.
@@ -27,10 +28,147 @@ constexpr double kDeg = 180.0 / 3.14159265358979323846;
 
 // Per-peak body of ImageD11 src/cdiffraction.c:143-167 in the reference's
 // operation order (no FMA).  sin/cos come from CUDA's sincos (<= 2 ulp), the
-// only difference from the reference's libm.
+// only difference from the reference's libm in g.
 struct PeakGeo {
     double so, co, d0, d1, d2, inv, k0, k1, k2, g0, g1, g2;
 };
+
+// The angles are bound by the FP64 pipe (330 operations a peak with the library's
+// arctangents, IEEE root and division: 69% of the pipe busy at 225 us for 10M peaks;
+// the bytes take 147).  The two functions below take 14 operations for an
+// arctangent (about 45) and 9 for 1 / sqrt (about 18).
+//
+// atan2 by table: with mn <= mx the two magnitudes and c = j / 64 nearest mn / mx,
+//   atan(mn / mx) = atan(c) + atan(z),  z = (mn - c mx) / (mx + c mn), |z| < 2^-6.99,
+// where the Taylor series of atan(z) needs four terms (the fifth is below
+// 2^-59 z).  The table holds, per octant of the upper half plane, base +- atan(c)
+// as two doubles, so quadrants cost no arithmetic.  z comes from one Newton step
+// (2^-39) and its exact remainder goes into the sum's low part.  Against 64-bit
+// mantissas over 2M detector positions: two-theta within 2.9 ulp (rms 0.61; the
+// library's atan2 3.5 and 0.69, both with the root before and the degrees after),
+// eta 2.6 (0.48; 2.7 and 0.49).  Magnitudes outside 2^-100 .. 2^100, zeros,
+// infinities and NaN go to the library's.
+constexpr int kAtanN = 64;
+struct AtanTable {
+    double v[4][kAtanN + 1][2];  // [|y| > |x|] + 2 [x < 0]: (value, its rounding error)
+};
+
+// atan(j / 64) times 2^100 by Euler's series, sum over n of
+// 2^2n n!^2 / (2n+1)! x^(2n+1) / (1 + x^2)^(n+1), whose terms follow from one
+// another by ratios of small integers (the ratio is at most 1/2)
+constexpr unsigned __int128 atan_fixed(int j) {
+    unsigned __int128 term = ((unsigned __int128)1 << 100) * (64 * j) / (4096 + j * j), sum = 0;
+    for (int n = 0; term; n++) {
+        sum += term;
+        term = term * (unsigned)((2 * n + 2) * j * j) / (unsigned)((2 * n + 3) * (4096 + j * j));
+    }
+    return sum;
+}
+
+constexpr AtanTable make_atan_table() {
+    AtanTable t{};
+    const unsigned __int128 quarter = 2 * atan_fixed(kAtanN);  // pi / 2
+    for (int j = 0; j <= kAtanN; j++) {
+        const unsigned __int128 c = atan_fixed(j);
+        for (int o = 0; o < 4; o++) {
+            const unsigned __int128 v = o == 0 ? c : o == 1 ? quarter - c :
+                                        o == 2 ? 2 * quarter - c : quarter + c;
+            if (!v) continue;
+            int sh = 0;  // v = (53 bits) 2^sh + rest
+            while (v >> (sh + 53)) sh++;
+            const unsigned __int128 m = (v >> sh) + ((v >> (sh - 1)) & 1);
+            double a = (double)(long long)m,
+                   b = (double)(long long)((unsigned long long)v - (unsigned long long)(m << sh));
+            for (int k = 0; k < 100; k++) {
+                if (k >= sh) a *= 0.5;
+                b *= 0.5;
+            }
+            t.v[o][j][0] = a;
+            t.v[o][j][1] = b;
+        }
+    }
+    return t;
+}
+__device__ constexpr AtanTable kAtan = make_atan_table();
+
+// The CTA's copy in shared memory (the caller's next barrier makes it visible)
+struct AtanShared {
+    double2 v[4][kAtanN + 1];
+    __device__ __forceinline__ void load() {
+        double* b = &v[0][0].x;
+        for (int i = threadIdx.x; i < 8 * (kAtanN + 1); i += blockDim.x)
+            b[i] = (&kAtan.v[0][0][0])[i];
+    }
+};
+
+__device__ __forceinline__ double rcp_approx(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+__device__ __forceinline__ double rsqrt_approx(double x) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+
+// x 2^E for a normal x away from the ends of the range (integer addition)
+template <int E>
+__device__ __forceinline__ double times_pow2(double x) {
+    return __hiloint2double(__double2hiint(x) + E * 0x00100000, __double2loint(x));
+}
+
+// the leading 24 bits of a positive double in 2^-126 .. 2^127 as a float (integer
+// instructions only)
+__device__ __forceinline__ float top_float(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    return __uint_as_float(__funnelshift_l(lo, hi - 0x38000000u, 3));
+}
+
+__device__ __forceinline__ double fast_atan2(double y, double x, const AtanShared& tab) {
+    const int yh = __double2hiint(y), xh = __double2hiint(x);
+    const long long ay = __double_as_longlong(y) & 0x7fffffffffffffffll,
+                    ax = __double_as_longlong(x) & 0x7fffffffffffffffll;
+    const bool swap = ay > ax;
+    const double mx = __longlong_as_double(swap ? ay : ax),
+                 mn = __longlong_as_double(swap ? ax : ay);
+    // both within 2^-100 .. 2^100 (this leaves out zeros, infinities and NaN)
+    if (__double2hiint(mn) < 0x39b00000 || __double2hiint(mx) > 0x46300000) return atan2(y, x);
+    float q;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(top_float(mx)));
+    const float jm = fmaf(top_float(mn) * q, (float)kAtanN, 12582912.f);  // 1.5 2^23 + j
+    const int j = __float_as_int(jm) & 127;
+    const unsigned cf = __float_as_uint((jm - 12582912.f) * (1.f / kAtanN));
+    const double c = __hiloint2double(j ? (int)((cf >> 3) + 0x38000000u) : 0, 0);
+    const int flip = swap == (xh < 0) ? 0 : (int)0x80000000;  // base - atan(c) - atan(z)
+    double num = fma(-c, mx, mn);
+    num = __hiloint2double(__double2hiint(num) ^ flip, __double2loint(num));
+    const double den = fma(c, mn, mx);
+    double r = rcp_approx(den);
+    r = fma(fma(-den, r, 1.), r, r);
+    const double z = num * r, z2 = z * z;  // to 2^-39: the remainder goes into the low part
+    const double2 t = tab.v[(swap ? 1 : 0) + (xh < 0 ? 2 : 0)][j];
+    const double p = fma(z2, fma(z2, -1. / 7., 1. / 5.), -1. / 3.);
+    const double lo = fma(fma(-den, z, num), r, fma(z * z2, p, t.y));
+    const double a = t.x + (z + lo);
+    return __hiloint2double(__double2hiint(a) | (yh & (int)0x80000000), __double2loint(a));
+}
+
+// 1 / sqrt(x) as the two IEEE operations round it: s to 2^-80 before its rounding
+// (Newton steps from the hardware's 20-bit estimate and the exact residual), then
+// 1 / s to 2^-80 from the same estimate.  9 FP64 operations; the root and the
+// division by themselves take about 18.  k0 = d0 / |d| - 1 cancels near the direct
+// beam, so a last place here is seen in g.
+__device__ __forceinline__ double inv_sqrt(double x) {
+    const int hi = __double2hiint(x);
+    if (hi < 0x01000000 || hi > 0x7e000000) return ddiv(1., __dsqrt_rn(x));
+    const double r = rsqrt_approx(x), s0 = x * r, h0 = times_pow2<-1>(r);
+    const double e = fma(-s0, h0, 0.5);
+    const double s1 = fma(s0, e, s0), h1 = fma(h0, e, h0);
+    const double s = fma(fma(-s1, s1, x), h1, s1);
+    const double y = times_pow2<1>(h1);
+    return fma(fma(-s, y, 1.), y, y);
+}
 
 //
 // Two specialisations give results identical to the general expression
@@ -65,7 +203,7 @@ __device__ __forceinline__ void peak_geometry(const GvParams& P, double x0, doub
         r.d1 = x1;
         r.d2 = x2;
     }
-    r.inv = ddiv(1., __dsqrt_rn(ddot3(r.d0, r.d1, r.d2, r.d0, r.d1, r.d2)));
+    r.inv = inv_sqrt(ddot3(r.d0, r.d1, r.d2, r.d0, r.d1, r.d2));
     r.k0 = dmul(P.ds, dsub(dmul(r.d0, r.inv), 1.));
     r.k1 = dmul(dmul(P.ds, r.d1), r.inv);
     r.k2 = dmul(dmul(P.ds, r.d2), r.inv);
@@ -85,9 +223,10 @@ __device__ __forceinline__ void peak_geometry(const GvParams& P, double x0, doub
 }
 
 // tth, eta, ds, g of one peak (ImageD11 src/cdiffraction.c:74-91)
-__device__ __forceinline__ void geometry_out(const PeakGeo& r, double* o) {
-    o[0] = dmul(kDeg, atan2(__dsqrt_rn(dadd(dmul(r.d1, r.d1), dmul(r.d2, r.d2))), r.d0));
-    o[1] = dmul(kDeg, atan2(-r.d1, r.d2));
+__device__ __forceinline__ void geometry_out(const PeakGeo& r,
+                                             const AtanShared& tab, double* o) {
+    o[0] = dmul(kDeg, fast_atan2(__dsqrt_rn(dadd(dmul(r.d1, r.d1), dmul(r.d2, r.d2))), r.d0, tab));
+    o[1] = dmul(kDeg, fast_atan2(-r.d1, r.d2, tab));
     o[2] = __dsqrt_rn(ddot3(r.k0, r.k1, r.k2, r.k0, r.k1, r.k2));
     o[3] = r.g0;
     o[4] = r.g1;
@@ -100,6 +239,8 @@ __global__ void __launch_bounds__(kGeoThreads)
 k_geometry(const double* __restrict__ xyz, const double* __restrict__ omega, GvParams P,
            double* __restrict__ out, float4* __restrict__ g4, int64_t n) {
     constexpr int OUTW = MODE == 0 ? 3 : 6;
+    __shared__ AtanShared s_tab;  // (MODE 0 has no angles and no table)
+    if (MODE == 1) s_tab.load();
     __shared__ double s_in[3 * kGeoThreads];
     __shared__ double s_out[OUTW * kGeoThreads];
     const int tid = threadIdx.x;
@@ -124,7 +265,7 @@ k_geometry(const double* __restrict__ xyz, const double* __restrict__ omega, GvP
                 if (g4)
                     g4[base + tid] = make_float4((float)r.g0, (float)r.g1, (float)r.g2, 0.f);
             } else {
-                geometry_out(r, s_out + 6 * tid);
+                geometry_out(r, s_tab, s_out + 6 * tid);
             }
         }
         __syncthreads();
@@ -152,7 +293,9 @@ __global__ void __launch_bounds__(kGeoThreads, 4)
 k_geometry_tma(const double* __restrict__ xyz, const double* __restrict__ omega, GvParams P,
                double* __restrict__ out, float4* __restrict__ g4, int64_t n) {
     constexpr int OUTW = MODE == 0 ? 3 : 6;
-    constexpr int S = 4;
+    constexpr int S = MODE == 0 ? 4 : 3;  // MODE 1 also holds the table (48 KB in all)
+    __shared__ AtanShared s_tab;  // (MODE 0 has no angles and no table)
+    if (MODE == 1) s_tab.load();
     __shared__ __align__(128) double s_x[S][3 * kGeoThreads];
     __shared__ __align__(128) double s_w[S][kGeoThreads];
     __shared__ __align__(16) double s_out[OUTW * kGeoThreads];
@@ -213,7 +356,7 @@ k_geometry_tma(const double* __restrict__ xyz, const double* __restrict__ omega,
                 s_out[3 * tid + 2] = r.g2;
                 if (g4) g4[base + tid] = make_float4((float)r.g0, (float)r.g1, (float)r.g2, 0.f);
             } else {
-                geometry_out(r, s_out + 6 * tid);
+                geometry_out(r, s_tab, s_out + 6 * tid);
             }
         }
         __syncthreads();  // stage consumed by every lane; s_out complete
@@ -275,61 +418,71 @@ k_xlylzl(const double* __restrict__ s, const double* __restrict__ f, XyzParams P
 // produced by the same operations as the two separate kernels, so the results
 // are identical to calling them in turn.  sc, fc, omega are read once with
 // the next tile's loads issued before the current tile is computed.
+//
+// A warp owns tiles of 32 peaks: its outputs go through its own part of shared
+// memory, so no warp waits for another.  10M peaks with the lab positions: 225 us with
+// the library's arctangents and a CTA's 256 peaks behind two barriers, 178 now (5.4
+// TB/s); two waves of CTAs, since one ended unevenly (186).
 template <bool XYZ, bool G4>
 __global__ void __launch_bounds__(kGeoThreads, 4)
 k_update_geometry(const double* __restrict__ sc, const double* __restrict__ fc,
                   const double* __restrict__ omega, XyzParams X, GvParams P,
                   double* __restrict__ xyz, double* __restrict__ out, float4* __restrict__ g4,
                   int64_t n) {
+    __shared__ AtanShared s_tab;
     __shared__ double s_xyz[XYZ ? 3 * kGeoThreads : 1];
     __shared__ double s_out[6 * kGeoThreads];
-    const int tid = threadIdx.x;
-    const int64_t ntiles = (n + kGeoThreads - 1) / kGeoThreads;
+    s_tab.load();
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* const wx = s_xyz + (XYZ ? 96 * warp : 0);
+    double* const wo = s_out + 192 * warp;
+    const int64_t step = (int64_t)gridDim.x * kGeoThreads;
     double sn = 0., fn = 0., on = 0.;
-    auto load = [&](int64_t t) {
-        const int64_t k = t * kGeoThreads + tid;
-        if (t < ntiles && k < n) {
+    auto load = [&](int64_t base) {
+        const int64_t k = base + lane;
+        if (k < n) {
             sn = __ldcs(sc + k);
             fn = __ldcs(fc + k);
             on = __ldcs(omega + k);
         }
     };
-    load(blockIdx.x);
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    int64_t base = (int64_t)blockIdx.x * kGeoThreads + 32 * warp;
+    load(base);
+    for (; base < n; base += step) {
         const double s = sn, f = fn, om = on;
-        load(t + gridDim.x);
-        const int64_t base = t * kGeoThreads;
-        const int cnt = (int)min((int64_t)kGeoThreads, n - base);
-        if (tid < cnt) {
+        load(base + step);
+        const int cnt = (int)min((int64_t)32, n - base);
+        if (lane < cnt) {
             const double v1 = dmul(dsub(f, X.p[1]), X.p[3]);
             const double v2 = dmul(dsub(s, X.p[0]), X.p[2]);
             double x[3];
 #pragma unroll
             for (int j = 0; j < 3; j++) {
                 x[j] = dadd(dadd(dmul(X.r[3 * j + 1], v1), dmul(X.r[3 * j + 2], v2)), X.dist[j]);
-                if (XYZ) s_xyz[3 * tid + j] = x[j];
+                if (XYZ) wx[3 * lane + j] = x[j];
             }
             PeakGeo r;
             peak_geometry(P, x[0], x[1], x[2], om, r);
-            geometry_out(r, s_out + 6 * tid);
-            if (G4) g4[base + tid] = make_float4((float)r.g0, (float)r.g1, (float)r.g2, 0.f);
+            geometry_out(r, s_tab, wo + 6 * lane);
+            if (G4) g4[base + lane] = make_float4((float)r.g0, (float)r.g1, (float)r.g2, 0.f);
         }
-        __syncthreads();
+        __syncwarp();
         if (XYZ) {
             double* dx = xyz + 3 * base;
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                const int e = tid + j * kGeoThreads;
-                if (e < 3 * cnt) __stcs(dx + e, s_xyz[e]);
+                const int e = lane + 32 * j;
+                if (e < 3 * cnt) __stcs(dx + e, wx[e]);
             }
         }
         double* dst = out + 6 * base;
 #pragma unroll
         for (int j = 0; j < 6; j++) {
-            const int e = tid + j * kGeoThreads;
-            if (e < 6 * cnt) __stcs(dst + e, s_out[e]);
+            const int e = lane + 32 * j;
+            if (e < 6 * cnt) __stcs(dst + e, wo[e]);
         }
-        __syncthreads();
+        __syncwarp();
     }
 }
 
@@ -478,7 +631,7 @@ extern "C" int id11b_dev_update_geometry(const double* sc, const double* fc, con
     for (int i = 0; i < 3; i++) X.dist[i] = dist_host[i];
     GvParams P = make_gv_params(omegasign, wvln, wedge, chi, t_host);
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = geo_grid_tma(n);
+    const int grid = geo_grid(n);
     if (xlylzl && g4)
         k_update_geometry<true, true><<<grid, kGeoThreads, 0, st>>>(sc, fc, omega, X, P, xlylzl,
                                                                     out, (float4*)g4, n);

@@ -66,3 +66,43 @@ def test_ctransform_methods_match_drop_in(cuda):
     assert np.array_equal(g, out[:, 3:])
     with pytest.raises(ValueError):
         ct.sf2geometry(sc, fc[:10], om)
+
+
+@pytest.mark.parametrize("kind", ["nodes", "tiny", "special"])
+def test_angles(kind, cuda):
+    """Two-theta and eta of given positions (no rotation, no translation, so the
+    diffraction vector is the position) in every octant: ratios at and between the
+    arctangent table's nodes, tiny ratios, and what goes to the library's function.
+    Against numpy with 64-bit mantissas: the root before (1/2 ulp), the arctangent
+    (1 ulp) and the degrees (1/2 ulp and the constant's 1/2), each up to doubled by
+    the next one's spacing: 5 ulp."""
+    from imaged11_b200 import transform
+    rng = np.random.default_rng(73)
+    if kind == "nodes":
+        r = (np.arange(0, 129)[:, None] / 128.0 + [0.0, 1e-16, -1e-9, 1e-9, 3e-3]).ravel()
+        r = np.abs(r)
+        y, z = np.r_[r, np.ones_like(r)] * 1e4, np.r_[np.ones_like(r), r] * 1e4
+    elif kind == "tiny":
+        r = 10.0 ** rng.uniform(-40, -2, 3000)
+        y, z = np.r_[r, np.ones_like(r)] * 37.0, np.r_[np.ones_like(r), r] * 37.0
+    else:
+        v = np.array([0.0, 1.0, np.inf, np.nan, 2.0 ** -101, 2.0 ** -100, 2.0 ** 100, 2.0 ** 101,
+                      1e-160, 1e150])
+        y, z = (a.ravel() for a in np.meshgrid(v, v))
+    y, z = np.r_[y, -y, y, -y], np.r_[z, z, -z, -z]
+    xyz = np.stack([rng.choice(z, len(z)), y, z], axis=1)
+    p = dict(_pars(rng, False), wedge=0.0, chi=0.0)
+    out = transform.Ctransform(p).xyz2geometry(xyz, np.zeros(len(xyz)), 0.0, 0.0, 0.0)
+    d = xyz.astype(np.longdouble)
+    deg = np.longdouble(180) / np.arctan2(np.longdouble(0), np.longdouble(-1))
+    with np.errstate(all="ignore"):
+        q = np.sqrt(xyz[:, 1] ** 2 + xyz[:, 2] ** 2)      # overflows where the kernel's does
+        mid = (q > 1e-100) & (q < 1e150)
+        q = np.where(mid, np.sqrt(d[:, 1] ** 2 + d[:, 2] ** 2), q)
+        want = np.stack([np.arctan2(q, d[:, 0]), np.arctan2(-d[:, 1], d[:, 2])], axis=1) * deg
+    near = want.astype(np.float64)
+    assert np.array_equal(np.isnan(out[:, :2]), np.isnan(near))
+    ok = np.isfinite(near)
+    assert np.all(np.abs(out[:, :2].astype(np.longdouble) - want)[ok] <=
+                  5 * np.spacing(np.abs(near[ok])))
+    assert np.array_equal(np.signbit(out[:, 1][ok[:, 1]]), np.signbit(near[:, 1][ok[:, 1]]))
