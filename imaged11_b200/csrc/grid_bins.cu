@@ -73,9 +73,6 @@ constexpr int kEW = ID11B_ENUM_WARPS;
 constexpr int kET = 32 * kEW;
 constexpr int kJT = 256;            // threads per join CTA (one row at a time)
 constexpr int kJW = kJT / 32;
-#ifndef ID11B_JOIN_RANKED
-#define ID11B_JOIN_RANKED 1
-#endif
 #ifndef ID11B_JOIN_BMAX
 #define ID11B_JOIN_BMAX 4096
 #endif
@@ -136,6 +133,8 @@ struct JoinParams {
     int ord[ID11B_MAX_TOLS];
     double fix;                    // fixed-point scale of the sums (fixsum_scale)
     float hmax;
+    uint64_t nlo2[ID11B_MAX_TOLS];  // {-lo, -lo}
+    unsigned wband;                 // bits of the widest hi - lo
     // y/z region of row (iy, iz): [rlo + iy * cs, rhi + (iy + 1) * cs] (the
     // cell widened by W + eps; eps covers the FP32 rounding of the box
     // centres' cells and of these bounds); the halo in whole cells
@@ -209,6 +208,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 // FP32 form of a UBI's plan for the candidate work of the enumeration.  The
@@ -792,69 +796,67 @@ struct Staged {  // the tile of staged g, structure of arrays (pairs read as 64 
 // instructions (lane by lane the scalar operations): UBI.g - hkl with the
 // subtraction folded into the first FMA (hh holds -hkl), three roundings of
 // partial sums below |hkl| + S gmax.
-__device__ __forceinline__ void screen_pair(const Staged& t, int q, const uint64_t uu[9],
-                                            const uint64_t hh[3], float& sa, float& sb) {
+__device__ __forceinline__ uint64_t screen_two(const Staged& t, int q, const uint64_t uu[9],
+                                               const uint64_t hh[3]) {
     const uint64_t gx = *reinterpret_cast<const uint64_t*>(t.x + q);
     const uint64_t gy = *reinterpret_cast<const uint64_t*>(t.y + q);
     const uint64_t gz = *reinterpret_cast<const uint64_t*>(t.z + q);
     const uint64_t d0 = fma2(uu[2], gz, fma2(uu[1], gy, fma2(uu[0], gx, hh[0])));
     const uint64_t d1 = fma2(uu[5], gz, fma2(uu[4], gy, fma2(uu[3], gx, hh[1])));
     const uint64_t d2 = fma2(uu[8], gz, fma2(uu[7], gy, fma2(uu[6], gx, hh[2])));
-    upk2(fma2(d2, d2, fma2(d1, d1, mul2(d0, d0))), sa, sb);
+    return fma2(d2, d2, fma2(d1, d1, mul2(d0, d0)));
 }
 
 // The box of one lane against staged g [ga, gb), counting.  The range is
 // widened to even bounds (an odd tile ends with a NaN g): testing g beyond a
 // run's range is harmless, every g of a tile being tested at most once per
-// box.  Counting is free of branches; one branch per pair of g catches the
-// rare band cases.
+// box.
 //
-// RANKED (lo and hi both non-decreasing in j): a value below lo_j is below
-// every later lo, so the only band it can lie in is that of the largest lo_j
-// not above it -- one select chain and one compare instead of a test per
-// tolerance.  (If s lies in band i <= J, J the largest j with lo_j <= s, then
-// s < hi_i <= hi_J.)
-template <int NT, bool RANKED>
+// The loop is bound by issue (58% of the slots busy, half of them counting), so a
+// tolerance takes three instructions per two g: d = s - lo as a packed addition,
+// and its sign bits added to the count.  (The rounded d keeps the sign of the
+// exact one; a NaN s gives the canonical NaN, whose sign is clear.)  A value of
+// some band has 0 <= d <= hi - lo: as unsigned integers the smallest d of kNear g
+// is then at most the widest band's, one test for all of them, and those g are
+// looked at again tolerance by tolerance.  20,000 UBIs x 1.1M g at three tolerances:
+// the join takes 1445 us, with compares and a band test per pair 1556.
+constexpr int kNear = 8;
+
+template <int NT>
 __device__ __forceinline__ void test_range(const Staged& t, int ga, int gb, const uint64_t uu[9],
                                            const uint64_t hh[3], const float* hkf,
                                            const JoinParams& P, const double* __restrict__ ubis,
                                            int64_t ubi, const double* __restrict__ gs, int cnt[NT],
                                            unsigned& ntest) {
-    for (int q = ga & ~1; q < gb; q += 2) {
-        float sa, sb;
-        screen_pair(t, q, uu, hh, sa, sb);
-        bool ra, rb;
-        if (RANKED) {
-            bool ia[NT], ib[NT];
+    for (int q = ga & ~1; q < gb;) {
+        const int q0 = q, qe = min(q + kNear, gb);
+        unsigned near = 0xffffffffu;
+        for (; q < qe; q += 2) {
+            const uint64_t s = screen_two(t, q, uu, hh);
 #pragma unroll
             for (int j = 0; j < NT; j++) {
-                ia[j] = sa < P.lo[j];
-                ib[j] = sb < P.lo[j];
-                cnt[j] += (int)ia[j] + (int)ib[j];
-            }
-            float ha = P.hi[NT - 1], hb = P.hi[NT - 1];
-#pragma unroll
-            for (int j = NT - 2; j >= 0; j--) {
-                ha = ia[j + 1] ? P.hi[j] : ha;
-                hb = ib[j + 1] ? P.hi[j] : hb;
-            }
-            ra = !ia[0] && sa < ha;
-            rb = !ib[0] && sb < hb;
-        } else {
-            ra = rb = false;
-#pragma unroll
-            for (int j = 0; j < NT; j++) {
-                const bool ia = sa < P.lo[j], ib = sb < P.lo[j];
-                cnt[j] += (int)ia + (int)ib;
-                ra |= !ia && sa < P.hi[j];
-                rb |= !ib && sb < P.hi[j];
+                const uint64_t d = add2(s, P.nlo2[j]);
+                const unsigned da = (unsigned)d, db = (unsigned)(d >> 32);
+                cnt[j] += da >> 31;
+                cnt[j] += db >> 31;
+                near = min(near, min(da, db));
             }
         }
-        if (ra || rb) {
-            ntest += (unsigned)ra + (unsigned)rb;
-            if (ra) rare_pair<NT>(sa, t.pos[q], P, ubis, ubi, gs, hkf, cnt);
-            if (rb) rare_pair<NT>(sb, t.pos[q + 1], P, ubis, ubi, gs, hkf, cnt);
-        }
+        if (near <= P.wband)
+            for (int k = q0; k < qe; k += 2) {
+                float v[2];
+                upk2(screen_two(t, k, uu, hh), v[0], v[1]);
+#pragma unroll 1
+                for (int e = 0; e < 2; e++) {
+                    bool in = false;
+#pragma unroll
+                    for (int j = 0; j < NT; j++) in |= !(v[e] < P.lo[j]) && v[e] < P.hi[j];
+                    if (in) {
+                        ntest++;
+                        rare_pair<NT>(v[e], t.pos[k + e], P, ubis, ubi, gs, hkf, cnt);
+                    }
+                }
+            }
     }
 }
 
@@ -878,7 +880,7 @@ __device__ __forceinline__ void exact_range(const Staged& t, int ga, int gb, con
         int left = 32;
         for (int q = q0; q < qe; q += 2) {
             float sa, sb;
-            screen_pair(t, q, uu, hh, sa, sb);
+            upk2(screen_two(t, q, uu, hh), sa, sb);
             mask = (mask >> 2) | (sa < hmax ? 0x40000000u : 0u) | (sb < hmax ? 0x80000000u : 0u);
             left -= 2;
         }
@@ -978,7 +980,7 @@ __device__ __forceinline__ void block_scan(const int* a, int* b, int len, int* s
 // tiles of at most kGMax, each sorted by x cell, and every run of 32 sorted
 // boxes (one warp) is tested against the staged g in the x cells its boxes
 // can reach.
-template <int NT, bool SUMS, bool RANKED, int AS = 0>
+template <int NT, bool SUMS, int AS = 0>
 __global__ void __launch_bounds__(kJT, kJoinMinBlocks)
 k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nrows,
        int nhalo, BinInfo* __restrict__ info, const float4* __restrict__ packs,
@@ -999,7 +1001,7 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
     int* s_gs = s_gh + nh1;          // staged g before each x cell of the tile
     int* s_rp = s_gs + nh1;          // halo rows: candidate prefix (nhalo + 1)
     int* s_rs = s_rp + (nhalo + 1);  // halo rows: first g
-    __shared__ int s_row, s_w[kJW], s_base;
+    __shared__ int s_row, s_w[kJW], s_base, s_run;
     const Staged T{s_gx, s_gy, s_gz, s_gp};
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned ntest = 0;
@@ -1122,6 +1124,7 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                     cend = min(cend + kJT, ncand);
                 }
                 block_scan(s_gh, s_gs, gw + 1, s_w);
+                if (threadIdx.x == 0) s_run = kJW;
                 for (int x = threadIdx.x; x <= gw; x += kJT) s_gh[x] = 0;
                 __syncthreads();
                 for (int q = c0 + threadIdx.x; q < cend; q += kJT) {
@@ -1144,8 +1147,17 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                     s_gp[s_gs[gw]] = 0;
                 }
                 __syncthreads();
-                // runs of 32 sorted boxes, one warp each
-                for (int k0 = 32 * w; k0 < nb; k0 += 32 * kJW) {
+                // runs of 32 sorted boxes, one warp each.  Where pairs are evaluated
+                // exactly the runs' times differ and a warp takes the next run when it
+                // is done (10,000 x 560k with sums: 619 us, 656 with fixed turns);
+                // counting alone, fixed turns are as fast on long rows and faster on
+                // short ones (1,500 x 60k: 60 us, 63).
+                auto next_run = [&] {
+                    int k = 0;
+                    if (lane == 0) k = atomicAdd(&s_run, 1);
+                    return 32 * __shfl_sync(0xffffffffu, k, 0);
+                };
+                for (int k0 = 32 * w; k0 < nb; k0 = SUMS ? next_run() : k0 + 32 * kJW) {
                     const int nrun = min(32, nb - k0);
                     const int ga = s_gs[max(box_fx(s_box[k0]) - P.Rx, gxa) - gxa];
                     const int gb = s_gs[min(box_fx(s_box[k0 + nrun - 1]) + P.Rx, gxb) - gxa + 1];
@@ -1185,8 +1197,7 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                         int cnt[NT];
 #pragma unroll
                         for (int j = 0; j < NT; j++) cnt[j] = 0;
-                        test_range<NT, RANKED>(T, ga, gb, uu, hh, hkf, P, ubis, ubi, gs, cnt,
-                                               ntest);
+                        test_range<NT>(T, ga, gb, uu, hh, hkf, P, ubis, ubi, gs, cnt, ntest);
 #pragma unroll
                         for (int j = 0; j < NT; j++)
                             if (cnt[j]) atomicAdd(counts + ubi * NT + P.ord[j], cnt[j]);
@@ -1323,33 +1334,18 @@ k_assign_fallback(const double* __restrict__ ubis, const int* __restrict__ list,
     }
 }
 
-template <int NT, bool SUMS, bool RANKED, int AS = 0>
-int launch_join_k(int grid, size_t smem, const uint64_t* recs, const int* rstart, int nrows,
+template <int NT, bool SUMS, int AS = 0>
+int launch_join(int grid, size_t smem, const uint64_t* recs, const int* rstart, int nrows,
                   int nhalo, BinInfo* info, const float4* packs, const double* ubis, Header* H,
                   const int* start, const double* gs, const float4* g4, const JoinParams& P,
                   int* counts, double* sums, cudaStream_t st) {
-    ID11B_CHECK(cudaFuncSetAttribute(k_join<NT, SUMS, RANKED, AS>,
+    ID11B_CHECK(cudaFuncSetAttribute(k_join<NT, SUMS, AS>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_join<NT, SUMS, RANKED, AS><<<grid, kJT, smem, st>>>(recs, rstart, nrows, nhalo, info, packs,
+    k_join<NT, SUMS, AS><<<grid, kJT, smem, st>>>(recs, rstart, nrows, nhalo, info, packs,
                                                           ubis, H, start, gs, g4, P, counts,
                                                           sums);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
-}
-
-// the ranked test where it applies (no sums, at least two tolerances, the
-// thresholds monotone); the per-tolerance test otherwise
-template <int NT, bool SUMS>
-int launch_join(int grid, size_t smem, bool ranked, const uint64_t* recs, const int* rstart,
-                int nrows, int nhalo, BinInfo* info, const float4* packs, const double* ubis,
-                Header* H, const int* start, const double* gs, const float4* g4,
-                const JoinParams& P, int* counts, double* sums, cudaStream_t st) {
-    if (!SUMS && NT > 1 && ranked)
-        return launch_join_k<NT, SUMS, !SUMS && NT != 1>(grid, smem, recs, rstart, nrows, nhalo,
-                                                         info, packs, ubis, H, start, gs, g4, P,
-                                                         counts, sums, st);
-    return launch_join_k<NT, SUMS, false>(grid, smem, recs, rstart, nrows, nhalo, info, packs,
-                                          ubis, H, start, gs, g4, P, counts, sums, st);
 }
 
 template <int NT, bool SUMS>
@@ -1384,10 +1380,8 @@ int ctas_per_sm(K kernel, int threads, size_t smem) {
 }
 
 template <int NT, bool SUMS>
-int join_ctas(size_t smem, bool ranked) {
-    if (!SUMS && NT > 1 && ranked)
-        return ctas_per_sm(k_join<NT, SUMS, !SUMS && NT != 1>, kJT, smem);
-    return ctas_per_sm(k_join<NT, SUMS, false>, kJT, smem);
+int join_ctas(size_t smem) {
+    return ctas_per_sm(k_join<NT, SUMS>, kJT, smem);
 }
 
 // float nearest to x in the given direction (x itself when representable)
@@ -1471,7 +1465,6 @@ extern "C" int64_t id11b_grid_bins_workspace_bytes(int64_t m, int32_t nx, int32_
 struct JoinLaunch {
     int grid;
     size_t smem;
-    bool ranked;
     const uint64_t* recs;
     const int* rstart;
     int nrows, nhalo;
@@ -1489,7 +1482,7 @@ struct JoinLaunch {
 // region; then for each pass, for each range, the box records (written again
 // only when there are several ranges) and join(pass, launch), and after the
 // ranges after(pass, fallback list, its length, g outside the regular range,
-// ...).  ctas(smem, ranked): resident join CTAs per SM.  P.fix is T.fix; the
+// ...).  ctas(smem): resident join CTAs per SM.  P.fix is T.fix; the
 // assignment's fields of P are set by the caller's P0.
 template <class Ctas, class Join, class After>
 static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, int32_t xsub,
@@ -1591,7 +1584,6 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     // row sum of the binned UBIs; the region geometry
     JoinParams P = P0;
     P.fix = T.fix;
-    bool ranked = false;
     {
         const double G = -hh.lo;
         float smax;
@@ -1604,6 +1596,7 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
         // origin in every component, and hkl = UBI.c)
         const double E = kEps32 * (double)smax * (8.0 * G + 3.0 * W) * (1. + 1e-6);
         P.hmax = 0.f;
+        float wband = 0.f;
         // ascending order of tolerance (stable), unused slots last
         int ord[ID11B_MAX_TOLS];
         for (int j = 0; j < ID11B_MAX_TOLS; j++) ord[j] = j;
@@ -1616,11 +1609,14 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
             P.hi[j] = float_ru(TT + band);
             P.t2[j] = TT;
             P.ord[j] = ord[j];
-            if (j < ntol) P.hmax = fmaxf(P.hmax, P.hi[j]);
+            if (j < ntol) {
+                P.hmax = fmaxf(P.hmax, P.hi[j]);
+                wband = fmaxf(wband, float_ru((double)P.hi[j] - (double)P.lo[j]));
+            }
+            const float nlo[2] = {-P.lo[j], -P.lo[j]};
+            memcpy(&P.nlo2[j], nlo, sizeof(nlo));
         }
-        ranked = ID11B_JOIN_RANKED != 0;
-        for (int j = 1; j < ntol; j++)
-            ranked = ranked && P.lo[j] >= P.lo[j - 1] && P.hi[j] >= P.hi[j - 1];
+        memcpy(&P.wband, &wband, sizeof(wband));
         // eps: far above the FP32 rounding of the box centres' cells (about
         // 2^-23 of |c| + |lo|) and of the FP32 region bounds
         const double eps = 2e-5 * (1. + G);
@@ -1639,7 +1635,7 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
                          4 * sizeof(int) * (size_t)(std::max(nxx, nhalo) + 1) +
                          2 * sizeof(int) * (size_t)(nhalo + 1) +
                          (exact ? sizeof(Pend) * kPend * kJW : 0);
-    const int jgrid = num_sms() * ctas(jsmem, ranked);
+    const int jgrid = num_sms() * ctas(jsmem);
     cudaEvent_t ev0 = t_join_start, ev1 = t_join_stop;
     t_join_start = t_join_stop = nullptr;
     bool ev0_done = false;
@@ -1673,7 +1669,7 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
                 ID11B_CHECK(cudaEventRecord(ev0, st));
                 ev0_done = true;
             }
-            const int rc = join(pass, JoinLaunch{jgrid, jsmem, ranked, recs, rstart, nrows, nhalo,
+            const int rc = join(pass, JoinLaunch{jgrid, jsmem, recs, rstart, nrows, nhalo,
                                                  info, packs, H, start, gs, g4, &P});
             if (rc) return rc;
         }
@@ -1715,9 +1711,9 @@ extern "C" int id11b_dev_score_grid_bins(const double* ubis, int64_t m, const do
     JoinParams P0 = {};
     const int rc = bins_pipeline(
         ubis, m, n, nx, xsub, gridbuf, T, ntol, tmax, ws, ws_bytes, st, 1, sums != nullptr, P0,
-        [&](size_t smem, bool ranked) { return ID11B_BINS_DISPATCH(join_ctas, smem, ranked); },
+        [&](size_t smem) { return ID11B_BINS_DISPATCH(join_ctas, smem); },
         [&](int, const JoinLaunch& J) {
-            return ID11B_BINS_DISPATCH(launch_join, J.grid, J.smem, J.ranked, J.recs, J.rstart,
+            return ID11B_BINS_DISPATCH(launch_join, J.grid, J.smem, J.recs, J.rstart,
                                        J.nrows, J.nhalo, J.info, J.packs, ubis, J.H, J.start,
                                        J.gs, J.g4, *J.P, counts, sums, st);
         },
@@ -1762,14 +1758,14 @@ extern "C" int id11b_dev_assign_grid_bins(const double* ubis, int64_t m, const d
     P0.lab = lab;
     return bins_pipeline(
         ubis, m, n, nx, xsub, gridbuf, T, 1, tol, ws, ws_bytes, st, 2, true, P0,
-        [&](size_t smem, bool) { return ctas_per_sm(k_join<1, true, false, 1>, kJT, smem); },
+        [&](size_t smem) { return ctas_per_sm(k_join<1, true, 1>, kJT, smem); },
         [&](int pass, const JoinLaunch& J) {
             if (pass == 0)
-                return launch_join_k<1, true, false, 1>(J.grid, J.smem, J.recs, J.rstart, J.nrows,
+                return launch_join<1, true, 1>(J.grid, J.smem, J.recs, J.rstart, J.nrows,
                                                         J.nhalo, J.info, J.packs, ubis, J.H,
                                                         J.start, J.gs, J.g4, *J.P, nullptr,
                                                         nullptr, st);
-            return launch_join_k<1, true, false, 2>(J.grid, J.smem, J.recs, J.rstart, J.nrows,
+            return launch_join<1, true, 2>(J.grid, J.smem, J.recs, J.rstart, J.nrows,
                                                     J.nhalo, J.info, J.packs, ubis, J.H, J.start,
                                                     J.gs, J.g4, *J.P, nullptr, nullptr, st);
         },

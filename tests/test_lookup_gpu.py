@@ -163,3 +163,28 @@ def test_box_estimate(m, cuda):
             want += est if est <= g.n else 0.0
     got = batch.bins_box_estimate(torch.from_numpy(u).cuda(), g, tol)
     assert abs(got - (1.25 * want + 64 * m)) <= 1 + 1e-9 * want
+
+
+@pytest.mark.parametrize("tols", [[0.05], [0.0], [1e-5, 0.05], [0.05, 0.05], [0.1, 0.05, 0.03],
+                                  [0.39, 1e-4, 0.05, np.nextafter(0.05, 1)]])
+@pytest.mark.parametrize("n", [4000, 4001])
+def test_binned_counts_at_the_thresholds(oracle, tols, n, cuda):
+    """Most g lie one tolerance from a lattice point to within rounding, so their
+    FP32 values fall into the bands that are evaluated exactly (and into several at
+    once for equal tolerances); the counts must be the oracle's."""
+    import torch
+    from imaged11_b200 import batch
+    rng = np.random.default_rng(n)
+    ub = np.linalg.qr(rng.normal(size=(3, 3)))[0] / 4.05
+    hkl = rng.integers(-5, 6, (n, 3))
+    d = rng.normal(size=(n, 3))
+    d *= rng.choice(tols, n)[:, None] / np.linalg.norm(d, axis=1, keepdims=True)
+    g = (hkl + d) @ ub.T
+    u = np.linalg.inv(ub)[None] + rng.normal(size=(40, 3, 3)) * 1e-6
+    u[0] = np.linalg.inv(ub)
+    grid = batch.GvecGrid(torch.from_numpy(g).cuda())
+    want = oracle.score_many(u, g, tols)
+    for sums in (False, True):
+        got = batch.score_grid(u, grid, tols, method="bins", sums=sums)
+        got = got[0] if sums else got
+        assert np.array_equal(got.cpu().numpy(), want)
