@@ -7,10 +7,12 @@
 // widths w are conservative).  Here every box that can reach the data is
 // enumerated once per UBI (the lookup scorer's enumeration, its per-candidate
 // work in FP32 with the rounding folded into w) and the boxes are sorted by
-// the row of grid cells holding their centre (fixed y and z cell): counts per
-// block of 16 rows in shared memory per CTA, a scan, a second enumeration that
-// writes each CTA's boxes of a block as one sequential stream, and a split of
-// each block into its rows.  One CTA then takes one
+// the row of grid cells holding their centre (fixed y and z cell): each CTA of
+// the enumeration writes its boxes of a block of 16 rows as one sequential
+// stream, into room predicted from the UBIs' expected number of boxes per block
+// (k_stream_room; a stream that outgrows its room, or a workspace too small for
+// the prediction, falls back to counting and a second enumeration), and each
+// block is split into its rows.  One CTA then takes one
 // row: it sorts the row's boxes by x cell in shared memory, stages the
 // g-vectors of the row's region (its y/z cell widened by the largest half
 // width W, all x cells the boxes need) sorted by x cell, and every run of 32
@@ -111,7 +113,7 @@ constexpr int kJoinMinBlocks = ID11B_JOIN_MINB;  // resident join CTAs per SM co
 
 struct BinInfo {
     unsigned long long wmax_bits;  // largest (widened) box half width (positive doubles order as integers)
-    unsigned long long total;      // boxes enumerated by the first counting pass
+    unsigned long long total;      // boxes found by the first enumeration
     unsigned int smax_bits;        // largest row sum of |UBI| over binned UBIs (float, rounded up)
     int nfallback;                 // UBIs scored by the plain scan
     int next_row;                  // row counter of the join
@@ -124,7 +126,7 @@ struct BinInfo {
 };
 
 // Everything the join needs that is uniform over the launch, computed on the
-// host after the counting pass (kernel parameters: no registers).
+// host after the first enumeration (kernel parameters: no registers).
 struct JoinParams {
     // thresholds in ascending order of tolerance; ord[j]: the caller's index
     // of the j-th (where its count and sum are written)

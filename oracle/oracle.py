@@ -170,6 +170,26 @@ class Oracle(_Lib):
                                 _ptr(npk), _ptr(d))
         return u.reshape(-1, 3, 3), npk, d
 
+    def assign_seq(self, ubis, gv, tol, drlv2, labels):
+        """score_and_assign of grains 0 .. m-1 in order on (drlv2, labels),
+        updated in place (float64 / int32 C arrays); a peak's outcome depends on
+        that peak alone, so the peaks are shared among threads."""
+        from concurrent.futures import ThreadPoolExecutor
+        u = _c64(ubis).reshape(-1, 9)
+        g = _c64(gv).reshape(-1, 3)
+        assert drlv2.dtype == np.float64 and labels.dtype == np.int32
+        assert drlv2.flags.c_contiguous and labels.flags.c_contiguous
+        f = self.lib.orc_score_and_assign
+        edges = np.linspace(0, len(g), self.max_threads() + 1).astype(int)
+
+        def run(k):
+            a, b = int(edges[k]), int(edges[k + 1])
+            for i in range(len(u)):
+                f(_ptr(u[i]), _ptr(g[a:b]), float(tol), _ptr(drlv2[a:b]), _ptr(labels[a:b]), i,
+                  b - a)
+        with ThreadPoolExecutor(len(edges) - 1) as pool:
+            list(pool.map(run, range(len(edges) - 1)))
+
     def inverse3x3(self, m):
         a = _c64(m).reshape(9).copy()
         rc = self.lib.orc_inverse3x3(_ptr(a))
