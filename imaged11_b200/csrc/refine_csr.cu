@@ -256,7 +256,10 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 // and 80.2 (128) with a CTA for every grain, 17 warp sums and five barriers a
 // round.  500 such grains 36.0 -> 17.0, 8,000 of up to 400 peaks, three rounds, 86
 // -> 35 us.  kSolo at 128 threads: 256 43.0, 512 43.2, 768 36.6, 1,024 41.9 us.
-constexpr int kSolo = 768;
+// The F32C variant does more per peak, so fewer go to one warp: the first of these 84
+// -> 69 us at 128 threads and 384 (768: 74; 64 threads: 91), 200 grains of 500 ..
+// 4,000 peaks 94 -> 46 (64 threads: 77).
+constexpr int kSoloFp64 = 768, kSoloF32c = 384;
 
 template <int NT, bool F32C = false>
 __global__ void __launch_bounds__(NT)
@@ -267,6 +270,7 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     __shared__ RefineSmem sm[NT / 32];
     __shared__ double s_red[NT / 32][17];
     __shared__ int s_next;
+    constexpr int kSolo = F32C ? kSoloF32c : kSoloFp64;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     int slot = blockIdx.x;
     while (slot < ngrains) {
@@ -392,6 +396,6 @@ extern "C" int id11b_dev_refine_csr_f32c(double* ubis, const double* gv, const i
     cudaStream_t st = (cudaStream_t)stream;
     int* queue = (int*)workspace;
     ID11B_CHECK(cudaMemsetAsync(queue, 0, sizeof(int), st));
-    return launch_refine<64, true>(ubis, gv, offsets, order, ngrains, tol * tol, iters, queue,
+    return launch_refine<128, true>(ubis, gv, offsets, order, ngrains, tol * tol, iters, queue,
                                    npk, mean_drlv2, st, gmax);
 }
