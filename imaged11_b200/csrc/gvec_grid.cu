@@ -464,22 +464,24 @@ __device__ __forceinline__ void lookup_batch(const volatile WarpPlan* wp, Batch*
         }
         bool full = !have;
         if (have) {
-            // prefixes of g (low half) and segments (high half) over the lanes
-            unsigned long long own = 0;
+            // prefixes of g (low bits) and segments (high bits) over the lanes
+            constexpr int kHigh = 24;
+            static_assert(32 * kRowsAhead * (kMark + 1) < 1 << kHigh && 32 * kRowsAhead < 256, "");
+            unsigned own = 0;
 #pragma unroll
             for (int k = 0; k < kRowsAhead; k++)
-                own += ((unsigned long long)(len[k] > 0) << 32) + (unsigned)min(len[k], kMark + 1);
-            unsigned long long incl = own;
+                own += ((unsigned)(len[k] > 0) << kHigh) + (unsigned)min(len[k], kMark + 1);
+            unsigned incl = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+                const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += t;
             }
-            const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
-            const int asum = (int)(unsigned)all, acnt = (int)(all >> 32);
+            const unsigned all = __shfl_sync(0xffffffffu, incl, 31);
+            const int asum = (int)(all & ((1u << kHigh) - 1)), acnt = (int)(all >> kHigh);
             if (acnt <= kSeg - nseg && asum <= kMark - total) {
-                int at = total + (int)(unsigned)(incl - own);
-                int slot = nseg + (int)((incl - own) >> 32);
+                int at = total + (int)((incl - own) & ((1u << kHigh) - 1));
+                int slot = nseg + (int)((incl - own) >> kHigh);
 #pragma unroll
                 for (int k = 0; k < kRowsAhead; k++)
                     if (len[k] > 0) {
