@@ -117,6 +117,7 @@ struct BinInfo {
     unsigned int smax_bits;        // largest row sum of |UBI| over binned UBIs (float, rounded up)
     int nfallback;                 // UBIs scored by the plain scan
     int next_row;                  // row counter of the join
+    int blk_done;                  // CTAs of k_blk_offsets that are done
     int overflow;                  // a stream was longer than its room: the records are not whole
     unsigned long long vmax_bits;  // largest sum of |det UBI| over an enumeration CTA's items
     unsigned long long wbound_bits;  // bound on the half widths, for the streams' room
@@ -164,13 +165,13 @@ __device__ __forceinline__ int box_rowlo(uint64_t r) {
 }
 
 struct BinLayout {
-    size_t info, packs, cnt_ubi, fallback, cta_blk, blktot, blkstart, room, rstart, tot, tmp,
-        recs, bytes;
+    size_t info, packs, cnt_ubi, fallback, cta_blk, blktot, blkstart, room, rstart, tmp, recs,
+        bytes;
 };
 
-// workspace: info | packs (m x 3 float4) | per-UBI box counts | fallback list |
+// workspace: info | per-UBI box counts | packs (m x 3 float4) | fallback list |
 // per-CTA block counts / offsets | block totals | block starts | streams' room
-// before each block | row starts | scan totals | boxes by block | boxes by row
+// before each block | row starts | boxes by block | boxes by row
 inline BinLayout bin_layout(int64_t m, int64_t nrows, int64_t cap) {
     BinLayout L;
     const size_t mm = (size_t)(m > 0 ? m : 1);
@@ -178,15 +179,14 @@ inline BinLayout bin_layout(int64_t m, int64_t nrows, int64_t cap) {
     const size_t cc = (size_t)(cap > 0 ? cap : 1);
     size_t o = 0;
     L.info = o;     o = al256(o + sizeof(BinInfo));
+    L.cnt_ubi = o;  o = al256(o + sizeof(int) * mm);  // (zeroed together with info)
     L.packs = o;    o = al256(o + 3 * sizeof(float4) * mm);
-    L.cnt_ubi = o;  o = al256(o + sizeof(int) * mm);
     L.fallback = o; o = al256(o + sizeof(int) * mm);
     L.cta_blk = o;  o = al256(o + sizeof(int) * (size_t)kMaxEnumCtas * (size_t)nblk);
-    L.blktot = o;   o = al256(o + sizeof(int) * (size_t)(nblk + 1));
+    L.blktot = o;   o = al256(o + sizeof(int) * (size_t)nblk);
     L.blkstart = o; o = al256(o + sizeof(int) * (size_t)(nblk + 1));
     L.room = o;     o = al256(o + sizeof(int) * (size_t)(nblk + 1));
     L.rstart = o;   o = al256(o + sizeof(int) * (size_t)(nrows + 1));
-    L.tot = o;      o = al256(o + sizeof(int) * (size_t)((nblk + 1 + kScanPer - 1) / kScanPer + 1));
     L.tmp = o;      o = al256(o + sizeof(uint64_t) * cc);
     L.recs = o;     o = al256(o + sizeof(uint64_t) * cc);
     L.bytes = o;
@@ -622,10 +622,15 @@ k_enum(int mode, const double* __restrict__ ubis, int64_t i0, int64_t mc, int pa
 }
 
 // Per block: the CTAs' counts turned into exclusive offsets inside the block
-// (in place), and the block's total.  One warp per block.
+// (in place), and the block's total.  One warp per block.  The last CTA done adds
+// the totals up to the blocks' starts (blkstart[nblk]: all boxes), which took a scan
+// of three launches.
 __global__ void __launch_bounds__(kGT)
-k_blk_offsets(int* __restrict__ cta_blk, int nctas, int nblk, int* __restrict__ blktot) {
-    const int lane = threadIdx.x & 31;
+k_blk_offsets(int* __restrict__ cta_blk, int nctas, int nblk, int* __restrict__ blktot,
+              int* __restrict__ blkstart, BinInfo* __restrict__ info) {
+    __shared__ int s_w[kGT / 32];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int64_t b = ((int64_t)blockIdx.x * kGT + threadIdx.x) >> 5; b < nblk;
          b += ((int64_t)gridDim.x * kGT) >> 5) {
         int run = 0;
@@ -638,6 +643,31 @@ k_blk_offsets(int* __restrict__ cta_blk, int nctas, int nblk, int* __restrict__ 
             run += tot;
         }
         if (lane == 0) blktot[b] = run;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&info->blk_done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int base = 0;
+    for (int b0 = 0; b0 < nblk; b0 += kGT) {  // uniform over the CTA
+        const int b = b0 + threadIdx.x;
+        int tot, all = 0;
+        int at = warp_excl_scan(b < nblk ? __ldcg(blktot + b) : 0, lane, tot);
+        if (lane == 0) s_w[w] = tot;
+        __syncthreads();
+        for (int q = 0; q < kGT / 32; q++) {
+            if (q < w) at += s_w[q];
+            all += s_w[q];
+        }
+        if (b < nblk) blkstart[b] = base + at;
+        base += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        blkstart[nblk] = base;
+        info->blk_done = 0;
     }
 }
 
@@ -697,7 +727,9 @@ __device__ __forceinline__ void each_box(const uint64_t* __restrict__ tmp, int p
 __global__ void __launch_bounds__(kRS)
 k_rowsplit(const uint64_t* __restrict__ tmp, const int* __restrict__ blkstart, int nblk,
            int nrows, int nseg, const int* __restrict__ cta_blk, const int* __restrict__ room,
-           int* __restrict__ rstart, uint64_t* __restrict__ recs) {
+           int* __restrict__ rstart, uint64_t* __restrict__ recs,
+           const BinInfo* __restrict__ info) {
+    if (nseg && info->overflow) return;  // the streams are not whole: the host counts first
     __shared__ int s_wh[kRSW][kRowBlock];
     __shared__ int s_off[kMaxEnumCtas + 1];
     const int w = threadIdx.x >> 5;
@@ -1430,6 +1462,13 @@ struct PinnedReport {
     }
 };
 thread_local PinnedReport t_report;
+
+struct Event {
+    cudaEvent_t e = nullptr;
+    ~Event() {
+        if (e) cudaEventDestroy(e);
+    }
+};
 }  // namespace
 
 extern "C" int id11b_dev_bins_box_estimate(const double* ubis, int64_t m, double rmax, double tmax,
@@ -1518,12 +1557,10 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     int* blkstart = (int*)(w + B.blkstart);
     int* room = (int*)(w + B.room);
     int* rstart = (int*)(w + B.rstart);
-    int* tot = (int*)(w + B.tot);
     uint64_t* tmp = (uint64_t*)(w + B.tmp);
     uint64_t* recs = (uint64_t*)(w + B.recs);
     ID11B_CHECK(cudaMemsetAsync(&H->nfallback, 0, 3 * sizeof(unsigned long long), st));
     if (m == 0) return ID11B_OK;
-    ID11B_CHECK(cudaMemsetAsync(info, 0, sizeof(BinInfo), st));
     // the enumeration's CTAs (same count and UBI ranges in both passes)
     static thread_local int enum_per_sm = 0;
     if (!enum_per_sm) enum_per_sm = ctas_per_sm(k_enum, kET, 0);
@@ -1545,7 +1582,16 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     // 2.19 -> 1.89 ms, 100,000 19.1 -> 15.3, 5,003 x 170k 0.56 -> 0.48; trials of 20
     // grains 2.48 -> 2.16; trials all of one grain, counted first, 2.57 -> 2.62.
     const bool once = m <= (int64_t(1) << kUbiBits);
-    if (parts > 1) ID11B_CHECK(cudaMemsetAsync(cnt_ubi, 0, sizeof(int) * (size_t)m, st));
+    ID11B_CHECK(cudaMemsetAsync(info, 0, parts > 1 ? B.cnt_ubi - B.info + sizeof(int) * (size_t)m
+                                                   : sizeof(BinInfo), st));
+    auto offsets = [&](int grid) {
+        k_blk_offsets<<<grid_for((int64_t)nblk * 32, kGT), kGT, 0, st>>>(cta_blk, grid, nblk, blktot,
+                                                                        blkstart, info);
+    };
+    auto rowsplit = [&](int nseg) {
+        k_rowsplit<<<(unsigned)std::min(nblk, num_sms() * kRSPerSM), kRS, 0, st>>>(
+            tmp, blkstart, nblk, nrows, nseg, cta_blk, room, rstart, recs, info);
+    };
     if (once) {
         const int64_t per = enum_per(m);
         k_stream_room<<<(unsigned)((m * parts + per - 1) / per), kRoomT, 0, st>>>(
@@ -1560,7 +1606,18 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     k_report<<<1, 96, 0, st>>>(info, H, (const int*)(g + L.spos + sizeof(int) * (size_t)n),
                                t_report.p);
     ID11B_CHECK_LAUNCH();
-    ID11B_CHECK(cudaStreamSynchronize(st));
+    // the offsets and the split need nothing of the host: they run while it waits for
+    // the report and prepares the join (the device was idle for 20 us)
+    Event reported;
+    ID11B_CHECK(cudaEventCreateWithFlags(&reported.e, cudaEventDisableTiming));
+    ID11B_CHECK(cudaEventRecord(reported.e, st));
+    if (once) {
+        offsets(egrid);
+        ID11B_CHECK_LAUNCH();
+        rowsplit(egrid);
+        ID11B_CHECK_LAUNCH();
+    }
+    ID11B_CHECK(cudaEventSynchronize(reported.e));
     const BinInfo bi = t_report.p->info;
     const Header hh = t_report.p->header;
     const int nspecial = t_report.p->nspecial;
@@ -1649,23 +1706,18 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
                 if (cuts.size() > 2) {
                     egrid = enumerate(0, i0, mc, 0);
                     ID11B_CHECK_LAUNCH();
-                }
-                k_blk_offsets<<<grid_for((int64_t)nblk * 32, kGT), kGT, 0, st>>>(cta_blk, egrid,
-                                                                                nblk, blktot);
-                ID11B_CHECK_LAUNCH();
-                ID11B_CHECK(cudaMemsetAsync(blktot + nblk, 0, sizeof(int), st));
-                int rc = scan(blktot, nblk + 1, blkstart, tot, st);
-                if (rc) return rc;
-                const bool written = once && !bi.overflow && cuts.size() == 2;
-                if (!written) {
-                    enumerate(1, i0, mc, 0);
+                    offsets(egrid);
                     ID11B_CHECK_LAUNCH();
                 }
-                k_rowsplit<<<(unsigned)std::min(nblk, num_sms() * kRSPerSM), kRS, 0, st>>>(
-                    tmp, blkstart, nblk, nrows, written ? egrid : 0, cta_blk, room, rstart, recs);
-                ID11B_CHECK_LAUNCH();
+                if (cuts.size() > 2 || bi.overflow) {
+                    enumerate(1, i0, mc, 0);
+                    ID11B_CHECK_LAUNCH();
+                    rowsplit(0);
+                    ID11B_CHECK_LAUNCH();
+                }
             }
-            ID11B_CHECK(cudaMemsetAsync(&info->next_row, 0, sizeof(int), st));
+            if (pass > 0 || c > 0)
+                ID11B_CHECK(cudaMemsetAsync(&info->next_row, 0, sizeof(int), st));
             P.i0 = i0;
             if (ev0 && !ev0_done) {
                 ID11B_CHECK(cudaEventRecord(ev0, st));
