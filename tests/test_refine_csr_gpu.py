@@ -122,3 +122,35 @@ def test_refine_csr_more_grains_than_ctas(oracle, threads, ordered, cuda):
     _check(u[big], npk.cpu().numpy()[big], mean.cpu().numpy()[big], ref_u[big], ref_n[big],
            ref_m[big])
     assert np.array_equal(npk.cpu().numpy(), ref_n)
+
+
+@pytest.mark.parametrize("ordered", [True, False])
+def test_compensated_more_grains_than_ctas(oracle, ordered, cuda):
+    """The same for the compensated-FP32 variant, whose one-warp grains end at 384
+    peaks; grains of 20 peaks and more, with that variant's tolerances above."""
+    import torch
+    from imaged11_b200 import batch, synth
+    from imaged11_b200._lib import lib, check
+    rng = np.random.default_rng(44)
+    counts = rng.integers(20, 41, 5200)
+    counts[:9] = [0, 1, 31, 383, 384, 385, 769, 2000, 386]
+    rng.shuffle(counts)
+    gv, off, ubis = synth.grain_gvectors(counts, "Ti_hcp", rng)
+    u0 = synth.perturb_ubis(ubis, 0.2, 0.002, rng)
+    ref_u, ref_n, ref_m = oracle.refine_csr(u0, gv, off, 0.05, 3)
+    gs = batch.GrainSet(gv, off, u0)
+    u, npk, mean = gs.refine(0.05, 3, precision="f32c")
+    if not ordered:
+        other = torch.tensor(u0, device=cuda).contiguous()
+        check(lib.id11b_dev_refine_csr_f32c(other.data_ptr(), gs.gv.data_ptr(),
+                                            gs.offsets.data_ptr(), None, gs.ngrains, 0.05, 3,
+                                            gs.gmax, npk.data_ptr(), mean.data_ptr(),
+                                            gs.ws.data_ptr(), gs.ws.numel(), None), "f32c")
+        torch.cuda.synchronize()
+        assert torch.equal(other.view(-1, 3, 3), u)
+    big = counts >= 20
+    u, npk, mean = u.cpu().numpy()[big], npk.cpu().numpy()[big], mean.cpu().numpy()[big]
+    assert np.array_equal(npk, ref_n[big])
+    scale = np.abs(ref_u[big]).reshape(len(u), -1).max(1)
+    assert np.all(np.abs(u - ref_u[big]).reshape(len(u), -1).max(1) <= 1e-9 * scale)
+    assert np.all(np.abs(mean - ref_m[big]) <= 1e-4 * np.abs(ref_m[big]) + 1e-18)
