@@ -1458,7 +1458,11 @@ struct PinnedReport {
         return ID11B_OK;
     }
     ~PinnedReport() {  // at thread exit (the runtime may already be shutting down)
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return;
+        cudaFreeHost(p);
+        cudaThreadExchangeStreamCaptureMode(&mode);
     }
 };
 thread_local PinnedReport t_report;
