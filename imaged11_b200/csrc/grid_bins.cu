@@ -727,14 +727,16 @@ __device__ __forceinline__ void each_box(const uint64_t* __restrict__ tmp, int p
 __global__ void __launch_bounds__(kRS)
 k_rowsplit(const uint64_t* __restrict__ tmp, const int* __restrict__ blkstart, int nblk,
            int nrows, int nseg, const int* __restrict__ cta_blk, const int* __restrict__ room,
-           int* __restrict__ rstart, uint64_t* __restrict__ recs,
+           int* __restrict__ rstart, uint64_t* __restrict__ recs, int cap,
            const BinInfo* __restrict__ info) {
     if (nseg && info->overflow) return;  // the streams are not whole: the host counts first
     __shared__ int s_wh[kRSW][kRowBlock];
     __shared__ int s_off[kMaxEnumCtas + 1];
     const int w = threadIdx.x >> 5;
     for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
-        const int p0 = blkstart[b], p1 = blkstart[b + 1];
+        // (a range's boxes fit cap; were they more, the rest would be left out here as
+        // k_enum leaves it out)
+        const int p0 = min(blkstart[b], cap), p1 = min(blkstart[b + 1], cap);
         for (int c = threadIdx.x; c <= nseg; c += kRS)
             s_off[c] = c < nseg ? cta_blk[(int64_t)c * nblk + b] : p1 - p0;
         if (threadIdx.x < kRSW * kRowBlock) s_wh[threadIdx.x / kRowBlock][threadIdx.x % kRowBlock] = 0;
@@ -1586,15 +1588,16 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     // 2.19 -> 1.89 ms, 100,000 19.1 -> 15.3, 5,003 x 170k 0.56 -> 0.48; trials of 20
     // grains 2.48 -> 2.16; trials all of one grain, counted first, 2.57 -> 2.62.
     const bool once = m <= (int64_t(1) << kUbiBits);
-    ID11B_CHECK(cudaMemsetAsync(info, 0, parts > 1 ? B.cnt_ubi - B.info + sizeof(int) * (size_t)m
-                                                   : sizeof(BinInfo), st));
+    // (the per-UBI counts too: a UBI that is scanned plainly writes none, and the host
+    // cuts the ranges by all of them)
+    ID11B_CHECK(cudaMemsetAsync(info, 0, B.cnt_ubi - B.info + sizeof(int) * (size_t)m, st));
     auto offsets = [&](int grid) {
         k_blk_offsets<<<grid_for((int64_t)nblk * 32, kGT), kGT, 0, st>>>(cta_blk, grid, nblk, blktot,
                                                                         blkstart, info);
     };
     auto rowsplit = [&](int nseg) {
         k_rowsplit<<<(unsigned)std::min(nblk, num_sms() * kRSPerSM), kRS, 0, st>>>(
-            tmp, blkstart, nblk, nrows, nseg, cta_blk, room, rstart, recs, info);
+            tmp, blkstart, nblk, nrows, nseg, cta_blk, room, rstart, recs, (int)cap, info);
     };
     if (once) {
         const int64_t per = enum_per(m);

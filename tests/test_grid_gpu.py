@@ -241,6 +241,28 @@ def test_bins_workspace_ranges(B, oracle, scene, cuda):
         B.score_grid(u, grid, tols, method="bins", workspace=B.BinsWorkspace(len(u), grid, 10))
 
 
+def test_bins_ranges_with_plainly_scanned_ubis(B, oracle, scene, cuda):
+    """The ranges are cut by the UBIs' box counts: a UBI that is scanned plainly
+    has none, whatever the workspace held before.  8,000 UBIs are one work item
+    each; the stale counts would be above every capacity."""
+    from imaged11_b200 import synth
+    ps, _ = scene
+    u = synth.trial_ubis(ps.ubis, 8000, 0.1, 0.5, np.random.default_rng(33))
+    u[::97] = 0.0                       # singular
+    u[5::1000, 1] = u[5::1000, 0]       # two equal rows
+    u[7] = np.nan
+    grid = B.GvecGrid(ps.gv)
+    tols = [0.02, 0.1]
+    ref = oracle.score_many(u, ps.gv, tols)
+    est = B.bins_box_estimate(u, grid, 0.1)
+    for frac in (1.0, 0.4):
+        ws = B.BinsWorkspace(len(u), grid, int(est * frac))
+        ws.buf.fill_(0x7f)
+        c = B.score_grid(u, grid, tols, method="bins", workspace=ws).cpu().numpy()
+        assert np.array_equal(c, ref), frac
+    assert grid.stats()["fallback_ubis"] == 83 + 8 + 1
+
+
 def test_bins_rejects_large_tolerances(B, scene, cuda):
     ps, ubis = scene
     with pytest.raises(Exception):
