@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <utility>
 
 #include "common.cuh"
 
@@ -200,6 +201,7 @@ k_lsq_cluster(double* __restrict__ ubi, const double* __restrict__ gv, double to
     __shared__ __align__(16) double s_g[3 * kLsqTile];
     __shared__ double s_warp[kThreads / 32][17], s_cta[8][17], s_m[27];
     cg::cluster_group cl = cg::this_cluster();
+    auto started = cl.barrier_arrive();  // this CTA runs: its shared memory may be written
     const int rank = (int)cl.block_rank(), nblk = (int)cl.num_blocks();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     // an even share, so that every share starts 16-byte aligned when gv does
@@ -279,6 +281,7 @@ k_lsq_cluster(double* __restrict__ ubi, const double* __restrict__ gv, double to
     const double part = ScatterSum<17, 16>::run(acc, lane);
     if (field >= 0) s_warp[w][field] = part;
     __syncthreads();
+    cl.barrier_wait(std::move(started));  // every CTA runs (met behind the loads)
     if (w == 0 && lane < 17) {
         double t = 0.;
         for (int q = 0; q < kThreads / 32; q++) t += s_warp[q][lane];
