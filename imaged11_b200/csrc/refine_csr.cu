@@ -248,17 +248,31 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 // warps takes grains by itself, so that the rounds' fixed part (the reduction
 // and the 3x3 solves, which one warp does) of several grains overlap.  A larger
 // grain met after that (an order that is not by size) is done by one warp as the
-// CTA would, so a grain's result depends on its size alone.
+// CTA would.  So the order of a grain's sums, and with it the last bits of its UBI,
+// follows from its size, from NT and, for grains of up to kSolo peaks, from whether
+// the call has more grains than CTAs; never from the order of the grains or of the
+// CTAs.  (One order for both, kept here, would cost more than it gives: the CTA's by
+// one warp 2,000 grains of 20 .. 2,000 peaks 39 -> 49 us, one warp's where there are
+// few grains 500 of 20 .. 768 peaks 16.4 -> 22.6 us.)
 //
 // Bound: instruction issue and FP64 latency at 16 resident warps (123
 // registers), then the largest grains' own five rounds.  2,000 grains of 20 ..
 // 2,000 peaks (859k), five rounds: 36.6 us with 128 threads, 42 with 64; 55.9 (64)
 // and 80.2 (128) with a CTA for every grain, 17 warp sums and five barriers a
 // round.  500 such grains 36.0 -> 17.0, 8,000 of up to 400 peaks, three rounds, 86
-// -> 35 us.  kSolo at 128 threads: 256 43.0, 512 43.2, 768 36.6, 1,024 41.9 us.
-// The F32C variant does more per peak, so fewer go to one warp: the first of these 84
-// -> 69 us at 128 threads and 384 (768: 74; 64 threads: 91), 200 grains of 500 ..
-// 4,000 peaks 94 -> 46 (64 threads: 77).
+// -> 35 us.
+//
+// kSolo of 256, 512, 768 and 1,024 at 128 threads, five rounds, us (the launch among
+// others): 1,000 grains of 20 .. 2,000 peaks 30.3, 30.6, 30.3, 30.6; 2,000 of up to
+// 1,000 37.4, 33.4, 34.8, 37.1 and of up to 2,000 45.9, 45.0, 39.1, 43.2; 4,000 of up
+// to 1,000 57.3, 53.0, 50.2, 54.0; 8,000 of up to 2,000 119, 110, 106, 109; 3,000 of
+// 600 .. 760 75.2, 75.0, 78.1, 78.1 and of 780 .. 1,000 84.1, 84.0, 84.1, 94.1.  768
+// is the best or within 4% of it on all of them.
+// The F32C variant does more per peak, so fewer go to one warp.  192, 256, 384, 512,
+// 768: 1,000 of up to 2,000 peaks 49.0, 51.1, 56.0, 56.1, 54.7; 2,000 74.6, 74.1,
+// 71.4, 76.7, 74.8; 8,000 of up to 400, three rounds, 75.9, 67.5, 57.7, 57.4, 57.4;
+// 8,000 of up to 2,000 225, 219, 211, 204, 200; with a CTA of 64 threads for every
+// grain the second took 84.
 constexpr int kSoloFp64 = 768, kSoloF32c = 384;
 
 template <int NT, bool F32C = false>

@@ -386,7 +386,11 @@ int id11b_dev_refine_batch(double *ubis, int64_t m, const double *gv, const floa
  * npk / mean_drlv2 (optional, ngrains) receive the last round's count and mean
  * drlv2.  threads: CTA size 32, 64, 128, 256 or 512 (0 = 128, the fastest for
  * 2,000 grains of 20..2,000 peaks); with more grains than resident CTAs, grains
- * of up to 768 peaks are refined by one warp each.  Exact FP64 per pair; the
+ * of up to 768 peaks are refined by one warp each.  Counts are the same either
+ * way; a UBI's last bits follow from the order of its sums, that is from the
+ * grain's size, from threads and, for those grains, from whether the launch has
+ * more grains than resident CTAs (so a grain refined alone and among thousands
+ * can differ there; with threads = 32 it does not).  Exact FP64 per pair; the
  * persistent launch (counter reset + kernel) can be captured in a CUDA graph and
  * replayed. */
 int64_t id11b_refine_csr_workspace_bytes(void);
@@ -395,7 +399,8 @@ int id11b_dev_refine_csr(double *ubis, const double *gv, const int64_t *offsets,
                          int persistent, int threads, int32_t *npk, double *mean_drlv2,
                          void *workspace, int64_t ws_bytes, void *stream);
 
-/* Per-grain refinement as id11b_dev_refine_csr (persistent, 64-thread CTAs)
+/* Per-grain refinement as id11b_dev_refine_csr (persistent, 128-thread CTAs;
+ * one warp for grains of up to 384 peaks where there are more grains than CTAs)
  * with FP32 screening -- the proven error band of id11b_dev_score_batch, FP64
  * inside it -- and compensated FP32 normal-equation sums (error-free products
  * and TwoSum; H as exact integers), FP64 3x3 solves.  The same accepted pairs

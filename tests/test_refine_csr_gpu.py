@@ -124,6 +124,29 @@ def test_refine_csr_more_grains_than_ctas(oracle, threads, ordered, cuda):
     assert np.array_equal(npk.cpu().numpy(), ref_n)
 
 
+@pytest.mark.parametrize("threads", [32, 128])
+def test_refine_csr_grain_alone_and_among_many(threads, cuda):
+    """The same grains in a call of 16 and among 5,200: the same peaks, and the same
+    bits where the sums' order is the same -- with 32 threads always, with more for
+    the grains that a whole CTA refines in both (above 768 peaks).  The others
+    differ by the order of their sums."""
+    from imaged11_b200 import batch, synth
+    rng = np.random.default_rng(45)
+    counts = rng.integers(20, 41, 5200)
+    counts[:16] = [20, 31, 32, 33, 64, 127, 128, 129, 500, 767, 768, 769, 800, 1537, 2000, 2600]
+    gv, off, ubis = synth.grain_gvectors(counts, "Ti_hcp", rng)
+    u0 = synth.perturb_ubis(ubis, 0.2, 0.002, rng)
+    many = [t.cpu().numpy()[:16] for t in batch.GrainSet(gv, off, u0, threads=threads).refine(0.05, 3)]
+    few = [t.cpu().numpy() for t in
+           batch.GrainSet(gv[:off[16]], off[:17], u0[:16], threads=threads).refine(0.05, 3)]
+    assert np.array_equal(many[1], few[1])
+    same = (counts[:16] > 768) | (threads == 32)
+    assert np.array_equal(many[0][same], few[0][same])
+    assert np.array_equal(many[2][same], few[2][same])
+    scale = np.abs(few[0]).reshape(16, -1).max(1)
+    assert np.all(np.abs(many[0] - few[0]).reshape(16, -1).max(1) <= UBI_RTOL * scale)
+
+
 @pytest.mark.parametrize("ordered", [True, False])
 def test_compensated_more_grains_than_ctas(oracle, ordered, cuda):
     """The same for the compensated-FP32 variant, whose one-warp grains end at 384
