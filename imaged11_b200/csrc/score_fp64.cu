@@ -542,11 +542,11 @@ extern "C" int id11b_dev_score_many_fp64(const double* ubis, int64_t m, const do
 // array (kLsqMaxBlocks x 136 bytes = 136 KiB, held by every GPU that loads the
 // library until the process exits) instead of caller- or pool-provided memory.
 //
-// CUDA loads modules lazily (the default since CUDA 12.2): the module holding
-// this array and the kernels below is loaded, and its memory taken, on the
-// first call in each context.  A caller that reserves memory or caps a pool
-// afterwards makes one warm-up call per device first (one g-vector is enough;
-// it launches both kernels).
+// CUDA loads modules and kernels lazily (the default since CUDA 12.2): the module
+// holding this array and the kernels of every size of call are loaded, and their
+// memory taken, on the first call in each context.  A caller that reserves memory
+// or caps a pool afterwards makes one warm-up call per device first; one g-vector
+// is enough.
 //
 // Every call on a device shares the array.  Each partial-sum CTA writes its own
 // slot before the finishing CTA reads it, so the previous call's contents never
@@ -612,6 +612,14 @@ int lsq_scratch_address(void** out) {
     // device's primary context current first
     cudaError_t e = cudaGetSymbolAddress(&p, g_lsq_scratch);
     if (e != cudaSuccess) return id11b_record_cuda(e);
+    // the kernels lsq_launch chooses from: asking for a kernel's attributes loads it
+    const void* const kernels[] = {(const void*)k_lsq_cluster<0>, (const void*)k_lsq_partials<0>,
+                                   (const void*)k_lsq_finish};
+    for (const void* k : kernels) {
+        cudaFuncAttributes a;
+        e = cudaFuncGetAttributes(&a, k);
+        if (e != cudaSuccess) return id11b_record_cuda(e);
+    }
     if (!ctx) {
         if (g_ctx_get_current(&ctx) != CUDA_SUCCESS || !ctx) return ID11B_ERR_CUDA;
         if (g_ctx_get_id(ctx, &id) != CUDA_SUCCESS) return ID11B_ERR_CUDA;

@@ -79,6 +79,36 @@ def test_noalloc_rejects_sizes_beyond_maximum(cuda):
     assert lib.id11b_dev_score_and_refine_noalloc(8, 8, 0.1, -1, 8, 8, None) == 1
 
 
+def test_noalloc_one_peak_warms_every_size(cuda):
+    """In a process of its own: after one call with a single g-vector, the first
+    call that takes the other kernels (above 16,384 peaks) leaves the free memory
+    unchanged."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from imaged11_b200._lib import lib
+g = torch.ones((20000, 3), dtype=torch.float64, device='cuda')
+u = torch.eye(3, dtype=torch.float64, device='cuda')
+n = torch.zeros(1, dtype=torch.int32, device='cuda')
+m = torch.zeros(1, dtype=torch.float64, device='cuda')
+s = torch.cuda.current_stream().cuda_stream
+free = []
+for k in (1, 16385, 20000, 0):
+    assert lib.id11b_dev_score_and_refine_noalloc(u.data_ptr(), g.data_ptr(), 0.05, k,
+                                                  n.data_ptr(), m.data_ptr(), s) == 0
+    torch.cuda.synchronize()
+    assert int(n.item()) == k
+    free.append(torch.cuda.mem_get_info()[0])
+assert len(set(free)) == 1, free
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
+                         timeout=300)
+    assert run.returncode == 0, run.stderr
+
+
 def test_noalloc_warmed_call_takes_no_device_memory(golden, cuda):
     """After one warm-up call (which loads the library's module lazily), a call
     leaves the device's free memory unchanged: the entry point allocates nothing."""
