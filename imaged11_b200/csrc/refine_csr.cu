@@ -179,20 +179,25 @@ __device__ __forceinline__ void refine_peaks_f32c(const double u[9],
     }
     // to FP64 for the fixed reduction: s + c, exact integers
 #pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] = (double)rs[e] + (double)rc[e];
+    for (int e = 0; e < 9; e++) acc[e] += (double)rs[e] + (double)rc[e];
 #pragma unroll
-    for (int e = 0; e < 6; e++) acc[9 + e] = (double)hint[e];
-    acc[15] = (double)ss32 + (double)sc32;
+    for (int e = 0; e < 6; e++) acc[9 + e] += (double)hint[e];
+    acc[15] += (double)ss32 + (double)sc32;
 }
+
+// Peaks passed over with 32-bit counters at a time: a multiple of what N threads take
+// a step, so that the peaks of a longer grain go to the threads they would go to.
+constexpr int kSpan = 1 << 30;
 
 // `iters` rounds of one grain by N threads (tid of them; N == 32: one warp of the
 // CTA by itself).  red: N / 32 rows of per-warp partial sums.  V > 1 (N == 32):
 // the warp does the work of V warps in turn, peak by peak and sum by sum as they
-// would, so the result has the same bits.
-template <int N, bool F32C, int V = 1>
+// would, so the result has the same bits.  Len: 64 bits for a grain that may be
+// longer than kSpan, else int (64 bits for all: 2 to 6% slower for a few grains).
+template <int N, bool F32C, int V = 1, class Len>
 __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], int tid, int g,
                                              double* __restrict__ ubis,
-                                             const double* __restrict__ gv, int64_t k0, int n,
+                                             const double* __restrict__ gv, int64_t k0, Len n,
                                              double tolsq, int iters, int* __restrict__ npk,
                                              double* __restrict__ mean, double gmax) {
     const int lane = tid & 31, w = tid >> 5;
@@ -214,10 +219,18 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 #pragma unroll
             for (int f = 0; f < 17; f++) acc[f] = 0.;
             int nacc = 0;
-            if (F32C)
-                refine_peaks_f32c<N * V>(u, gv + 3 * (k0 + first), first, n, tolsq, gmax, acc, nacc);
-            else
-                refine_peaks<N * V>(u, gv + 3 * (k0 + first), first, n, tolsq, acc, nacc);
+            auto span = [&](Len c) {
+                const double* p = gv + 3 * (k0 + c + first);
+                const int cn = (int)min(n - c, (Len)kSpan);
+                if (F32C)
+                    refine_peaks_f32c<N * V>(u, p, first, cn, tolsq, gmax, acc, nacc);
+                else
+                    refine_peaks<N * V>(u, p, first, cn, tolsq, acc, nacc);
+            };
+            Len c = 0;
+            do {
+                span(c);
+            } while (sizeof(Len) > 4 && (c += kSpan) < n);
             acc[16] = (double)nacc;
             part += ScatterSum<17, 16>::run(acc, lane);
         }
@@ -290,11 +303,15 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     while (slot < ngrains) {
         const int g = order ? order[slot] : slot;
         const int64_t k0 = off[g];
-        const int n = (int)(off[g + 1] - k0);
+        const int64_t n = max(off[g + 1] - k0, (int64_t)0);
         if (NT > 32 && queue && ngrains > (int)gridDim.x && n <= kSolo) break;
         if (tid == 0) s_next = queue ? (int)gridDim.x + atomicAdd(queue, 1) : ngrains;
-        refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
-                               gmax);
+        if (n <= kSpan)
+            refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, (int)n, tolsq, iters, npk,
+                                   mean, gmax);
+        else
+            refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
+                                   gmax);
         slot = s_next;
         if (NT == 32) __syncwarp(); else __syncthreads();
     }
@@ -311,12 +328,12 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     while (mine < ngrains) {
         const int g = order ? order[mine] : mine;
         const int64_t k0 = off[g];
-        const int n = (int)(off[g + 1] - k0);
+        const int64_t n = max(off[g + 1] - k0, (int64_t)0);
         int next = 0;
         if (lane == 0) next = (int)gridDim.x + atomicAdd(queue, 1);
         if (n <= kSolo)
-            refine_grain<32, F32C>(sm[w], s_red + w, lane, g, ubis, gv, k0, n, tolsq, iters, npk,
-                                   mean, gmax);
+            refine_grain<32, F32C>(sm[w], s_red + w, lane, g, ubis, gv, k0, (int)n, tolsq, iters,
+                                   npk, mean, gmax);
         else
             refine_grain<32, F32C, NT / 32>(sm[w], s_red + w, lane, g, ubis, gv, k0, n, tolsq,
                                             iters, npk, mean, gmax);

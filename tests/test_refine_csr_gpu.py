@@ -177,3 +177,24 @@ def test_compensated_more_grains_than_ctas(oracle, ordered, cuda):
     scale = np.abs(ref_u[big]).reshape(len(u), -1).max(1)
     assert np.all(np.abs(u - ref_u[big]).reshape(len(u), -1).max(1) <= 1e-9 * scale)
     assert np.all(np.abs(mean - ref_m[big]) <= 1e-4 * np.abs(ref_m[big]) + 1e-18)
+
+
+def test_refine_csr_grain_longer_than_2_31(oracle, cuda):
+    """One grain of 2^31 + 300 peaks (its length, and a peak's index in it, need 64
+    bits): its peaks are at the start, around 2^30 and 2^31 and at the end, NaN
+    between them."""
+    import torch
+    from imaged11_b200 import batch, synth
+    n = (1 << 31) + 300
+    if torch.cuda.mem_get_info(cuda)[0] < 3 * 8 * n + (4 << 30):
+        pytest.skip("51.5 GB of g")
+    rng = np.random.default_rng(46)
+    gv, off, ubis = synth.grain_gvectors(np.array([900]), "Ti_hcp", rng)
+    u0 = synth.perturb_ubis(ubis, 0.2, 0.002, rng)
+    where = np.concatenate([np.arange(100), (1 << 30) - 250 + np.arange(500),
+                            (1 << 31) - 150 + np.arange(250), n - 50 + np.arange(50)])
+    g = torch.full((n, 3), float("nan"), dtype=torch.float64, device=cuda)
+    g[torch.as_tensor(where, device=cuda)] = torch.as_tensor(gv, device=cuda)
+    u, npk, mean = batch.GrainSet(g, np.array([0, n]), u0, threads=512).refine(0.05, 2)
+    ref_u, ref_n, ref_m = oracle.refine_csr(u0, gv, off, 0.05, 2)
+    _check(u.cpu().numpy(), npk.cpu().numpy(), mean.cpu().numpy(), ref_u, ref_n, ref_m)
