@@ -209,13 +209,13 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
     if (gi >= ngrains) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int64_t p0 = offsets[gi];
-    const int np = (int)(offsets[gi + 1] - p0);
+    const int64_t np = offsets[gi + 1] - p0;
     double* const keep = s_keep + tid;
     constexpr int kF = kKeep * kTT;  // doubles per field
-    auto angles = [&](int k, PeakG& q) {
+    auto angles = [&](int64_t k, PeakG& q) {
         sincos(kRad * omega[p0 + k] * P.omegasign, &q.so, &q.co);
     };
-    for (int i = 0, k = tid; k < np && i < kKeep; i++, k += kTT) {
+    for (int64_t i = 0, k = tid; k < np && i < kKeep; i++, k += kTT) {
         PeakG q;
         angles(k, q);
         keep[i * kTT] = q.so;
@@ -243,7 +243,7 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         double a[15];
 #pragma unroll
         for (int q = 0; q < 15; q++) a[q] = 0.;
-        for (int i = 0, k = tid; k < np; i++, k += kTT) {
+        for (int64_t i = 0, k = tid; k < np; i++, k += kTT) {
             const double* x = xyz + 3 * (p0 + k);
             PeakG q;
             if (i < kKeep) {
@@ -277,7 +277,7 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         Acc acc;
 #pragma unroll
         for (int q = 0; q < 11; q++) acc.a[q] = 0.;
-        for (int i = 0, k = tid; k < np; i++, k += kTT) {
+        for (int64_t i = 0, k = tid; k < np; i++, k += kTT) {
             PeakG q;
             const double* x = xyz + 3 * (p0 + k);
             if (i < kKeep) {
