@@ -149,7 +149,7 @@ __device__ void make_geom(const double* p, const double sc[10], const AdjDet& D,
     P.t[0] = p[9];
     P.t[1] = p[10];
     P.t[2] = p[11];
-    P.wavelength = p[6];
+    P.wavelength = isinf(p[6]) ? 0. : p[6];  // (div_by's remainder; the quotient is 0)
     P.inv_wavelength = 1.0 / p[6];
     P.distance = p[0];
     P.y_center = p[1];
@@ -175,7 +175,8 @@ __device__ __forceinline__ void peak_sincos(const AdjGeom& P, const double* __re
 }
 
 // a / y given ry = 1 / y rounded: the quotient's remainder corrects the product
-// (three operations; the rounding is that of a division but for rare last bits)
+// (Markstein's division; three operations, the rounding is that of a division but
+// for rare last bits).  An infinite y is passed as 0: its remainder would be NaN.
 __device__ __forceinline__ double div_by(double a, double y, double ry) {
     const double q = a * ry;
     return fma(fma(-q, y, a), ry, q);

@@ -53,6 +53,22 @@ def test_loss_and_gradient_match_reference(golden, cuda):
         assert abs(gu[G, i, j] - ref) <= GRAD_RTOL * abs(ref) + 1e-9
 
 
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_infinite_wavelength(golden, sign, cuda):
+    """g is k / wavelength: zero, so the residuals are -hkl and no gradient is left."""
+    import torch
+    from imaged11_b200 import adjoint
+    d = golden["adjoint"]
+    peaks = _peaks(d)
+    params = torch.tensor(d["adj_params"], dtype=torch.float64, device=cuda)
+    params[adjoint.PARAMS.index("wavelength")] = sign * float("inf")
+    ubis = torch.tensor(d["adj_ubis"], dtype=torch.float64, device=cuda)
+    assert torch.equal(adjoint.residuals(params, ubis, peaks), -peaks.hkl)
+    assert not adjoint.gvectors(params, peaks).any()
+    L, gp, gu = _grad(params, ubis, peaks)
+    assert L == 0.5 * float((peaks.hkl ** 2).sum()) and not gp.any() and not gu.any()
+
+
 def test_gradient_matches_own_central_differences(golden, cuda):
     import torch
     from imaged11_b200 import adjoint
