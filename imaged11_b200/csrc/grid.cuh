@@ -399,7 +399,6 @@ struct BoxWalk {
 int num_sms();
 unsigned grid_for(int64_t items, int per);
 int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st);
-int score_parts(int64_t m);
 Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells);
 bool grid_dims_ok(int32_t nx, int32_t xsub);
 

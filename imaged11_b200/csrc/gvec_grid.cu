@@ -1116,24 +1116,42 @@ int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st) {
                      ScanJob{nullptr, 0, nullptr, nullptr, 0}, st);
 }
 
-// work items (warps) per UBI: about two waves of the resident warps, and two
-// items where there are fewer than about four waves of UBIs.  More items
-// balance better but each sets up the UBI's plan and reduces its sums: 2,000
-// UBIs x 1.1M g refine in 0.39 ms a round at two waves and 0.42 at four, 1,000
-// score in 0.25 and 0.30 ms; 20,000 score in 6.4 ms with one item each, 6.1
-// with two.  A refinement's item also reduces its 17 sums, so it takes the
-// second item only for a second slab of an index past 96 MB: 20,000 UBIs refine
-// in 1.78 ms with one and 2.17 with two over 1.1M g, 13.3 and 11.5 ms over 10.2M.
-static int item_parts(int64_t m, int64_t floor) {
+// Work items (warps) per UBI: enough for twice `warps` of them per SM, at least
+// `floor`.  More items balance better, but each sets up the UBI's plan and reduces
+// its sums.
+static int item_parts(int64_t m, int64_t floor, int warps) {
     if (m <= 0) return 1;
-    int64_t p = std::max((2 * (int64_t)num_sms() * 64 + m - 1) / m, floor);
-    return (int)std::min<int64_t>(p, kMaxParts);
+    int64_t p = std::max((2 * (int64_t)num_sms() * warps + m - 1) / m, floor);
+    return (int)std::min(std::min<int64_t>(p, kMaxParts), INT32_MAX / m);  // one block each
 }
 
-int score_parts(int64_t m) { return item_parts(m, m < 4 * (int64_t)num_sms() * 64 ? 2 : 1); }
+static bool few_ubis(int64_t m) { return m < 4 * (int64_t)num_sms() * 64; }
 
+static int64_t index_bytes(int64_t n, int64_t ncells) { return 20 * n + 4 * ncells; }
+
+// An index from which on a second slab (split_for) pays for every UBI's second item,
+// however many UBIs there are.  One against two items, us: 20,000 UBIs refined over
+// indexes of 34, 45, 53, 58, 59, 73 and 105 MB 2215, 2323, 2773, 3064, 3396, 4201, 6969
+// against 2561, 2654, 2835, 3000, 3136, 3607, 5614; 60,000 scored over 13 MB (40,000 of
+// them), 59, 70, 82, 105 and 233 MB 3289, 7152, 8867, 11905, 17257, 31497 against 3332,
+// 6901, 7882, 10329, 14913, 29055.
+constexpr int64_t kTwoSlabs = 56 << 20;
+
+// Scoring: 32 warps an SM (24 are resident).  64, 32 and 24, us: 300 UBIs x 11k, 112k
+// and 1.1M g 107, 123, 156; 80, 96, 129; 70, 86, 117 -- 1,000 110, 164, 223; 91, 139, 198;
+// 91, 139, 211 -- 3,000 175, 321, 483; 178, 313, 494; 189, 313, 484.  Where there are few
+// waves of UBIs two items each: 20,000 x 1.1M at three tolerances 5649 us, 5719 as one.
+static int score_parts(int64_t m, int64_t n, int64_t ncells) {
+    const bool two = few_ubis(m) || index_bytes(n, ncells) > kTwoSlabs;
+    return item_parts(m, two ? 2 : 1, 32);
+}
+
+// Assignment, and what a caller's workspace has to hold.
+static int least_parts(int64_t m) { return item_parts(m, few_ubis(m) ? 2 : 1, 64); }
+
+// Refinement: an item also reduces 17 sums, so the second is taken only for a slab.
 static int refine_parts(int64_t m, int64_t n, int64_t ncells) {
-    return 20 * n + 4 * ncells > (96 << 20) ? score_parts(m) : item_parts(m, 1);
+    return item_parts(m, index_bytes(n, ncells) > kTwoSlabs ? 2 : 1, 64);
 }
 
 // `parts` work items per UBI as slabs x columns: as many slabs as it takes for a
@@ -1144,8 +1162,7 @@ static int refine_parts(int64_t m, int64_t n, int64_t ncells) {
 // 1.1M-g index (52 MB) is two slabs where there are parts to split: 20,000 UBIs
 // score in 6.1 ms, in 6.4 as one.
 Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells) {
-    const double bytes = 20. * (double)n + 4. * (double)ncells;
-    int slabs = (int)fmin(16., ceil(bytes / (32. * 1048576.)));
+    int slabs = (int)std::min<int64_t>(16, (index_bytes(n, ncells) + (32 << 20) - 1) >> 25);
     if (slabs < 1) slabs = 1;
     if (!more && slabs > parts) slabs = parts;
     while (slabs > 1 && m > INT32_MAX / (2 * (int64_t)slabs)) slabs--;  // one block per item
@@ -1246,11 +1263,16 @@ extern "C" int id11b_dev_build_grid(const double* gv, int64_t n, float gmax, flo
 
 // partials: (m * parts + m) x ntol ints, then the same doubles (the last m x
 // ntol of each: the g outside the regular range)
+static int64_t score_bytes(int64_t m, int ntol, int parts) {
+    const int64_t mm = m > 0 ? m : 1;
+    const int64_t items = (mm * parts + mm) * ntol;
+    return (int64_t)(al256(sizeof(int) * (size_t)items) + al256(sizeof(double) * (size_t)items));
+}
+
+// room for two items per UBI; a call takes one where the workspace has no more
 extern "C" int64_t id11b_grid_score_workspace_bytes(int64_t m, int ntol) {
     if (m < 0 || ntol < 1 || ntol > ID11B_MAX_TOLS) return -1;
-    const int64_t mm = m > 0 ? m : 1;
-    const int64_t items = (mm * score_parts(m) + mm) * ntol;
-    return (int64_t)(al256(sizeof(int) * (size_t)items) + al256(sizeof(double) * (size_t)items));
+    return score_bytes(m, ntol, std::max(least_parts(m), 2));
 }
 
 extern "C" int id11b_dev_score_grid(const double* ubis, int64_t m, const double* gv, int64_t n,
@@ -1267,21 +1289,23 @@ extern "C" int id11b_dev_score_grid(const double* ubis, int64_t m, const double*
     for (int j = 0; j < ntol; j++)
         if (!(tols_host[j] >= 0.) || !(tols_host[j] < 1e3)) return ID11B_ERR_ARG;
     if (((uintptr_t)gridbuf & 255) || ((uintptr_t)ws & 255)) return ID11B_ERR_ALIGN;
-    if (ws_bytes < id11b_grid_score_workspace_bytes(m, ntol)) return ID11B_ERR_SIZE;
+    if (ws_bytes < score_bytes(m, ntol, least_parts(m))) return ID11B_ERR_SIZE;
     if (m > INT32_MAX) return ID11B_ERR_SIZE;
     cudaStream_t st = (cudaStream_t)stream;
-    const Layout L = layout(n, (int64_t)nx * nx * nx * xsub);
+    const int64_t ncells = (int64_t)nx * nx * nx * xsub;
+    const Layout L = layout(n, ncells);
     char* b = (char*)gridbuf;
     Header* H = (Header*)b;
     ID11B_CHECK(cudaMemsetAsync(&H->nfallback, 0, 3 * sizeof(unsigned long long), st));
     if (m == 0) return ID11B_OK;
-    const int parts = score_parts(m);
+    int parts = score_parts(m, n, ncells);
+    if (score_bytes(m, ntol, parts) > ws_bytes) parts = 1;
     const int64_t items = (m * parts + m) * ntol;
     int* pcnt = (int*)ws;
     double* psum = (double*)((char*)ws + al256(sizeof(int) * (size_t)items));
     int* scnt = pcnt + m * parts * ntol;
     double* ssum = psum + m * parts * ntol;
-    const Split sp = split_for(parts, false, m, n, (int64_t)nx * nx * nx * xsub);
+    const Split sp = split_for(parts, false, m, n, ncells);
     const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     const int* start = (const int*)(b + L.start);
     const double* gs = (const double*)(b + L.g);
@@ -1359,7 +1383,7 @@ extern "C" int id11b_dev_score_and_assign_grid(const double* ubis, int64_t m,
     k_assign_entries<<<grid_for(n, kGT), kGT, 0, st>>>(start, ncells, gidx, tol, drlv2, entry,
                                                        limit);
     ID11B_CHECK_LAUNCH();
-    const Split sp = split_for(score_parts(m), true, m, n, ncells);
+    const Split sp = split_for(least_parts(m), true, m, n, ncells);
     k_assign_once<<<(unsigned)((m * sp.parts() + kSW - 1) / kSW), kST, 0, st>>>(
         ubis, m, sp, H, start, (const double*)(b + L.g), (const float4*)(b + L.g4), tol, entry,
         limit);
@@ -1374,11 +1398,14 @@ extern "C" int id11b_dev_score_and_assign_grid(const double* ubis, int64_t m,
     return ID11B_OK;
 }
 
-// partials: 17 doubles per work item
+// partials: 17 doubles per work item (the same two sizes as scoring)
+static int64_t refine_bytes(int64_t m, int parts) {
+    return (int64_t)al256(sizeof(double) * kLsqF * (size_t)(m > 0 ? m : 1) * parts);
+}
+
 extern "C" int64_t id11b_grid_refine_workspace_bytes(int64_t m) {
     if (m < 0) return -1;
-    const size_t mm = (size_t)(m > 0 ? m : 1);
-    return (int64_t)al256(sizeof(double) * kLsqF * mm * score_parts(m));
+    return refine_bytes(m, std::max(least_parts(m), 2));
 }
 
 extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, int64_t n,
@@ -1389,7 +1416,7 @@ extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, 
         (m > 0 && !ubis) || (n > 0 && !gv) || !(tol >= 0.) || !(tol < 1e3))
         return ID11B_ERR_ARG;
     if (((uintptr_t)gridbuf & 255) || ((uintptr_t)ws & 255)) return ID11B_ERR_ALIGN;
-    if (ws_bytes < id11b_grid_refine_workspace_bytes(m)) return ID11B_ERR_SIZE;
+    if (ws_bytes < refine_bytes(m, least_parts(m))) return ID11B_ERR_SIZE;
     if (m > INT32_MAX) return ID11B_ERR_SIZE;
     cudaStream_t st = (cudaStream_t)stream;
     if (m == 0) return ID11B_OK;
@@ -1397,7 +1424,8 @@ extern "C" int id11b_dev_refine_grid(double* ubis, int64_t m, const double* gv, 
     const char* b = (const char*)gridbuf;
     const Header* H = (const Header*)b;
     const int64_t ncells = (int64_t)nx * nx * nx * xsub;
-    const int parts = refine_parts(m, n, ncells);
+    int parts = refine_parts(m, n, ncells);
+    if (refine_bytes(m, parts) > ws_bytes) parts = 1;
     const Split sp = split_for(parts, false, m, n, ncells);
     const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     double* part = (double*)ws;
@@ -1439,7 +1467,7 @@ extern "C" int id11b_dev_assign_grid_pass(const double* ubis, int64_t m, int64_t
     if (m == 0) return ID11B_OK;
     const Layout L = layout(n, (int64_t)nx * nx * nx * xsub);
     const char* b = (const char*)gridbuf;
-    const Split sp = split_for(score_parts(m), true, m, n, (int64_t)nx * nx * nx * xsub);
+    const Split sp = split_for(least_parts(m), true, m, n, (int64_t)nx * nx * nx * xsub);
     const unsigned blocks = (unsigned)((m * sp.parts() + kSW - 1) / kSW);
     if (pass == 0)
         k_assign<0><<<blocks, kST, 0, st>>>(ubis, m, sp, (const Header*)b,

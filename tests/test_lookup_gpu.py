@@ -49,6 +49,53 @@ def test_rows_and_slabs(scene, oracle, cell, xsub, n, tol, cuda):
         assert np.abs(ur[i] - x).max() <= 1e-11 * np.abs(x).max()
 
 
+@pytest.mark.parametrize("two", [True, False])
+def test_second_slab_with_many_ubis(scene, oracle, two, cuda):
+    """An index past the size from which every UBI gets a second item, 38,000 UBIs:
+    with the workspace the size functions give, and with one that holds one item
+    each (the least a call takes)."""
+    import torch
+    from imaged11_b200 import batch, synth
+    from imaged11_b200._lib import lib
+    g = scene[0][:700]
+    grid = batch.GvecGrid(g, cell=0.0115, xsub=4)
+    assert 20 * grid.n + 4 * grid.nx ** 3 * grid.xsub > 60 << 20
+    m = 38000
+    u = np.repeat(scene[1], m // 60 + 1, 0)[:m] * np.linspace(0.9, 1.1, m)[:, None, None]
+    tols = np.array([0.1, 0.3])
+    ub = torch.as_tensor(u, device=cuda).reshape(-1, 9).contiguous()
+    cnt = torch.zeros((m, 2), dtype=torch.int32, device=cuda)
+    al = lambda b: (b + 255) // 256 * 256
+    ws = lib.id11b_grid_score_workspace_bytes(m, 2) if two else al(16 * m) + al(32 * m)
+    buf = torch.empty(ws, dtype=torch.uint8, device=cuda)
+    args = (ub.data_ptr(), m, grid.gv.data_ptr(), grid.n, grid.nx, grid.xsub, grid.buf.data_ptr())
+
+    def score(size):
+        return lib.id11b_dev_score_grid(*args, tols.ctypes.data, 2, cnt.data_ptr(), None,
+                                        buf.data_ptr(), size, None)
+    assert score(al(16 * m) + al(32 * m) - 256) == 4     # ID11B_ERR_SIZE
+    assert score(ws) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(cnt.cpu().numpy(), oracle.score_many(u, g, tols))
+    npk = torch.zeros(m, dtype=torch.int32, device=cuda)
+    mean = torch.zeros(m, dtype=torch.float64, device=cuda)
+    ws = lib.id11b_grid_refine_workspace_bytes(m) if two else al(136 * m)
+    buf = torch.empty(ws, dtype=torch.uint8, device=cuda)
+
+    def refine(size):
+        return lib.id11b_dev_refine_grid(*args, 0.1, 1, npk.data_ptr(), mean.data_ptr(),
+                                         buf.data_ptr(), size, None)
+    assert refine(al(136 * m) - 256) == 4
+    assert refine(ws) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(npk.cpu().numpy(), oracle.score_many(u, g, [0.1])[:, 0])
+    ur = ub.cpu().numpy().reshape(-1, 3, 3)
+    for i in range(0, m, 997):
+        k, mn, x = oracle.score_and_refine(u[i], g, 0.1)
+        assert npk[i] == k and abs(float(mean[i]) - mn) <= 1e-12 * mn
+        assert np.abs(ur[i] - x).max() <= 1e-11 * np.abs(x).max()
+
+
 def test_assignment_starting_values(scene, oracle, cuda):
     """drlv2 on entry: NaN, infinities, zeros of both signs, negative, above
     tol^2, and exactly a grain's drlv2 (not below it: the label stays)."""
