@@ -68,6 +68,26 @@ def test_ctransform_methods_match_drop_in(cuda):
         ct.sf2geometry(sc, fc[:10], om)
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 255, 256, 257, 700])
+def test_positions_off_16_bytes(n, cuda):
+    """Positions and omega that are 8 bytes off a 16-byte boundary (a slice of a larger
+    table) take another kernel: the same bits, nothing read past the end."""
+    import torch
+    from imaged11_b200._lib import lib, check
+    rng = np.random.default_rng(74)
+    xyz = torch.tensor(rng.uniform(-1e5, 1e5, 3 * n + 1), device=cuda)
+    om = torch.tensor(rng.uniform(0, 360, n + 1), device=cuda)
+    t = np.array([5.0, -3.0, 2.0])
+    out = torch.full((2, 6 * n + 1), -7.0, dtype=torch.float64, device=cuda)
+    for row, x, w in ((0, xyz[1:], om[1:]), (1, xyz[1:].clone(), om[1:].clone())):
+        assert (x.data_ptr() % 16, w.data_ptr() % 16) == ((8, 8) if row == 0 else (0, 0))
+        check(lib.id11b_dev_compute_geometry(x.data_ptr(), w.data_ptr(), -1.0, 0.28, 0.01, 0.02,
+                                             t.ctypes.data, out[row].data_ptr(), n, None),
+              "compute_geometry")
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1]) and bool((out[:, -1] == -7.0).all())
+
+
 @pytest.mark.parametrize("kind", ["nodes", "tiny", "special"])
 def test_angles(kind, cuda):
     """Two-theta and eta of given positions (no rotation, no translation, so the
