@@ -169,11 +169,14 @@ __device__ __forceinline__ double fast_atan2(double y, double x, const AtanShare
     return __hiloint2double(__double2hiint(a) | (yh & (int)0x80000000), __double2loint(a));
 }
 
-// 1 / sqrt(x) as the two IEEE operations round it: s to 2^-80 before its rounding
-// (Newton steps from the hardware's 20-bit estimate and the exact residual), then
-// 1 / s to 2^-80 from the same estimate.  9 FP64 operations; the root and the
-// division by themselves take about 18.  k0 = d0 / |d| - 1 cancels near the direct
-// beam, so a last place here is seen in g.
+// 1 / sqrt(x) as the two IEEE operations round it but for rare last bits: s to 2^-80
+// before its rounding (Newton's steps for 1 / sqrt from the hardware's 20-bit estimate,
+// then the root corrected by its exact residual, Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990), then 1 / s to 2^-80 from the
+// same estimate.  A value within 2^-80 of halfway between two doubles can round the
+// other way: a few of 1.6e9 arguments with these steps on a CPU, by one last place.
+// 9 FP64 operations; the root and the division by themselves take about 18.
+// k0 = d0 / |d| - 1 cancels near the direct beam, so a last place here is seen in g.
 __device__ __forceinline__ double inv_sqrt(double x) {
     const int hi = __double2hiint(x);
     if (hi < 0x01000000 || hi > 0x7e000000) return ddiv(1., __dsqrt_rn(x));
@@ -306,9 +309,9 @@ k_geometry(const double* __restrict__ xyz, const double* __restrict__ omega, GvP
 }
 
 // Pipelined variant for 16-byte-aligned inputs: a persistent CTA walks its
-// tiles (blockIdx.x, +gridDim.x, ...) with a 4-stage ring of 1-D TMA bulk
+// tiles (blockIdx.x, +gridDim.x, ...) with a ring of S stages of 1-D TMA bulk
 // copies (xyz 6 KB + omega 2 KB per tile) completed on mbarriers, so the loads
-// of the next three tiles are in flight while the current one is computed and
+// of the next S - 1 tiles are in flight while the current one is computed and
 // stored.  The final partial tile, whose byte counts need not be multiples of
 // 16, is read with ordinary loads.  Bounded waits: on a timeout the CTA stops
 // and counts the event in g_geo_timeouts.
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kGeoThreads, 4)
 k_geometry_tma(const double* __restrict__ xyz, const double* __restrict__ omega, GvParams P,
                double* __restrict__ out, float4* __restrict__ g4, int64_t n) {
     constexpr int OUTW = MODE == 0 ? 3 : 6;
-    constexpr int S = MODE == 0 ? 4 : 3;  // MODE 1 also holds the table (48 KB in all)
+    constexpr int S = MODE == 0 ? 4 : 3;  // (38 KB in all; MODE 1, with the table, 40)
     __shared__ AtanShared s_tab;  // (MODE 0 has no angles and no table)
     double tab[AtanShared::kPer];
     if (MODE == 1) AtanShared::fetch(tab);
@@ -561,7 +564,7 @@ static int geo_grid(int64_t n) {
         if (sms <= 0) sms = 148;
     }
     int64_t tiles = (n + kGeoThreads - 1) / kGeoThreads;
-    int64_t g = (int64_t)sms * 8;  // 8 CTAs of 256 threads resident per SM
+    int64_t g = (int64_t)sms * 8;  // two waves of the kernels with 4 CTAs per SM
     return (int)(tiles < g ? (tiles > 0 ? tiles : 1) : g);
 }
 

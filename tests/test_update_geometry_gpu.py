@@ -68,6 +68,27 @@ def test_ctransform_methods_match_drop_in(cuda):
         ct.sf2geometry(sc, fc[:10], om)
 
 
+def test_inverse_root_rounds_as_root_and_division(oracle, cuda):
+    """With no rotation g is ds (d / |d| - beam) in the reference's operations, exactly
+    but for 1 / |d|, which the kernel takes in one go: every bit as the IEEE root and
+    division give it, but for values within 2^-80 of halfway between two doubles.
+    Of 4 million two roundings at odds of some 2^-27 each make 0.06; at most two may
+    differ, by a last place of 1 / |d|."""
+    from imaged11_b200 import cImageD11
+    rng = np.random.default_rng(75)
+    n = 4_000_000
+    x = rng.normal(size=(n, 3)) * 10.0 ** rng.uniform(-6, 9, (n, 1))
+    x[: n // 2, 0] = 10.0 ** rng.uniform(3, 6, n // 2)         # near the direct beam
+    x[: n // 2, 1:] *= 1e-3
+    om, t, wvln = np.zeros(n), np.zeros(3), 0.2846
+    g = np.empty((n, 3))
+    cImageD11.compute_gv(x, om, 1.0, wvln, 0.0, 0.0, t, g)
+    ref = oracle.compute_gv(x, om, 1.0, wvln, 0.0, 0.0, t)
+    diff = np.abs(g - ref).max(1)
+    assert np.count_nonzero(diff) <= 2
+    assert np.all(diff <= 2.0 ** -51 / wvln)
+
+
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 255, 256, 257, 700])
 def test_positions_off_16_bytes(n, cuda):
     """Positions and omega that are 8 bytes off a 16-byte boundary (a slice of a larger
