@@ -398,7 +398,6 @@ struct BoxWalk {
 // host helpers defined in gvec_grid.cu
 int num_sms();
 unsigned grid_for(int64_t items, int per);
-int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st);
 Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells);
 bool grid_dims_ok(int32_t nx, int32_t xsub);
 

@@ -85,7 +85,7 @@ k_count(const double* __restrict__ gv, int64_t n, const Header H, Header* __rest
     }
 }
 
-// Exclusive scans of one or two arrays x[0 .. len) into y (16-byte aligned), the
+// Exclusive scans of two arrays x[0 .. len) into y (16-byte aligned), the
 // CTAs' totals in tot: blocks 0 .. nb - 1 of the first, then the second's.
 struct ScanJob {
     const int* x;
@@ -743,8 +743,9 @@ __device__ __forceinline__ void lsq_add(double* acc, double s, const double* g,
     acc[16 * 32] += 1.0;
 }
 
-// (24 CTAs, what its shared memory allows, with 80 registers: 2,000 UBIs x 1.1M g
-// 0.42 ms a round; compiled for 32 it spills, 0.53 ms)
+// (24 CTAs with 80 registers, of which its shared memory, 8.6 KB and 1 KB reserved,
+// lets 23 be resident: 2,000 UBIs x 1.1M g 0.42 ms a round; compiled for 32 it
+// spills, 0.53 ms)
 __global__ void __launch_bounds__(kST, 24)
 k_refine(const double* __restrict__ ubis, int64_t m, Split sp, const Header* __restrict__ Hp,
          const int* __restrict__ start, const double* __restrict__ gs,
@@ -1103,17 +1104,11 @@ static int scan_jobs(const ScanJob& a, const ScanJob& b, cudaStream_t st) {
     const unsigned nb = (unsigned)(a.nb + b.nb);
     k_scan_local<<<nb, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
-    k_scan_totals<<<b.nb ? 2 : 1, kScanT, 0, st>>>(a, b);
+    k_scan_totals<<<2, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
     k_scan_add<<<nb, kScanT, 0, st>>>(a, b);
     ID11B_CHECK_LAUNCH();
     return ID11B_OK;
-}
-
-// exclusive scan of x[0..len) into y (len >= 1; both 16-byte aligned), tot: scratch
-int scan(const int* x, int64_t len, int* y, int* tot, cudaStream_t st) {
-    return scan_jobs(ScanJob{x, len, y, tot, (int)scan_blocks(len)},
-                     ScanJob{nullptr, 0, nullptr, nullptr, 0}, st);
 }
 
 // Work items (warps) per UBI: enough for twice `warps` of them per SM, at least
