@@ -38,13 +38,12 @@ sys.path.insert(0, REPO)
 
 TOLS = [0.02, 0.05, 0.1]
 # DRAM bytes (read + write) of one binned-join launch on this workload, from an ncu
-# capture of the same command (profiles/): the traffic is the box records
-K_JOIN_DRAM_BYTES = 404.0e6
+# capture of the present kernel (profiles/): the traffic is the box records
+K_JOIN_DRAM_BYTES = 404.6e6
 K_JOIN_TRAFFIC_NOTE = ("dram__bytes_read.sum + dram__bytes_write.sum of one k_join<3> launch "
-                       "(399.5 + 4.5 MB; 20,000 UBIs, cell factor 0.9, x cut 8x -- the "
-                       "autotuner's pick in the runs recorded; 401.0 MB at 0.8 x 4x; ncu "
-                       "--set full capture in "
-                       "profiles/k_join_binned_20000ubi_1.1Mg.md): mostly the box records, "
+                       "(400.3 + 4.3 MB; 20,000 UBIs, cell factor 0.9, x cut 8x -- the "
+                       "autotuner's pick in the runs recorded; ncu capture in "
+                       "profiles/counters_by_kernel.md): mostly the box records, "
                        "read once; the staged g come from L2")
 N_GRAINS = 2000
 GMAX = 1.5
@@ -894,10 +893,15 @@ def cfg0_measure(cpu=True, reps=3):
 def run_reference(args, rank, world):
     if rank != 0:
         return 0
-    ps, ubis = workload()
     from oracle import oracle as orc
-    lib = orc.Reference() if orc.have_reference() else orc.Oracle()
-    kind = "reference" if isinstance(lib, orc.Reference) else "port"
+    if not orc.have_reference():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "oracle/_ref/libimaged11_ref.so (the reference's own C, "
+                                         "made by oracle/Makefile from a checkout) is absent"}),
+              flush=True)
+        return 0
+    ps, ubis = workload()
+    lib = orc.Reference()
     gv = np.ascontiguousarray(ps.gv)
     cores = lib.max_threads()
     m = max(cores * 4, 64)         # each step: a bounded sample of the workload
@@ -917,7 +921,7 @@ def run_reference(args, rank, world):
         "ms_per_step": 1e3 * sum(times) / len(times), "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": config_dict(len(gv), N_UBI),
-        "cpu_baseline": {"value": value, "unit": "pairs/s", "cores": cores, "kind": kind,
+        "cpu_baseline": {"value": value, "unit": "pairs/s", "cores": cores, "kind": "reference",
                          "sample": "%d UBIs x %d g x %d tols per step" % (m, len(gv), len(TOLS))},
         "e2e": {"value": value, "unit": "pairs/s", "h2d_bytes_per_step": 0,
                 "d2h_bytes_per_step": 0},
@@ -1179,7 +1183,10 @@ def run_ours(args, rank, world, local_rank):
     achieved32 = (m * n * FLOP_PER_EVAL) / (k_ms * 1e-3) / 1e12
     cpu, ref_counts = cpu_reference_rate(ps, ubis) if world == 1 else (None, None)
     parity = {"cfg1": {
-        "vs": "the reference's own score() (oracle/_ref, the unmodified src/closest.c)",
+        "vs": None if cpu is None else
+              "the reference's own score() (oracle/_ref, the unmodified src/closest.c)"
+              if cpu["kind"] == "reference" else
+              "the oracle's score() (oracle/id11_oracle.c, pinned to the reference by fixtures)",
         "ubis_checked": int(len(ref_counts)) if ref_counts is not None else 0,
         "counts_identical": bool(np.array_equal(
             counts[:len(ref_counts)].cpu().numpy(), ref_counts))
