@@ -42,8 +42,8 @@ __device__ __forceinline__ void comp_add(float& s, float& c, float x) {
     s = t;
 }
 
-// One round's pass over the grain's peaks (tid, tid + N, ...), in the reference's
-// FP64 arithmetic: the accepted peaks' normal-equation terms.  Two peaks a step,
+// One round's pass over a thread's n peaks (every N-th of the grain's from first on),
+// in the reference's FP64 arithmetic: the accepted peaks' normal-equation terms.  Two peaks a step,
 // their tests side by side (each is a chain of dependent operations) and the
 // next two's loads in flight; the segment is read-only and re-read every round,
 // so later rounds hit L1.  The terms use fused multiply-adds: H (products of
@@ -67,16 +67,15 @@ __device__ __forceinline__ void add_peak(const double ih[3], const double g[3], 
 
 template <int N>
 __device__ __forceinline__ void refine_peaks(const double u[9], const double* __restrict__ first,
-                                             int tid, int n, double tolsq, double acc[17],
-                                             int& nacc) {
+                                             int n, double tolsq, double acc[17], int& nacc) {
     double nxt[2][3];
 #pragma unroll
     for (int q = 0; q < 2; q++)
 #pragma unroll
         for (int i = 0; i < 3; i++)
-            nxt[q][i] = tid + q * N < n ? __ldg(first + 3 * q * N + i) : 0.;
+            nxt[q][i] = q < n ? __ldg(first + 3 * q * N + i) : 0.;
     const double* p = first;
-    for (int k = tid; k < n; k += 2 * N) {
+    for (int left = n; left > 0; left -= 2) {
         double g[2][3], ih[2][3];
 #pragma unroll
         for (int q = 0; q < 2; q++)
@@ -85,13 +84,13 @@ __device__ __forceinline__ void refine_peaks(const double u[9], const double* __
         p += 6 * N;
 #pragma unroll
         for (int q = 0; q < 2; q++)
-            if (k + (2 + q) * N < n)
+            if (left > 2 + q)
 #pragma unroll
                 for (int i = 0; i < 3; i++) nxt[q][i] = __ldg(p + 3 * q * N + i);
         const double s0 = drlv2_exact(u, g[0][0], g[0][1], g[0][2], ih[0]);
         const double s1 = drlv2_exact(u, g[1][0], g[1][1], g[1][2], ih[1]);
         if (s0 < tolsq) add_peak(ih[0], g[0], s0, acc, nacc);
-        if (k + N < n && s1 < tolsq) add_peak(ih[1], g[1], s1, acc, nacc);
+        if (left > 1 && s1 < tolsq) add_peak(ih[1], g[1], s1, acc, nacc);
     }
 }
 
@@ -99,7 +98,7 @@ __device__ __forceinline__ void refine_peaks(const double u[9], const double* __
 // (score_batch.cu) for this UBI, compensated R and drlv2 sums, exact integer H.
 template <int N>
 __device__ __forceinline__ void refine_peaks_f32c(const double u[9],
-                                                  const double* __restrict__ first, int tid, int n,
+                                                  const double* __restrict__ first, int n,
                                                   double tolsq, double gmax, double acc[17],
                                                   int& nacc) {
     float u32[9], rs[9], rc[9], ss32 = 0.f, sc32 = 0.f;
@@ -121,16 +120,16 @@ __device__ __forceinline__ void refine_peaks_f32c(const double u[9],
     // kU peaks per lane per step: all their loads are issued before any is used
     constexpr int kU = 4;
     const double* p = first;
-    for (int k = tid; k < n; k += kU * N, p += 3 * kU * N) {
+    for (int k = 0; k < n; k += kU, p += 3 * kU * N) {
         double gg[kU][3];
 #pragma unroll
         for (int q = 0; q < kU; q++)
-            if (k + q * N < n)
+            if (k + q < n)
 #pragma unroll
                 for (int i = 0; i < 3; i++) gg[q][i] = __ldg(p + 3 * q * N + i);
 #pragma unroll
         for (int q = 0; q < kU; q++) {
-            if (k + q * N >= n) break;
+            if (k + q >= n) break;
             // g split exactly enough into hi + lo floats
             float gh[3], gl[3], ihf[3], d[3];
 #pragma unroll
@@ -179,21 +178,16 @@ __device__ __forceinline__ void refine_peaks_f32c(const double u[9],
     }
     // to FP64 for the fixed reduction: s + c, exact integers
 #pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] += (double)rs[e] + (double)rc[e];
+    for (int e = 0; e < 9; e++) acc[e] = (double)rs[e] + (double)rc[e];
 #pragma unroll
-    for (int e = 0; e < 6; e++) acc[9 + e] += (double)hint[e];
-    acc[15] += (double)ss32 + (double)sc32;
+    for (int e = 0; e < 6; e++) acc[9 + e] = (double)hint[e];
+    acc[15] = (double)ss32 + (double)sc32;
 }
-
-// Peaks passed over with 32-bit counters at a time: a multiple of what N threads take
-// a step, so that the peaks of a longer grain go to the threads they would go to.
-constexpr int kSpan = 1 << 30;
 
 // `iters` rounds of one grain by N threads (tid of them; N == 32: one warp of the
 // CTA by itself).  red: N / 32 rows of per-warp partial sums.  V > 1 (N == 32):
 // the warp does the work of V warps in turn, peak by peak and sum by sum as they
-// would, so the result has the same bits.  Len: 64 bits for a grain that may be
-// longer than kSpan, else int (64 bits for all: 2 to 6% slower for a few grains).
+// would, so the result has the same bits.
 template <int N, bool F32C, int V = 1, class Len>
 __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], int tid, int g,
                                              double* __restrict__ ubis,
@@ -207,6 +201,9 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
     const int field = slot_of<17>(lane);
     if (tid < 9) sm.ubi[tid] = ubis[9 * (int64_t)g + tid];
     sync();
+    // peaks of the thread that begins at `first`: an int whatever the grain's length
+    auto count = [&](int first) { return (int)((n - first + (N * V - 1)) / (N * V)); };
+    const int mine = count(tid);
     for (int it = 0; it < iters; it++) {
         double u[9];
 #pragma unroll
@@ -219,18 +216,12 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 #pragma unroll
             for (int f = 0; f < 17; f++) acc[f] = 0.;
             int nacc = 0;
-            auto span = [&](Len c) {
-                const double* p = gv + 3 * (k0 + c + first);
-                const int cn = (int)min(n - c, (Len)kSpan);
-                if (F32C)
-                    refine_peaks_f32c<N * V>(u, p, first, cn, tolsq, gmax, acc, nacc);
-                else
-                    refine_peaks<N * V>(u, p, first, cn, tolsq, acc, nacc);
-            };
-            Len c = 0;
-            do {
-                span(c);
-            } while (sizeof(Len) > 4 && (c += kSpan) < n);
+            const int cnt = V == 1 ? mine : count(first);
+            const double* p = gv + 3 * (k0 + first);
+            if (F32C)
+                refine_peaks_f32c<N * V>(u, p, cnt, tolsq, gmax, acc, nacc);
+            else
+                refine_peaks<N * V>(u, p, cnt, tolsq, acc, nacc);
             acc[16] = (double)nacc;
             part += ScatterSum<17, 16>::run(acc, lane);
         }
@@ -303,15 +294,11 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     while (slot < ngrains) {
         const int g = order ? order[slot] : slot;
         const int64_t k0 = off[g];
-        const int64_t n = max(off[g + 1] - k0, (int64_t)0);
+        const int64_t n = off[g + 1] - k0;
         if (NT > 32 && queue && ngrains > (int)gridDim.x && n <= kSolo) break;
         if (tid == 0) s_next = queue ? (int)gridDim.x + atomicAdd(queue, 1) : ngrains;
-        if (n <= kSpan)
-            refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, (int)n, tolsq, iters, npk,
-                                   mean, gmax);
-        else
-            refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
-                                   gmax);
+        refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
+                               gmax);
         slot = s_next;
         if (NT == 32) __syncwarp(); else __syncthreads();
     }
@@ -328,7 +315,7 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     while (mine < ngrains) {
         const int g = order ? order[mine] : mine;
         const int64_t k0 = off[g];
-        const int64_t n = max(off[g + 1] - k0, (int64_t)0);
+        const int64_t n = off[g + 1] - k0;
         int next = 0;
         if (lane == 0) next = (int)gridDim.x + atomicAdd(queue, 1);
         if (n <= kSolo)
