@@ -248,13 +248,13 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 }
 
 // Persistent mode with more grains than CTAs: CTAs of NT threads take grains of
-// more than kSolo peaks whole; from the first smaller one on, each of a CTA's
+// more than `solo` peaks whole; from the first smaller one on, each of a CTA's
 // warps takes grains by itself, so that the rounds' fixed part (the reduction
 // and the 3x3 solves, which one warp does) of several grains overlap.  A larger
 // grain met after that (an order that is not by size) is done by one warp as the
 // CTA would.  So the order of a grain's sums, and with it the last bits of its UBI,
-// follows from its size, from NT and, for grains of up to kSolo peaks, from whether
-// the call has more grains than CTAs; never from the order of the grains or of the
+// follows from its size, from NT and, for grains of up to `solo` peaks, from how many
+// more grains than CTAs the call has; never from the order of the grains or of the
 // CTAs.  (One order for both, kept here, would cost more than it gives: the CTA's by
 // one warp 2,000 grains of 20 .. 2,000 peaks 39 -> 49 us, one warp's where there are
 // few grains 500 of 20 .. 768 peaks 16.4 -> 22.6 us.)
@@ -266,18 +266,21 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 // round.  500 such grains 36.0 -> 17.0, 8,000 of up to 400 peaks, three rounds, 86
 // -> 35 us.
 //
-// kSolo of 256, 512, 768 and 1,024 at 128 threads, five rounds, us (the launch among
+// Solo grains of up to 256, 512, 768 and 1,024 at 128 threads, five rounds, us (the launch among
 // others): 1,000 grains of 20 .. 2,000 peaks 30.3, 30.6, 30.3, 30.6; 2,000 of up to
 // 1,000 37.4, 33.4, 34.8, 37.1 and of up to 2,000 45.9, 45.0, 39.1, 43.2; 4,000 of up
 // to 1,000 57.3, 53.0, 50.2, 54.0; 8,000 of up to 2,000 119, 110, 106, 109; 3,000 of
 // 600 .. 760 75.2, 75.0, 78.1, 78.1 and of 780 .. 1,000 84.1, 84.0, 84.1, 94.1.  768
 // is the best or within 4% of it on all of them.
-// The F32C variant does more per peak, so fewer go to one warp.  192, 256, 384, 512,
-// 768: 1,000 of up to 2,000 peaks 49.0, 51.1, 56.0, 56.1, 54.7; 2,000 74.6, 74.1,
-// 71.4, 76.7, 74.8; 8,000 of up to 400, three rounds, 75.9, 67.5, 57.7, 57.4, 57.4;
-// 8,000 of up to 2,000 225, 219, 211, 204, 200; with a CTA of 64 threads for every
-// grain the second took 84.
-constexpr int kSoloFp64 = 768, kSoloF32c = 384;
+// The F32C variant does more per peak, so fewer go to one warp where there are few
+// grains per CTA, and more where there are many.  192, 384, 768, 1,024: 500 of up to
+// 2,000 peaks 37.6, 38.0, 45.2, 48.7; 1,000 48.6, 53.2, 54.8, 55.4; 2,000 73.3, 69.8,
+// 73.9, 75.4; 4,000 of up to 1,000 92.3, 86.7, 79.3, 83.1; 8,000 of up to 2,000 221,
+// 207, 194, 192; 3,000 of 600 .. 760 135, 134, 106, 106 and of 780 .. 1,000 154, 153,
+// 154, 133; 20,000 of 300 .. 500 644, 508, 371, 371.  With a CTA of 64 threads for
+// every grain 2,000 of up to 2,000 took 86, the last three 124, 144, 551.
+constexpr int kSoloFp64 = 768, kSoloF32c = 384, kSoloF32cMany = 1024;
+constexpr int kManyPerCta = 6;
 
 template <int NT, bool F32C = false>
 __global__ void __launch_bounds__(NT)
@@ -288,14 +291,15 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
     __shared__ RefineSmem sm[NT / 32];
     __shared__ double s_red[NT / 32][17];
     __shared__ int s_next;
-    constexpr int kSolo = F32C ? kSoloF32c : kSoloFp64;
+    const int solo = !F32C ? kSoloFp64 :
+                     ngrains / kManyPerCta > (int)gridDim.x ? kSoloF32cMany : kSoloF32c;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     int slot = blockIdx.x;
     while (slot < ngrains) {
         const int g = order ? order[slot] : slot;
         const int64_t k0 = off[g];
         const int64_t n = off[g + 1] - k0;
-        if (NT > 32 && queue && ngrains > (int)gridDim.x && n <= kSolo) break;
+        if (NT > 32 && queue && ngrains > (int)gridDim.x && n <= solo) break;
         if (tid == 0) s_next = queue ? (int)gridDim.x + atomicAdd(queue, 1) : ngrains;
         refine_grain<NT, F32C>(sm[0], s_red, tid, g, ubis, gv, k0, n, tolsq, iters, npk, mean,
                                gmax);
@@ -318,7 +322,7 @@ k_refine_csr(double* __restrict__ ubis, const double* __restrict__ gv,
         const int64_t n = off[g + 1] - k0;
         int next = 0;
         if (lane == 0) next = (int)gridDim.x + atomicAdd(queue, 1);
-        if (n <= kSolo)
+        if (n <= solo)
             refine_grain<32, F32C>(sm[w], s_red + w, lane, g, ubis, gv, k0, (int)n, tolsq, iters,
                                    npk, mean, gmax);
         else

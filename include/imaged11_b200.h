@@ -400,9 +400,9 @@ int id11b_dev_refine_csr(double *ubis, const double *gv, const int64_t *offsets,
                          void *workspace, int64_t ws_bytes, void *stream);
 
 /* Per-grain refinement as id11b_dev_refine_csr (persistent, 128-thread CTAs;
- * one warp for grains of up to 384 peaks where there are more grains than CTAs)
- * with FP32 screening -- the proven error band of id11b_dev_score_batch, FP64
- * inside it -- and compensated FP32 normal-equation sums (error-free products
+ * one warp for grains of up to 384 peaks where there are more grains than CTAs,
+ * of up to 1,024 with more than six grains per CTA) with FP32 screening -- the
+ * proven error band of id11b_dev_score_batch, FP64 inside it -- and compensated FP32 normal-equation sums (error-free products
  * and TwoSum; H as exact integers), FP64 3x3 solves.  The same accepted pairs
  * and peak counts; UBIs agree with the FP64 sums to ~1e-14 relative, mean
  * drlv2 to the band (~1e-6 relative).  gmax: a bound on every |g_j| (<= 1024,

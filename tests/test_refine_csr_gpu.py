@@ -179,6 +179,26 @@ def test_compensated_more_grains_than_ctas(oracle, ordered, cuda):
     assert np.all(np.abs(mean - ref_m[big]) <= 1e-4 * np.abs(ref_m[big]) + 1e-18)
 
 
+@pytest.mark.parametrize("ngrains,edge", [(1000, 384), (5200, 1024)])
+def test_compensated_one_warp_sizes(oracle, ngrains, edge, cuda):
+    """The compensated variant on both sides of the size that one warp takes, with
+    few grains per CTA and with many; that variant's tolerances above."""
+    from imaged11_b200 import batch, synth
+    rng = np.random.default_rng(47)
+    counts = rng.integers(20, 41, ngrains)
+    counts[:8] = [edge - 1, edge, edge + 1, edge + 31, edge + 128, 1800, 127, 128]
+    rng.shuffle(counts)
+    gv, off, ubis = synth.grain_gvectors(counts, "Ti_hcp", rng)
+    u0 = synth.perturb_ubis(ubis, 0.2, 0.002, rng)
+    ref_u, ref_n, ref_m = oracle.refine_csr(u0, gv, off, 0.05, 3)
+    u, npk, mean = (t.cpu().numpy() for t in
+                    batch.GrainSet(gv, off, u0).refine(0.05, 3, precision="f32c"))
+    assert np.array_equal(npk, ref_n)
+    scale = np.abs(ref_u).reshape(ngrains, -1).max(1)
+    assert np.all(np.abs(u - ref_u).reshape(ngrains, -1).max(1) <= 1e-9 * scale)
+    assert np.all(np.abs(mean - ref_m) <= 1e-4 * np.abs(ref_m) + 1e-18)
+
+
 def test_refine_csr_grain_longer_than_2_31(oracle, cuda):
     """One grain of 2^31 + 300 peaks (its length, and a peak's index in it, need 64
     bits): its peaks are at the start, around 2^30 and 2^31 and at the end, NaN
