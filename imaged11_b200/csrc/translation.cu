@@ -27,12 +27,15 @@
 // by the thread that owns the peak.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace id11b {
 namespace trans {
 
 constexpr int kTT = 64;  // threads per grain
+constexpr int kResident = 4;  // CTAs per SM at most (226 registers)
 // peaks per thread kept in shared memory (three doubles each: 24 KB a CTA); the
 // peaks of a larger grain beyond 64 x 16 are computed in each pass
 constexpr int kKeep = 16;
@@ -194,8 +197,10 @@ __device__ __forceinline__ double refit_ubi(double a, double u0, double* m, int 
 
 // Bound: the FP64 pipe of the SMs that hold four grains (500 grains are 3.4 CTAs
 // per SM), at two warps per scheduler.  500 grains of 420 .. 560 peaks, 30
-// iterations: 0.31 ms; 0.43 with sin, cos and 1 / |d| taken in every pass, full
+// iterations: 0.30 ms; 0.43 with sin, cos and 1 / |d| taken in every pass, full
 // butterflies and one thread's 3x3 solves.  Two or four peaks at a time: 0.32, 0.35.
+// The peaks beyond the kept ones have loops of their own: in one loop with a branch
+// 10 grains of 14,700 peaks, 10 iterations, took 4.2 ms instead of 3.45.
 __global__ void __launch_bounds__(kTT)
 k_refine_translations(const double* __restrict__ xyz, const double* __restrict__ omega,
                       const int64_t* __restrict__ offsets, int32_t ngrains,
@@ -215,9 +220,12 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
     auto angles = [&](int64_t k, PeakG& q) {
         sincos(kRad * omega[p0 + k] * P.omegasign, &q.so, &q.co);
     };
-    for (int64_t i = 0, k = tid; k < np && i < kKeep; i++, k += kTT) {
+    // the thread's peaks that are kept, and their positions
+    const int kept = (int)min((int64_t)kKeep, (np - tid + kTT - 1) / kTT);
+    const double* const mine = xyz + 3 * (p0 + tid);
+    for (int i = 0; i < kept; i++) {
         PeakG q;
-        angles(k, q);
+        angles(tid + kTT * i, q);
         keep[i * kTT] = q.so;
         keep[kF + i * kTT] = q.co;
     }
@@ -243,17 +251,21 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         double a[15];
 #pragma unroll
         for (int q = 0; q < 15; q++) a[q] = 0.;
-        for (int64_t i = 0, k = tid; k < np; i++, k += kTT) {
-            const double* x = xyz + 3 * (p0 + k);
+        for (int i = 0; i < kept; i++) {
+            const double* x = mine + 3 * kTT * i;
             PeakG q;
-            if (i < kKeep) {
-                q.so = keep[i * kTT];
-                q.co = keep[kF + i * kTT];
-            } else {
-                angles(k, q);
-            }
+            q.so = keep[i * kTT];
+            q.co = keep[kF + i * kTT];
             peak_g<false>(P, t, x[0], x[1], x[2], q);
-            if (i < kKeep) keep[2 * kF + i * kTT] = q.inv;
+            keep[2 * kF + i * kTT] = q.inv;
+            refit_terms(P, u0, q, a);
+        }
+        for (int64_t k = tid + kKeep * kTT; k < np; k += kTT) {
+            const double* x = xyz + 3 * (p0 + k);
+            const double x0 = x[0], x1 = x[1], x2 = x[2];
+            PeakG q;
+            angles(k, q);
+            peak_g<false>(P, t, x0, x1, x2, q);
             refit_terms(P, u0, q, a);
         }
         {
@@ -277,18 +289,21 @@ k_refine_translations(const double* __restrict__ xyz, const double* __restrict__
         Acc acc;
 #pragma unroll
         for (int q = 0; q < 11; q++) acc.a[q] = 0.;
-        for (int64_t i = 0, k = tid; k < np; i++, k += kTT) {
+        for (int i = 0; i < kept; i++) {
             PeakG q;
+            const double* x = mine + 3 * kTT * i;
+            q.so = keep[i * kTT];
+            q.co = keep[kF + i * kTT];
+            q.inv = keep[2 * kF + i * kTT];
+            peak_g<true>(P, t, x[0], x[1], x[2], q);
+            peak_terms(P, u1, q, acc);
+        }
+        for (int64_t k = tid + kKeep * kTT; k < np; k += kTT) {
             const double* x = xyz + 3 * (p0 + k);
-            if (i < kKeep) {
-                q.so = keep[i * kTT];
-                q.co = keep[kF + i * kTT];
-                q.inv = keep[2 * kF + i * kTT];
-                peak_g<true>(P, t, x[0], x[1], x[2], q);
-            } else {
-                angles(k, q);
-                peak_g<false>(P, t, x[0], x[1], x[2], q);
-            }
+            const double x0 = x[0], x1 = x[1], x2 = x[2];
+            PeakG q;
+            angles(k, q);
+            peak_g<false>(P, t, x0, x1, x2, q);
             peak_terms(P, u1, q, acc);
         }
         {
@@ -372,9 +387,25 @@ extern "C" int id11b_dev_refine_translations(const double* xyz, const double* om
     P.omegasign = omegasign;
     P.ds = 1.0 / wvln;
     P.tol2 = tol * tol;
-    k_refine_translations<<<(unsigned)ngrains, kTT, sizeof(double) * 3 * kKeep * kTT,
-                            (cudaStream_t)stream>>>(
-        xyz, omega, offsets, ngrains, ubis, translations, P, iters, cost, npk, ubis_refit);
-    ID11B_CHECK_LAUNCH();
+    // Shared memory for the CTAs that will be on an SM, the rest of its 228 KB as L1: each
+    // pass reads the grain's peaks again (30 grains of 4,900 peaks, 196 KB each: 0.90 ms,
+    // 1.15 with the split the driver takes).
+    int dev = 0, sms = 0;
+    ID11B_CHECK(cudaGetDevice(&dev));
+    ID11B_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int each = (int)sizeof(double) * 3 * kKeep * kTT;
+    const int ctas = std::min((ngrains - 1) / std::max(sms, 1) + 1, kResident);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[0].val.sharedMemCarveout = 100 * ctas * (each + 2048) / (228 * 1024) + 1;  // percent
+    cfg.gridDim = dim3((unsigned)ngrains);
+    cfg.blockDim = dim3(kTT);
+    cfg.dynamicSmemBytes = each;
+    cfg.stream = (cudaStream_t)stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    ID11B_CHECK(cudaLaunchKernelEx(&cfg, k_refine_translations, xyz, omega, offsets, ngrains, ubis,
+                                   translations, P, iters, cost, npk, ubis_refit));
     return ID11B_OK;
 }
