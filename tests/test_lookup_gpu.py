@@ -57,7 +57,7 @@ def test_second_slab_with_many_ubis(scene, oracle, two, cuda):
     import torch
     from imaged11_b200 import batch, synth
     from imaged11_b200._lib import lib
-    g = scene[0][:700]
+    g = scene[0]
     grid = batch.GvecGrid(g, cell=0.0115, xsub=4)
     assert 20 * grid.n + 4 * grid.nx ** 3 * grid.xsub > 60 << 20
     m = 38000
@@ -76,6 +76,7 @@ def test_second_slab_with_many_ubis(scene, oracle, two, cuda):
     assert score(al(16 * m) + al(32 * m) - 256) == 4     # ID11B_ERR_SIZE
     assert score(ws) == 0
     torch.cuda.synchronize()
+    assert grid.stats()["fallback_ubis"] == np.count_nonzero(~u.any((1, 2)))
     assert np.array_equal(cnt.cpu().numpy(), oracle.score_many(u, g, tols))
     npk = torch.zeros(m, dtype=torch.int32, device=cuda)
     mean = torch.zeros(m, dtype=torch.float64, device=cuda)
