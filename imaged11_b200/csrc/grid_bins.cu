@@ -75,6 +75,7 @@ constexpr int kEW = ID11B_ENUM_WARPS;
 constexpr int kET = 32 * kEW;
 constexpr int kJT = 256;            // threads per join CTA (one row at a time)
 constexpr int kJW = kJT / 32;
+constexpr int kBigQ = 4;            // boxes a thread takes at a time from a crowded cell
 #ifndef ID11B_JOIN_BMAX
 #define ID11B_JOIN_BMAX 4096
 #endif
@@ -1037,7 +1038,7 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
     int* s_gs = s_gh + nh1;          // staged g before each x cell of the tile
     int* s_rp = s_gs + nh1;          // halo rows: candidate prefix (nhalo + 1)
     int* s_rs = s_rp + (nhalo + 1);  // halo rows: first g
-    __shared__ int s_row, s_w[kJW], s_base, s_run;
+    __shared__ int s_row, s_w[kJW], s_run;
     const Staged T{s_gx, s_gy, s_gz, s_gp};
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned ntest = 0;
@@ -1093,22 +1094,38 @@ k_join(const uint64_t* __restrict__ recs, const int* __restrict__ rstart, int nr
                         s_box[s_bs[fx] - s_bs[cur_wa] + atomicAdd(s_bc + fx, 1)] = rec;
                 }
             } else {  // boxes skip .. skip + nb - 1 of cell cur_wa, in storage order
-                if (threadIdx.x == 0) s_base = 0;
-                __syncthreads();
-                for (int i0 = b0; i0 < b1; i0 += kJT) {
-                    const int i = i0 + threadIdx.x;
-                    uint64_t rec = 0;
-                    const bool mine = i < b1 && box_fx(rec = recs[i]) == cur_wa;
-                    const unsigned bal = __ballot_sync(0xffffffffu, mine);
-                    if (lane == 0) s_w[w] = __popc(bal);
+                // kBigQ boxes a thread and step, the warps' counts in turn in two rows of
+                // the tile's (free) memory, so that a step takes one barrier
+                int* s_cnt = reinterpret_cast<int*>(s_gx);
+                int base = 0;  // boxes of the cell before the step (uniform)
+                for (int i0 = b0; i0 < b1 && base < skip + nb; i0 += kBigQ * kJT) {
+                    uint64_t rec[kBigQ];
+                    unsigned bal[kBigQ];
+#pragma unroll
+                    for (int q = 0; q < kBigQ; q++) {
+                        const int i = i0 + q * kJT + threadIdx.x;
+                        rec[q] = i < b1 ? recs[i] : ~0ull;  // (no cell's: nxx <= 8191)
+                    }
+#pragma unroll
+                    for (int q = 0; q < kBigQ; q++) {
+                        bal[q] = __ballot_sync(0xffffffffu, box_fx(rec[q]) == cur_wa);
+                        if (lane == 0) s_cnt[q * kJW + w] = __popc(bal[q]);
+                    }
                     __syncthreads();
-                    int rank = s_base + __popc(bal & ((1u << lane) - 1u));
-                    for (int k = 0; k < w; k++) rank += s_w[k];
-                    if (mine && rank >= skip && rank < skip + nb) s_box[rank - skip] = rec;
-                    __syncthreads();
-                    if (threadIdx.x == 0)
-                        for (int k = 0; k < kJW; k++) s_base += s_w[k];
-                    __syncthreads();
+#pragma unroll
+                    for (int q = 0; q < kBigQ; q++) {
+                        int rank = base + __popc(bal[q] & ((1u << lane) - 1u));
+#pragma unroll
+                        for (int k = 0; k < kJW; k++) {
+                            const int c = s_cnt[q * kJW + k];
+                            base += c;
+                            if (k < w) rank += c;
+                        }
+                        if ((bal[q] >> lane & 1u) && rank >= skip && rank < skip + nb)
+                            s_box[rank - skip] = rec[q];
+                    }
+                    s_cnt = reinterpret_cast<int*>(s_gx) +
+                            (s_cnt == reinterpret_cast<int*>(s_gx) ? kBigQ * kJW : 0);
                 }
             }
             __syncthreads();

@@ -263,6 +263,27 @@ def test_bins_ranges_with_plainly_scanned_ubis(B, oracle, scene, cuda):
     assert grid.stats()["fallback_ubis"] == 83 + 8 + 1
 
 
+@pytest.mark.parametrize("m", [4096, 4097, 8193, 9001])
+@pytest.mark.parametrize("spread", [0.0, 1e-3])
+def test_bins_crowded_cells(B, oracle, scene, m, spread, cuda):
+    """Trials around one orientation: x cells that hold more boxes than a window
+    (4,096), which the join takes in pieces; counts, and sums within their step."""
+    ps, ubis = scene
+    g = ps.gv
+    rng = np.random.default_rng(34)
+    u = ubis[:1] + spread * rng.normal(size=(m, 3, 3))
+    grid = B.GvecGrid(g, cell=0.1, xsub=2)
+    tols = [0.05, 0.1, 0.3]
+    ref = oracle.score_many(u, g, tols)
+    assert np.array_equal(B.score_grid(u, grid, tols, method="bins").cpu().numpy(), ref)
+    assert grid.stats()["fallback_ubis"] == 0
+    c, s = B.score_grid(u, grid, tols, sums=True, method="bins")
+    assert np.array_equal(c.cpu().numpy(), ref)
+    w = B.score_grid(u, grid, tols, sums=True, method="walk")[1]
+    step = 2.0 ** -(62 - np.ceil(np.log2(len(g) * max(tols) ** 2)))
+    assert np.all((s - w).abs().cpu().numpy() <= 1e-12 * w.cpu().numpy() + ref * step)
+
+
 def test_bins_rejects_large_tolerances(B, scene, cuda):
     ps, ubis = scene
     with pytest.raises(Exception):
