@@ -1562,7 +1562,8 @@ static int bins_pipeline(const double* ubis, int64_t m, int64_t n, int32_t nx, i
     if (ws_bytes < (int64_t)L0.bytes) return ID11B_ERR_SIZE;
     int64_t cap = (ws_bytes - (int64_t)L0.bytes) / (int64_t)(2 * sizeof(uint64_t));
     while (cap > 0 && (int64_t)bin_layout(m, nrows, cap).bytes > ws_bytes) cap -= 1 + cap / 1024;
-    if (cap > INT32_MAX - 1) cap = INT32_MAX - 1;
+    // (32-bit box indices: a CTA's step past the last box must fit too)
+    if (cap > INT32_MAX - 65536) cap = INT32_MAX - 65536;
     const BinLayout B = bin_layout(m, nrows, cap);
     const Layout L = layout(n, (int64_t)nrows * nxx);
     char* g = (char*)gridbuf;
