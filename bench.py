@@ -39,9 +39,9 @@ sys.path.insert(0, REPO)
 TOLS = [0.02, 0.05, 0.1]
 # DRAM bytes (read + write) of one binned-join launch on this workload, from an ncu
 # capture of the present kernel (profiles/): the traffic is the box records
-K_JOIN_DRAM_BYTES = 404.6e6
+K_JOIN_DRAM_BYTES = 404.1e6
 K_JOIN_TRAFFIC_NOTE = ("dram__bytes_read.sum + dram__bytes_write.sum of one k_join<3> launch "
-                       "(400.3 + 4.3 MB; 20,000 UBIs, cell factor 0.9, x cut 8x -- the "
+                       "(400.4 + 3.7 MB; 20,000 UBIs, cell factor 0.9, x cut 8x -- the "
                        "autotuner's pick in the runs recorded; ncu capture in "
                        "profiles/counters_by_kernel.md): mostly the box records, "
                        "read once; the staged g come from L2")

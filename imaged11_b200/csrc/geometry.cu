@@ -455,7 +455,7 @@ k_xlylzl(const double* __restrict__ s, const double* __restrict__ f, XyzParams P
 //
 // A warp owns tiles of 32 peaks: its outputs go through its own part of shared
 // memory, so no warp waits for another.  10M peaks with the lab positions: 225 us with
-// the library's arctangents and a CTA's 256 peaks behind two barriers, 178 now (5.4
+// the library's arctangents and a CTA's 256 peaks behind two barriers, 174 now (5.5
 // TB/s); two waves of CTAs, since one ended unevenly (186).
 template <bool XYZ, bool G4>
 __global__ void __launch_bounds__(kGeoThreads, 4)

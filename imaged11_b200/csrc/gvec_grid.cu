@@ -399,8 +399,8 @@ __device__ __forceinline__ void scan_segments(const volatile WarpPlan* wp, Batch
 // g come from the FP32 copy (one 16-byte load instead of three of 8), the
 // screen is the ellipsoid's (half the box's volume) and costs FP32
 // instructions, and only what passes it is read and evaluated in FP64.  20,000
-// UBIs scored at three tolerances over 1.1M g: 6.95 -> 6.1 ms; over 10.2M g at
-// one: 11.6 -> 8.7 ms; 2,000 refined over 1.1M g: 0.49 -> 0.38 ms a round.
+// UBIs scored at three tolerances over 1.1M g: 6.95 -> 5.64 ms; over 10.2M g at
+// one: 11.7 -> 9.9 ms; 2,000 refined over 1.1M g: 0.49 -> 0.37 ms a round.
 template <class Act>
 __device__ __forceinline__ void lookup_batch(const volatile WarpPlan* wp, Batch* bt,
                                              const unsigned long long* q_w, int take, bool last,
@@ -1154,8 +1154,7 @@ static int refine_parts(int64_t m, int64_t n, int64_t ncells) {
 // at least `parts` items with `more`, else at most.  32 MB: of a 10.2M-g index
 // (250 MB of them), 20,000 grains are assigned in 8.7 ms; one slab 11.8 ms, 96 MB
 // 9.9, 48 MB 9.0, 16 MB 9.2, 12 MB 9.3 (each slab goes through every column).  A
-// 1.1M-g index (52 MB) is two slabs where there are parts to split: 20,000 UBIs
-// score in 6.1 ms, in 6.4 as one.
+// 1.1M-g index (52 MB) is two slabs where there are parts to split.
 Split split_for(int parts, bool more, int64_t m, int64_t n, int64_t ncells) {
     int slabs = (int)std::min<int64_t>(16, (index_bytes(n, ncells) + (32 << 20) - 1) >> 25);
     if (slabs < 1) slabs = 1;
