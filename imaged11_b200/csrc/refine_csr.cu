@@ -259,15 +259,15 @@ __device__ __forceinline__ void refine_grain(RefineSmem& sm, double (*red)[17], 
 // one warp 2,000 grains of 20 .. 2,000 peaks 39 -> 49 us, one warp's where there are
 // few grains 500 of 20 .. 768 peaks 16.4 -> 22.6 us.)
 //
-// Bound: instruction issue and FP64 latency at 16 resident warps (123
-// registers), then the largest grains' own five rounds.  2,000 grains of 20 ..
+// Bound: instruction issue and FP64 latency at 16 resident warps (116 registers),
+// then the largest grains' own five rounds.  2,000 grains of 20 ..
 // 2,000 peaks (859k), five rounds: 36.6 us with 128 threads, 42 with 64; 55.9 (64)
 // and 80.2 (128) with a CTA for every grain, 17 warp sums and five barriers a
 // round.  500 such grains 36.0 -> 17.0, 8,000 of up to 400 peaks, three rounds, 86
 // -> 35 us.
 //
-// Solo grains of up to 256, 512, 768 and 1,024 at 128 threads, five rounds, us (the launch among
-// others): 1,000 grains of 20 .. 2,000 peaks 30.3, 30.6, 30.3, 30.6; 2,000 of up to
+// Solo grains of up to 256, 512, 768 and 1,024 at 128 threads, five rounds, us (the
+// launch among others): 1,000 grains of 20 .. 2,000 peaks 30.3, 30.6, 30.3, 30.6; 2,000 of up to
 // 1,000 37.4, 33.4, 34.8, 37.1 and of up to 2,000 45.9, 45.0, 39.1, 43.2; 4,000 of up
 // to 1,000 57.3, 53.0, 50.2, 54.0; 8,000 of up to 2,000 119, 110, 106, 109; 3,000 of
 // 600 .. 760 75.2, 75.0, 78.1, 78.1 and of 780 .. 1,000 84.1, 84.0, 84.1, 94.1.  768
